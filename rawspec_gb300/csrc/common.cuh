@@ -86,6 +86,25 @@ template <> struct Unpack<FMT_I16, 1> {
   static __device__ __forceinline__ void run(uint32_t w, float2 (&o)[1]) { unpack_word_int(w, o, 16); }
 };
 
+// 8-bit codes as floats without conversion instructions: the four codes of a
+// word, -128 clamped to -127 as above, moved to 1 .. 255 and placed by byte
+// permutes into the mantissa of 2^15, which gives code + kCodeBias exactly.
+// The first pass of a transform adds and subtracts such values exactly (sums
+// of up to 32 of them keep all integer bits), the offset cancels in every
+// difference and so ends in output 0 alone, R times kCodeBias in both parts,
+// where the pass takes it off (GroupFFT, BIASED).  Against I2F: 8 points
+// 93 -> 85 us, 1024 points 183 -> 179 us per 64 Mi samples.
+constexpr float kCodeBias = 32768.0f + 128.0f;
+__device__ __forceinline__ uint32_t offset_codes(uint32_t w) {
+  const uint32_t nonzero = (w & 0x7f7f7f7fu) + 0x7f7f7f7fu;      // bit 7 of a byte: its low bits are not all 0
+  const uint32_t lowest = ~nonzero & w & 0x80808080u;            // bytes of -128
+  return (w ^ 0x80808080u) | (lowest >> 7);
+}
+template <int K>
+__device__ __forceinline__ float code_float(uint32_t offset) {
+  return __uint_as_float(__byte_perm(offset, 0x47000000u, 0x7404 | (K << 4)));
+}
+
 // ----------------------------------------------------------------------------
 // Complex helpers.
 // ----------------------------------------------------------------------------
@@ -120,27 +139,6 @@ __host__ __device__ constexpr double cos_pi16(int t) {
 // sin(pi t / 16) for t in [0, 16).
 __host__ __device__ constexpr double sin_pi16(int t) {
   return t <= 8 ? cos_pi16(8 - t) : cos_pi16(t - 8);
-}
-
-// Multiply a by the forward twiddle exp(-2 pi i k / len) for 0 <= k < len/2,
-// len a power of two <= 32.  After loop unrolling k and len are constants, so
-// the trivial cases cost no multiplies.
-__device__ __forceinline__ float2 twiddle_fwd(float2 a, int k, int len) {
-  if (k == 0) return a;
-  const int t = (32 / len) * k;  // angle = pi t / 16
-  if (t == 8) return make_float2(a.y, -a.x);  // * (-i)
-  if (t == 4) {                               // * (1 - i)/sqrt(2)
-    constexpr float h = 0.70710678118654752f;
-    return make_float2((a.x + a.y) * h, (a.y - a.x) * h);
-  }
-  if (t == 12) {                              // * (-1 - i)/sqrt(2)
-    constexpr float h = 0.70710678118654752f;
-    return make_float2((a.y - a.x) * h, -(a.x + a.y) * h);
-  }
-  const float c = (float)cos_pi16(t);
-  const float s = (float)sin_pi16(t);
-  // (a.x + i a.y)(c - i s)
-  return make_float2(__fmaf_rn(a.x, c, a.y * s), __fmaf_rn(a.y, c, -a.x * s));
 }
 
 }  // namespace rsg

@@ -2,8 +2,8 @@
 //
 // Two levels:
 //   * dft_regs<R>: an R-point DFT (R a power of two <= 32) held entirely in
-//     registers; radix-2 decimation in frequency with compile-time twiddles,
-//     natural order in and out.
+//     registers; radix-2 decimation in time, natural order in and out, every
+//     twiddle multiplication fused into its butterfly.
 //   * GroupFFT<N, R, NV>: an N-point FFT computed by a group of T = N/R
 //     threads, each holding R values of NV independent vectors (the two
 //     polarisations share every twiddle).  Stockham auto-sort passes of radix
@@ -16,27 +16,34 @@
 // transform is obtained by the index reversal X_inv[k] = X_fwd[(N-k) mod N]
 // applied where results are stored.
 //
+// Butterflies.  The kernels are bound by the FMA pipe (on which a packed
+// f32x2 instruction takes two issue slots of a scalar one), so the engine
+// counts pipe slots.  a +- w b with w = c (1 - i t), t = tan of the angle, is
+// six fused multiply-adds,
+//   u = b.re + t b.im,  v = b.im - t b.re,  a +- c (u + i v),
+// against eight operations for a product followed by two sums (the form of
+// Linzer and Feig, "Implementation of efficient FFT algorithms on fused
+// multiply-add architectures", IEEE Trans. Signal Processing 41, 1993).  In a
+// twiddled pass the input factors w^r, r < R, need no multiplications of
+// their own: the stage of length L of a decimation-in-time DFT takes
+// w^(R/L) W_L^q, and q and q + L/4 differ by -i only, so a radix-R pass costs
+// 6 operations per butterfly and R/2 table entries (16 points: 192 operations
+// and 8 entries; separate factors: 228 and 15).
+//
 // Two vectors in lockstep (NV = 2, the two polarisations) run on the packed
-// FP32 instructions of sm_100 and later (add/sub/mul/fma .f32x2, each lane
+// FP32 instructions of sm_100 and later (add/sub/fma .f32x2, each lane
 // rounded exactly as the scalar _rn operation): element m of both vectors is
 // held as a cpair {re: (x0.re, x1.re), im: (x0.im, x1.im)}, so that one
 // instruction does the work of two, with the twiddles shared by both lanes.
-// RSG_PACKED=0 selects the scalar form.
 #pragma once
 
-#include "common.cuh"
+#include <type_traits>
 
-#ifndef RSG_PACKED
-#define RSG_PACKED 1
-#endif
+#include "common.cuh"
 
 namespace rsg {
 
 // ---- packed pairs -----------------------------------------------------------
-struct cpair {
-  float2 re, im;  // lane 0: vector 0, lane 1: vector 1
-};
-
 __device__ __forceinline__ float2 f2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 f2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
@@ -53,8 +60,23 @@ __device__ __forceinline__ float2 f2sub(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 f2dup(float x) { return make_float2(x, x); }
 
-__device__ __forceinline__ cpair padd(const cpair& a, const cpair& b) { return {f2add(a.re, b.re), f2add(a.im, b.im)}; }
-__device__ __forceinline__ cpair psub(const cpair& a, const cpair& b) { return {f2sub(a.re, b.re), f2sub(a.im, b.im)}; }
+// Elements of the engine: float (one vector) or float2 (two in lockstep),
+// with sums, differences and a multiply-add by a factor common to the lanes.
+__device__ __forceinline__ float eadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float2 eadd(float2 a, float2 b) { return f2add(a, b); }
+__device__ __forceinline__ float esub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float2 esub(float2 a, float2 b) { return f2sub(a, b); }
+__device__ __forceinline__ float esubk(float a, float k) { return __fadd_rn(a, -k); }
+__device__ __forceinline__ float2 esubk(float2 a, float k) { return f2add(a, f2dup(-k)); }
+__device__ __forceinline__ float efma(float a, float k, float c) { return __fmaf_rn(a, k, c); }
+__device__ __forceinline__ float2 efma(float2 a, float k, float2 c) { return f2fma(a, f2dup(k), c); }
+
+template <typename E>
+struct cx {
+  E re, im;
+};
+using cpair = cx<float2>;  // lane 0: vector 0, lane 1: vector 1
+
 // a * w for one twiddle w shared by both lanes
 __device__ __forceinline__ cpair pmul(const cpair& a, float2 w) {
   const float2 c = f2dup(w.x), s = f2dup(w.y), ns = f2dup(-w.y);
@@ -64,135 +86,127 @@ __device__ __forceinline__ cpair pack2(float2 x0, float2 x1) { return {make_floa
 __device__ __forceinline__ float2 lane0(const cpair& p) { return make_float2(p.re.x, p.im.x); }
 __device__ __forceinline__ float2 lane1(const cpair& p) { return make_float2(p.re.y, p.im.y); }
 
-// (a - b) * exp(-2 pi i k / len), 0 <= k < len/2, len a power of two <= 32;
-// k and len are compile-time constants after unrolling.
-__device__ __forceinline__ cpair pbfly_lo(const cpair& a, const cpair& b, int k, int len) {
-  if (k == 0) return psub(a, b);
-  const int t = (32 / len) * k;  // angle = pi t / 16
-  if (t == 8) return {f2sub(a.im, b.im), f2sub(b.re, a.re)};  // * (-i)
-  const cpair d = psub(a, b);
-  constexpr float h = 0.70710678118654752f;
-  if (t == 4) return {f2mul(f2add(d.re, d.im), f2dup(h)), f2mul(f2sub(d.im, d.re), f2dup(h))};
-  if (t == 12) return {f2mul(f2sub(d.im, d.re), f2dup(h)), f2mul(f2add(d.re, d.im), f2dup(-h))};
-  const float c = (float)cos_pi16(t);
-  const float s = (float)sin_pi16(t);
-  // (x + i y)(c - i s) = (x c + y s) + i (y c - x s)
-  return {f2fma(d.im, f2dup(s), f2mul(d.re, f2dup(c))), f2fma(d.re, f2dup(-s), f2mul(d.im, f2dup(c)))};
+// The four components of a word of 8-bit codes, (re, im) of lane 0 then of
+// lane 1, as a pair that carries kCodeBias.
+__device__ __forceinline__ cpair unpack_biased(uint32_t w) {
+  const uint32_t u = offset_codes(w);
+  return {make_float2(code_float<0>(u), code_float<2>(u)), make_float2(code_float<1>(u), code_float<3>(u))};
 }
 
-__host__ __device__ constexpr int ilog2(int n) { return n <= 1 ? 0 : 1 + ilog2(n >> 1); }
+// ---- butterflies: (a, b) -> (a + w b, a - w b) ------------------------------
+// w b = m (u + i v), or -i times that (MI).
+template <typename E>
+__device__ __forceinline__ void bfly_uv(cx<E>& a, cx<E>& b, E u, E v, float m, bool mi) {
+  const cx<E> x = a;
+  if (!mi) {
+    a = {efma(u, m, x.re), efma(v, m, x.im)};
+    b = {efma(u, -m, x.re), efma(v, -m, x.im)};
+  } else {
+    a = {efma(v, m, x.re), efma(u, -m, x.im)};
+    b = {efma(v, -m, x.re), efma(u, m, x.im)};
+  }
+}
+
+// w = exp(-2 pi i q / len), 0 <= q < len/2, len a power of two <= 32; q and
+// len are compile-time constants after unrolling.
+template <typename E>
+__device__ __forceinline__ void bfly_const(cx<E>& a, cx<E>& b, int q, int len) {
+  const int t = (32 / len) * q;  // angle = pi t / 16
+  const bool mi = t >= 8;
+  const int r = t & 7;           // remaining angle below pi/2
+  const cx<E> x = a, y = b;
+  if (r == 0) {
+    if (!mi) {
+      a = {eadd(x.re, y.re), eadd(x.im, y.im)};
+      b = {esub(x.re, y.re), esub(x.im, y.im)};
+    } else {
+      a = {eadd(x.re, y.im), esub(x.im, y.re)};
+      b = {esub(x.re, y.im), eadd(x.im, y.re)};
+    }
+    return;
+  }
+  if (r == 4) {  // (1 - i) / sqrt(2)
+    bfly_uv(a, b, eadd(y.re, y.im), esub(y.im, y.re), 0.70710678118654752f, mi);
+    return;
+  }
+  const float c = (float)cos_pi16(r), s = (float)sin_pi16(r);
+  if (r < 4) {  // c (1 - i tan)
+    const float k = (float)(sin_pi16(r) / cos_pi16(r));
+    bfly_uv(a, b, efma(y.im, k, y.re), efma(y.re, -k, y.im), c, mi);
+  } else {      // s (cot - i)
+    const float k = (float)(cos_pi16(r) / sin_pi16(r));
+    const E u = efma(y.re, k, y.im), nv = efma(y.im, -k, y.re);  // w y = s (u - i nv)
+    if (!mi) {
+      a = {efma(u, s, x.re), efma(nv, -s, x.im)};
+      b = {efma(u, -s, x.re), efma(nv, s, x.im)};
+    } else {
+      a = {efma(nv, -s, x.re), efma(u, -s, x.im)};
+      b = {efma(nv, s, x.re), efma(u, s, x.im)};
+    }
+  }
+}
+
+// w = c (1 - i t) from a table entry (c, t), times -i if mi.
+template <typename E>
+__device__ __forceinline__ void bfly_tab(cx<E>& a, cx<E>& b, float2 ct, bool mi) {
+  const cx<E> y = b;
+  bfly_uv(a, b, efma(y.im, ct.y, y.re), efma(y.re, -ct.y, y.im), ct.x, mi);
+}
+
+__host__ __device__ constexpr int ilog2(int n) {
+  int l = 0;
+  while ((2 << l) <= n) ++l;
+  return l;
+}
+// x with its low `bits` (<= 5) bits reversed (no loop, so that a constant
+// argument always folds)
 __host__ __device__ constexpr int bitrev(int x, int bits) {
-  return bits == 0 ? 0 : ((x & 1) << (bits - 1)) | bitrev(x >> 1, bits - 1);
+  return (((x & 1) << 4) | ((x & 2) << 2) | (x & 4) | ((x & 8) >> 2) | ((x & 16) >> 4)) >> (5 - bits);
 }
 
-// Compile-time bit-reversal permutation of a register array.
-template <int R, int M>
-struct BitrevSwap {
-  static __device__ __forceinline__ void apply(float2 (&v)[R]) {
-    constexpr int BR = bitrev(M, ilog2(R));
-    if constexpr (M < BR) {
-      const float2 t = v[M];
-      v[M] = v[BR];
-      v[BR] = t;
-    }
-    BitrevSwap<R, M + 1>::apply(v);
-  }
-};
-template <int R>
-struct BitrevSwap<R, R> {
-  static __device__ __forceinline__ void apply(float2 (&)[R]) {}
-};
-
-// In-register DFT of R points (R = 1, 2, 4, 8, 16, 32), natural order.
-template <int R>
-__device__ __forceinline__ void dft_regs(float2 (&v)[R]) {
-  if constexpr (R > 1) {
+// In-register DFT over the RP elements v[off + s*STRIDE] (RP <= 32), natural
+// order in and out.  tw: the pass's twiddle entries for this butterfly,
+// `tstride` apart (entry i of stage L = 2: i = 0; of stage L >= 4: i = L/4 +
+// q, q < L/4); TW = false: no input factors.
+template <int RP, int STRIDE, bool TW, typename E, int R>
+__device__ __forceinline__ void dft_subset(cx<E> (&v)[R], int off, const float2* __restrict__ tw, int tstride) {
+  if constexpr (RP > 1) {
+    constexpr int LOG = ilog2(RP);
+    cx<E> t[RP];
 #pragma unroll
-    for (int len = R; len >= 2; len >>= 1) {
-      const int half = len >> 1;
+    for (int s = 0; s < RP; ++s) t[s] = v[off + bitrev(s, LOG) * STRIDE];
 #pragma unroll
-      for (int i = 0; i < R; i += len) {
+    for (int l = 1; l <= LOG; ++l) {
+      const int len = 1 << l, half = len >> 1;
+      if constexpr (TW) {
+        const int nq = len >= 4 ? len / 4 : 1;
 #pragma unroll
-        for (int k = 0; k < half; ++k) {
-          const float2 a = v[i + k];
-          const float2 b = v[i + k + half];
-          v[i + k] = cadd(a, b);
-          v[i + k + half] = twiddle_fwd(csub(a, b), k, len);
+        for (int q = 0; q < nq; ++q) {
+          const float2 ct = tw[(len >= 4 ? len / 4 + q : 0) * tstride];
+#pragma unroll
+          for (int i = 0; i < RP; i += len) {
+            bfly_tab(t[i + q], t[i + q + half], ct, false);
+            if (len >= 4) bfly_tab(t[i + q + len / 4], t[i + q + len / 4 + half], ct, true);
+          }
         }
+      } else {
+#pragma unroll
+        for (int i = 0; i < RP; i += len)
+#pragma unroll
+          for (int q = 0; q < half; ++q) bfly_const(t[i + q], t[i + q + half], q, len);
       }
     }
-    // Outputs are in bit-reversed order: undo with compile-time swaps.
-    BitrevSwap<R, 0>::apply(v);
+#pragma unroll
+    for (int s = 0; s < RP; ++s) v[off + s * STRIDE] = t[s];
   }
 }
 
-template <int R, int M>
-struct BitrevSwapP {
-  static __device__ __forceinline__ void apply(cpair (&v)[R]) {
-    constexpr int BR = bitrev(M, ilog2(R));
-    if constexpr (M < BR) {
-      const cpair t = v[M];
-      v[M] = v[BR];
-      v[BR] = t;
-    }
-    BitrevSwapP<R, M + 1>::apply(v);
-  }
-};
-template <int R>
-struct BitrevSwapP<R, R> {
-  static __device__ __forceinline__ void apply(cpair (&)[R]) {}
-};
-
-// dft_regs on packed pairs.
-template <int R>
-__device__ __forceinline__ void dft_regs2(cpair (&v)[R]) {
-  if constexpr (R > 1) {
-#pragma unroll
-    for (int len = R; len >= 2; len >>= 1) {
-      const int half = len >> 1;
-#pragma unroll
-      for (int i = 0; i < R; i += len) {
-#pragma unroll
-        for (int k = 0; k < half; ++k) {
-          const cpair a = v[i + k];
-          const cpair b = v[i + k + half];
-          v[i + k] = padd(a, b);
-          v[i + k + half] = pbfly_lo(a, b, k, len);
-        }
-      }
-    }
-    BitrevSwapP<R, 0>::apply(v);
-  }
-}
-
-template <int RP, int STRIDE, int R>
-__device__ __forceinline__ void dft_subset2(cpair (&v)[R], int off) {
-  cpair t[RP];
-#pragma unroll
-  for (int s = 0; s < RP; ++s) t[s] = v[off + s * STRIDE];
-  dft_regs2<RP>(t);
-#pragma unroll
-  for (int s = 0; s < RP; ++s) v[off + s * STRIDE] = t[s];
-}
-
-// DFT over a strided subset of a register array: elements v[off + s*STRIDE],
-// s = 0..RP-1, with RP*STRIDE <= R.
-template <int RP, int STRIDE, int R>
-__device__ __forceinline__ void dft_subset(float2 (&v)[R], int off) {
-  float2 t[RP];
-#pragma unroll
-  for (int s = 0; s < RP; ++s) t[s] = v[off + s * STRIDE];
-  dft_regs<RP>(t);
-#pragma unroll
-  for (int s = 0; s < RP; ++s) v[off + s * STRIDE] = t[s];
-}
-
-// Shared-memory index with a padding word every 16 complex values, which
-// keeps the strided writes of the Stockham passes free of bank conflicts:
-// element e lives at e + (e >> 4).  GroupFFT computes these positions as a
-// per-thread base plus compile-time offsets, which is exact because every
-// pass's write stride Ns*R and read stride T are powers of two.
-__device__ __forceinline__ int smem_pad(int e) { return e + (e >> 4); }
+// Shared-memory positions of the exchanges, with a padding element every
+// 2^PS elements (PS = log2 R, 4 at least), which keeps the strided writes of
+// the Stockham passes free of bank conflicts: element e lives at
+// e + (e >> PS).  GroupFFT computes these positions as a per-thread base plus
+// compile-time offsets, which is exact because every pass's write stride
+// Ns*R and read stride T are powers of two.
 __host__ __device__ constexpr int smem_padded_len(int n) { return n + (n >> 4) + 1; }
 
 // Number of radix-R passes and the radix of the trailing pass.
@@ -207,15 +221,18 @@ struct FftShape {
 };
 
 // Twiddle table of a GroupFFT<N, R>, one block per twiddled pass, laid out so
-// that the lanes of a warp read consecutive (or identical) entries:
-//   full pass p >= 1 (Ns = R^p):    [r-1][k]  = W_N^(k r N/(Ns R)), k < Ns
-//   trailing pass (radix RL):       [r-1][b]  = W_N^(b r),          b < N/RL
-// StockhamTw<N, R>::offset(p) is the start of pass p's block; `size` the total.
+// that the lanes of a warp read consecutive (or identical) entries.  Entry
+// (i, k) of a pass of radix P after passes of total length M (M = R^p for the
+// full passes p >= 1, N/RL for the trailing one of radix RL) is (cos, tan) of
+// the angle 2 pi (k + q M) / (M L), with (L, q) of index i as in dft_subset:
+//   full pass p:    [i][k], i < R/2,  k < M
+//   trailing pass:  [i][k], i < RL/2, k < M
+// stockham_tw_offset(N, R, p) is the start of pass p's block.
 __host__ __device__ constexpr int stockham_tw_offset(int N, int R, int p) {
   // blocks of passes 1 .. p-1
   int off = 0, Ns = R;
   for (int q = 1; q < p; ++q) {
-    off += (R - 1) * Ns;
+    off += (R / 2) * Ns;
     Ns *= R;
   }
   return off;
@@ -228,163 +245,110 @@ __host__ __device__ constexpr int stockham_tw_size(int N, int R) {
     ++full;
   }
   const int rl = N / Ns;
-  return stockham_tw_offset(N, R, full) + (rl > 1 ? (rl - 1) * (N / rl) : 0);
+  return stockham_tw_offset(N, R, full) + (rl > 1 ? (rl / 2) * (N / rl) : 0);
 }
 
 // Group FFT.  tw: the pass-ordered twiddle table described above (shared or
-// global memory).  sm: this group's exchange buffers, NV buffers of
-// smem_padded_len(N) float2 each, spaced by `sm_stride` float2.  SYNC is a
-// functor performing the barrier required between the group's threads.
+// global memory).  sm: this group's exchange buffers, two buffers (the re and
+// the im parts) of smem_padded_len(N) elements each, `sm_stride` elements
+// apart.  SYNC is a functor performing the barrier required between the
+// group's threads.
 template <int N, int R, int NV>
 struct GroupFFT {
   using S = FftShape<N, R>;
   static constexpr int T = S::T;
+  static constexpr int PS = R >= 32 ? 5 : 4;
+  using E = std::conditional_t<NV == 2, float2, float>;
 
   template <typename Sync>
-  static __device__ __forceinline__ void run(float2 (&v)[NV][R], int j, float2* sm, int sm_stride,
+  static __device__ __forceinline__ void run(float2 (&v)[NV][R], int j, E* sm, int sm_stride,
                                              const float2* __restrict__ tw, Sync sync) {
-    if constexpr (NV == 2 && RSG_PACKED) {
-      cpair p[R];
+    cx<E> p[R];
 #pragma unroll
-      for (int m = 0; m < R; ++m) p[m] = pack2(v[0][m], v[1][m]);
-      run_packed(p, j, sm, sm_stride, tw, sync);
+    for (int m = 0; m < R; ++m) {
+      if constexpr (NV == 2) p[m] = pack2(v[0][m], v[1][m]);
+      else p[m] = {v[0][m].x, v[0][m].y};
+    }
+    run_packed(p, j, sm, sm_stride, tw, sync);
 #pragma unroll
-      for (int m = 0; m < R; ++m) {
+    for (int m = 0; m < R; ++m) {
+      if constexpr (NV == 2) {
         v[0][m] = lane0(p[m]);
         v[1][m] = lane1(p[m]);
+      } else {
+        v[0][m] = make_float2(p[m].re, p[m].im);
       }
-    } else {
-      run_scalar(v, j, sm, sm_stride, tw, sync);
     }
   }
 
-  // Both vectors as packed pairs; the exchange buffers hold the re pairs
-  // (first buffer) and the im pairs (second buffer) at the positions the
-  // scalar form gives the two vectors' values.  SPLIT: one exchange buffer
-  // only (sm_stride unused), the re pairs and then the im pairs passing
-  // through it (twice the barriers, half the shared memory).
-  template <bool SPLIT = false, typename Sync>
-  static __device__ __forceinline__ void run_packed(cpair (&v)[R], int j, float2* sm, int sm_stride,
+  template <bool BIASED>
+  static __device__ __forceinline__ void first_pass(cx<E> (&v)[R]) {
+    dft_subset<R, 1, false>(v, 0, nullptr, 0);
+    if constexpr (BIASED) {
+      v[0].re = esubk(v[0].re, R * kCodeBias);
+      v[0].im = esubk(v[0].im, R * kCodeBias);
+    }
+  }
+
+  // SPLIT: one exchange buffer only (sm_stride unused), the re parts and then
+  // the im parts passing through it (twice the barriers, half the shared
+  // memory).  BIASED: the input values carry kCodeBias.  sync(first, last) is told whether the barrier is the
+  // transform's first (every thread of the group has taken its input) or its
+  // last.
+  template <bool SPLIT = false, bool BIASED = false, typename Sync>
+  static __device__ __forceinline__ void run_packed(cx<E> (&v)[R], int j, E* sm, int sm_stride,
                                                     const float2* __restrict__ tw, Sync sync) {
     if constexpr (T == 1) {
-      dft_regs2<R>(v);
+      first_pass<BIASED>(v);
     } else {
       int Ns = 1;
 #pragma unroll
       for (int p = 0; p < S::FULL; ++p) {
-        if (p > 0) {
+        if (p == 0) {
+          first_pass<BIASED>(v);
+        } else {
           const int k = j & (Ns - 1);
-          const float2* twp = tw + stockham_tw_offset(N, R, p) + k;
-#pragma unroll
-          for (int r = 1; r < R; ++r) v[r] = pmul(v[r], twp[(r - 1) * Ns]);
+          dft_subset<R, 1, true>(v, 0, tw + stockham_tw_offset(N, R, p) + k, Ns);
         }
-        dft_regs2<R>(v);
         const bool last = (p == S::FULL - 1) && (S::RLAST == 1);
         if (!last) {
           const int lo = j & (Ns - 1);
           const int hi = j / Ns;
           const int idxD = hi * Ns * R + lo;
-          const int wbase = idxD + ((hi * Ns * R) >> 4) + (Ns >= 16 ? (lo >> 4) : 0);
-          const int rbase = j + (T >= 16 ? (j >> 4) : 0);
+          const int wbase = idxD + ((hi * Ns * R) >> PS) + (Ns >> PS ? (lo >> PS) : 0);
+          const int rbase = j + (T >> PS ? (j >> PS) : 0);
           if constexpr (SPLIT) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
 #pragma unroll
               for (int r = 0; r < R; ++r) {
-                const int off = Ns >= 16 ? r * (Ns + (Ns >> 4)) : r * Ns + ((r * Ns) >> 4);
+                const int off = Ns >> PS ? r * (Ns + (Ns >> PS)) : r * Ns + ((r * Ns) >> PS);
                 sm[wbase + off] = h == 0 ? v[r].re : v[r].im;
               }
-              sync();
+              sync(p == 0 && h == 0, false);
 #pragma unroll
               for (int m = 0; m < R; ++m) {
-                const int off = T >= 16 ? m * (T + (T >> 4)) : m * T + ((m * T) >> 4);
+                const int off = T >> PS ? m * (T + (T >> PS)) : m * T + ((m * T) >> PS);
                 if (h == 0) v[m].re = sm[rbase + off]; else v[m].im = sm[rbase + off];
               }
-              sync();
+              sync(false, h == 1 && p == S::PASSES - 2);
             }
           } else {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-              const int off = Ns >= 16 ? r * (Ns + (Ns >> 4)) : r * Ns + ((r * Ns) >> 4);
+              const int off = Ns >> PS ? r * (Ns + (Ns >> PS)) : r * Ns + ((r * Ns) >> PS);
               sm[wbase + off] = v[r].re;
               sm[sm_stride + wbase + off] = v[r].im;
             }
-            sync();
+            sync(p == 0, false);
 #pragma unroll
             for (int m = 0; m < R; ++m) {
-              const int off = T >= 16 ? m * (T + (T >> 4)) : m * T + ((m * T) >> 4);
+              const int off = T >> PS ? m * (T + (T >> PS)) : m * T + ((m * T) >> PS);
               v[m].re = sm[rbase + off];
               v[m].im = sm[sm_stride + rbase + off];
             }
-            sync();
+            sync(false, p == S::PASSES - 2);
           }
-        }
-        Ns *= R;
-      }
-      if constexpr (S::RLAST > 1) {
-        constexpr int RL = S::RLAST;
-        constexpr int Q = R / RL;
-        constexpr int NSL = N / RL;
-        const float2* twl = tw + stockham_tw_offset(N, R, S::FULL) + j;
-#pragma unroll
-        for (int qb = 0; qb < Q; ++qb) {
-#pragma unroll
-          for (int r = 1; r < RL; ++r) v[qb + r * Q] = pmul(v[qb + r * Q], twl[(r - 1) * NSL + qb * T]);
-          dft_subset2<RL, Q>(v, qb);
-        }
-      }
-    }
-  }
-
-  template <typename Sync>
-  static __device__ __forceinline__ void run_scalar(float2 (&v)[NV][R], int j, float2* sm, int sm_stride,
-                                                    const float2* __restrict__ tw, Sync sync) {
-    if constexpr (T == 1) {
-      // One thread holds the whole transform.
-#pragma unroll
-      for (int q = 0; q < NV; ++q) dft_regs<R>(v[q]);
-    } else {
-      int Ns = 1;
-#pragma unroll
-      for (int p = 0; p < S::FULL; ++p) {
-        // Twiddles (identity on the first pass).
-        if (p > 0) {
-          const int k = j & (Ns - 1);
-          const float2* twp = tw + stockham_tw_offset(N, R, p) + k;
-#pragma unroll
-          for (int r = 1; r < R; ++r) {
-            const float2 w = twp[(r - 1) * Ns];
-#pragma unroll
-            for (int q = 0; q < NV; ++q) v[q][r] = cmul(v[q][r], w);
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < NV; ++q) dft_regs<R>(v[q]);
-        const bool last = (p == S::FULL - 1) && (S::RLAST == 1);
-        if (!last) {
-          // Padded write positions idxD + r*Ns as a runtime base plus a
-          // compile-time offset per r (see smem_pad).
-          const int lo = j & (Ns - 1);
-          const int hi = j / Ns;
-          const int idxD = hi * Ns * R + lo;
-          const int wbase = idxD + ((hi * Ns * R) >> 4) + (Ns >= 16 ? (lo >> 4) : 0);
-#pragma unroll
-          for (int q = 0; q < NV; ++q)
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              const int off = Ns >= 16 ? r * (Ns + (Ns >> 4)) : r * Ns + ((r * Ns) >> 4);
-              sm[q * sm_stride + wbase + off] = v[q][r];
-            }
-          sync();
-          const int rbase = j + (T >= 16 ? (j >> 4) : 0);
-#pragma unroll
-          for (int q = 0; q < NV; ++q)
-#pragma unroll
-            for (int m = 0; m < R; ++m) {
-              const int off = T >= 16 ? m * (T + (T >> 4)) : m * T + ((m * T) >> 4);
-              v[q][m] = sm[q * sm_stride + rbase + off];
-            }
-          sync();
         }
         Ns *= R;
       }
@@ -396,17 +360,7 @@ struct GroupFFT {
         constexpr int NSL = N / RL;
         const float2* twl = tw + stockham_tw_offset(N, R, S::FULL) + j;
 #pragma unroll
-        for (int qb = 0; qb < Q; ++qb) {
-          // butterfly b = j + qb*T; its twiddles W_N^(b r) sit at [r-1][b]
-#pragma unroll
-          for (int r = 1; r < RL; ++r) {
-            const float2 w = twl[(r - 1) * NSL + qb * T];
-#pragma unroll
-            for (int q = 0; q < NV; ++q) v[q][qb + r * Q] = cmul(v[q][qb + r * Q], w);
-          }
-#pragma unroll
-          for (int q = 0; q < NV; ++q) dft_subset<RL, Q>(v[q], qb);
-        }
+        for (int qb = 0; qb < Q; ++qb) dft_subset<RL, Q, true>(v, qb, twl + qb * T, NSL);
       }
     }
   }

@@ -43,7 +43,9 @@ struct SmallLaunch {
   const void* in = nullptr;
   float* out = nullptr;       // [units_per_chan][|P|][Nc][N], FFT-shifted
   float* partial = nullptr;   // [n_units][chunks][|P|][N] (chunks > 1)
-  const float2* tw = nullptr; // W_N^m, m < N
+  unsigned* arrived = nullptr;  // [arrivals] CTAs that have written their partials, zero between launches (chunks > 1)
+  int arrivals = 0;           // blocks of units (set by small_configure, 0 if no unit is split)
+  const float2* tw = nullptr; // pass-ordered Stockham table
   // per call
   int mode = ACC_WRITE, inverse = 0, conj = 0;
   float scale = 1.0f;         // SNORM scale squared, applied to the results
@@ -56,8 +58,10 @@ struct SmallLaunch {
 
 // Chooses block size, units per block and chunks per unit.  target_ctas is
 // the number of CTAs that fills the GPU.  Returns 0, or -1 if N is out of
-// range.  partial_floats receives the scratch the launch needs (0 if none).
-int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int pipe_groups = 1);
+// range.  partial_floats receives the scratch the launch needs (0 if none),
+// which max_partial (floats) and max_arrivals limit where they are not 0.
+int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int pipe_groups = 1,
+                    size_t max_partial = 0, int max_arrivals = 0);
 cudaError_t small_launch(const SmallLaunch& L, cudaStream_t s);
 // Up to kSmallGroupMax launches of the same kernel configuration (FFT length,
 // sample format, polarisations, mode) in one grid, e.g. the buffers of

@@ -32,27 +32,30 @@ __device__ __forceinline__ float2 w_of(long long e, long long n) {
   return make_float2((float)c, (float)(-s));
 }
 
-// Pass-ordered twiddle table of a GroupFFT<N, R> (layout in fft_core.cuh):
-// full passes p >= 1 with Ns = R^p hold [r-1][k] = W_N^(k r N/(Ns R)); the
-// trailing pass of radix RL holds [r-1][b] = W_N^(b r).
+// Pass-ordered twiddle table of a GroupFFT<N, R> (layout and use in
+// fft_core.cuh): full passes after M = R^p points, then the trailing pass;
+// entry (i, k) is (cos, tan) of 2 pi (k + q M) / (M L).
 __global__ void k_stockham_twiddle(float2* dst, int N, int R, int size) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= size) return;
-  int off = 0, Ns = R;
-  while (Ns * R <= N) {  // full passes 1 .. FULL-1
-    const int blk = (R - 1) * Ns;
-    if (i < off + blk) {
-      const int r = (i - off) / Ns + 1, k = (i - off) % Ns;
-      dst[i] = w_of((long long)k * r * (N / (Ns * R)), N);
-      return;
-    }
-    off += blk;
-    Ns *= R;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= size) return;
+  int off = 0, M = R;
+  while (M * R <= N && e >= off + (R / 2) * M) {
+    off += (R / 2) * M;
+    M *= R;
   }
-  const int rl = N / Ns;  // trailing pass
-  const int nsl = N / rl;
-  const int r = (i - off) / nsl + 1, b = (i - off) % nsl;
-  dst[i] = w_of((long long)b * r, N);
+  const int i = (e - off) / M, k = (e - off) % M;
+  int L = 2, q = 0;
+  if (i > 0) {
+    L = 4;
+    while (L / 2 <= i) L *= 2;
+    q = i - L / 4;
+  }
+  double s, c;
+  sincospi(2.0 * (double)(k + (long long)q * M) / ((double)M * L), &s, &c);
+  // A quarter turn has cos 0 (stage L = 2, k = M/2): a cosine of 1e-18 with
+  // the tangent 1e18 gives a + c (b.re + t b.im) = a + b.im to FP32 rounding.
+  if (c == 0.0) c = 1e-18;
+  dst[e] = make_float2((float)c, (float)(s / c));
 }
 
 cudaError_t stockham_twiddle_fill(float2* dst, int N, int R, cudaStream_t s) {

@@ -47,7 +47,7 @@ template <int POL>
 __host__ __device__ constexpr int pass_b_radix() { return POL == POL_TP ? 16 : 8; }
 
 struct BlockSyncL {
-  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+  __device__ __forceinline__ void operator()(bool, bool) const { __syncthreads(); }
 };
 
 // float2 between the exchange areas of neighbouring sub-FFTs (NV buffers of
@@ -119,8 +119,9 @@ k_large_a(LargeLaunch a) {
   const int e0 = n1 * j;
   const float2 w0 = cmul(__ldg(a.twLo + (e0 & ((1 << a.h) - 1))), __ldg(a.twHi + (e0 >> a.h)));
   __syncthreads();  // twiddle table in shared memory
-  GroupFFT<N2, R, NV>::run(v, j, xch + (size_t)col * sub_stride<N2, C, NV>(), smem_padded_len(N2), tw_s,
-                            BlockSyncL{});
+  using E = typename GroupFFT<N2, R, NV>::E;
+  GroupFFT<N2, R, NV>::run(v, j, reinterpret_cast<E*>(xch + (size_t)col * sub_stride<N2, C, NV>()),
+                            smem_padded_len(N2), tw_s, BlockSyncL{});
 
   // Output k2 = j + m*T: W_N^(n1*k2) = W_N^(n1*j) * W_N^(n1*m*T).
   float2* dst = a.scratch + (size_t)slab * NV * N2 * N1 + n1;
@@ -171,7 +172,8 @@ k_large_b(LargeLaunch a) {
 #pragma unroll
     for (int p = 0; p < NP; ++p) acc[m][p] = 0.0f;
 
-  float2* my_xch = xch + (size_t)row * sub_stride<N1, C, NV>();
+  using E = typename GroupFFT<N1, R, NV>::E;
+  E* my_xch = reinterpret_cast<E*>(xch + (size_t)row * sub_stride<N1, C, NV>());
   for (int sl = s_begin; sl < s_end; ++sl) {
     const int slab = c * a.Nss + d * a.M + sl;
     const float2* src = a.scratch + ((size_t)slab * NV * N2 + k2) * N1 + j;

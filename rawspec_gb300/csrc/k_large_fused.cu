@@ -151,7 +151,7 @@ __device__ __forceinline__ size_t ring_index_il(int k2, int n1) {
 }
 
 struct Sync {
-  __device__ __forceinline__ void operator()() const { __syncthreads(); }
+  __device__ __forceinline__ void operator()(bool, bool) const { __syncthreads(); }
 };
 
 __device__ __forceinline__ int load_acquire(const int* p) {

@@ -23,65 +23,100 @@
 
 namespace rsg {
 
-// R (values per thread per polarisation) is 16 for total power and 8 for the
-// four-plane modes, whose 4*R accumulators would otherwise not fit the
-// register cap of two resident CTAs per SM.
-template <int N, int NP>
+__host__ __device__ constexpr int small_r(int N, int NP) {
+  const int most = NP == 1 && (N == 32 || N == 512 || N == 1024) ? 32 : 16;
+  return N < most ? N : most;
+}
+// The smallest number >= x that is r modulo m.
+__host__ __device__ constexpr int pad_mod(int x, int m, int r) { return x + ((r - x) % m + m) % m; }
+
+// Geometry of a configuration.
+//
+// Vectors in lockstep: the two polarisations of a spectrum, or (one
+// polarisation, PAIR) two spectra of the unit, so that every transform runs
+// on the packed instructions.
+//
+// R, the values per thread per vector: as many as the accumulators leave
+// registers for, since every halving of the passes removes a trip through
+// shared memory, whose bandwidth is the bound next to the FMA pipe.  Total
+// power (one accumulator per bin): 32 where that leaves one exchange (N =
+// 512, 1024: 32 x 16, 32 x 32) or none (N = 32), else 16.  Four planes: 16.
+//
+// MINB: resident CTAs per SM the register budget is cut for: 168 registers a
+// thread for R = 32 and for the four planes at R = 16, 128 otherwise, and for
+// 4096 points in four planes, whose 256-thread CTAs would be alone on their
+// SM (410 us per 64 Mi samples; two of them with spills: 367).
+template <int N, int FMT, int NV, int POL>
 struct SmallCfg {
-  static constexpr int RMAX = NP == 1 ? 16 : 8;
-  static constexpr int R = N < RMAX ? N : RMAX;
+  static constexpr int NP = PolOut<POL>::NP;
+  static constexpr int R = small_r(N, NP);
   static constexpr int T = N / R;            // threads per FFT
-  static constexpr int TPB = T > 256 ? T : 256;
+  static constexpr bool PAIR = NV == 1;      // spectra (not polarisations) in lockstep
+  static constexpr int SPI = PAIR ? 2 : 1;   // spectra a group takes per iteration
+  static constexpr int REGS = R >= 32 || (NP == 4 && R == 16 && T <= 128) ? 168 : 128;
+  static constexpr int TPB = T > 128 ? T : 128;
   static constexpr int G = TPB / T;          // FFT groups per CTA
-  static constexpr int MINB = 65536 / (TPB * 128) > 0 ? 65536 / (TPB * 128) : 1;
+  static constexpr int MINB = 65536 / (TPB * REGS);
   static constexpr int TW = stockham_tw_size(N, R);  // twiddle table entries
+  // Staged input (N >= 16): every group copies its next spectrum into shared
+  // memory with cp.async while it transforms the current one, so that no
+  // registers hold words in flight.  Spectra are RAW bytes apart, the groups
+  // of a warp in different banks.
+  static constexpr bool STAGED = N >= 16;
+  using W = typename SampleWord<FMT, NV>::type;
+  static constexpr int RAW = N * (int)sizeof(W) + (T >= 32 ? 0 : (T * (int)sizeof(W) + 15) / 16 * 16);
+  static constexpr int RAW_GROUP = STAGED ? RAW * SPI : 0;
+  // Exchange: re and im parts through one buffer in turn (SPLIT) where the
+  // group is within a warp, whose barriers cost next to nothing.
+  static constexpr bool SPLIT = T <= 32;
+  static constexpr int PLANE = smem_padded_len(N);
+  // Elements between the groups' exchange buffers: the groups of a half-warp
+  // start T elements apart modulo 16, so that they use different banks.
+  static constexpr int XCH = T == 1 ? 0 : pad_mod(SPLIT ? PLANE : 2 * PLANE, 16, T < 16 ? T : 0);
+  // Floats between the groups' slices of the reduction area (NP R T floats
+  // each): the groups of a warp start T banks apart.
+  static constexpr int RED = T >= 32 ? NP * R * T : pad_mod(NP * R * T, 32, T);
+  // Shared memory: the twiddle table, then the staged input and the exchange
+  // buffers of the groups, or the reduction area.
+  static constexpr size_t TW_BYTES = (size_t)((TW + 1) & ~1) * sizeof(float2);
+  static constexpr size_t WORK = (size_t)G * (RAW_GROUP + XCH * sizeof(float2));
+  static constexpr size_t REDUCE = (size_t)G * RED * sizeof(float);
+  static constexpr size_t SMEM = TW_BYTES + (WORK > REDUCE ? WORK : REDUCE);
 };
 
-struct WarpSync {
-  __device__ __forceinline__ void operator()() const { __syncwarp(); }
-};
 // Barrier of one transform group that spans whole warps (named barrier
 // 1 + group, `threads` = the group's thread count), so that the groups of a
 // CTA progress independently.
-struct GroupSync {
-  int id, threads;
-  __device__ __forceinline__ void operator()() const {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-  }
-};
-
-// Floats between the groups' slices of the reduction area: the slice
-// (NP R T floats) padded so that, with T < 32 threads per group, the groups
-// of a warp start T banks apart and their writes fall into distinct banks.
-template <int N, int NP>
-__host__ __device__ constexpr int small_red_stride() {
-  using C = SmallCfg<N, NP>;
-  constexpr int rb = NP * C::R * C::T;
-  return C::T >= 32 ? rb : rb + ((C::T - rb % 32) % 32 + 32) % 32;
+__device__ __forceinline__ void group_barrier(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-template <int N, int NV, int NP>
-__host__ __device__ constexpr size_t small_smem_bytes() {
-  using C = SmallCfg<N, NP>;
-  const size_t tw = (size_t)((C::TW + 1) & ~1) * sizeof(float2);
-  const size_t xch = (C::T > 1) ? (size_t)C::G * NV * smem_padded_len(N) * sizeof(float2) : 0;
-  const size_t red = (size_t)C::G * small_red_stride<N, NP>() * sizeof(float);
-  return tw + (xch > red ? xch : red);
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
 }
+// The same through L1 (neighbouring copies share a 32-byte sector).
+__device__ __forceinline__ void cp_async16_l1(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The kernel body for CTA `bid` of launch `a` (k_small: one launch;
 // k_small_group: several launches of the same configuration, e.g. the
 // buffers of several jobs, in one grid).
 template <int N, int FMT, int NV, int POL>
 __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) {
-  constexpr int NP = PolOut<POL>::NP;
-  using C = SmallCfg<N, NP>;
-  constexpr int R = C::R, T = C::T, G = C::G, TPB = C::TPB;
+  using C = SmallCfg<N, FMT, NV, POL>;
+  using W = typename C::W;
+  constexpr int NP = C::NP, R = C::R, T = C::T, G = C::G, TPB = C::TPB, SPI = C::SPI;
   extern __shared__ __align__(16) unsigned char smem_raw[];
 
   float2* tw_s = reinterpret_cast<float2*>(smem_raw);
-  float2* xch = tw_s + ((C::TW + 1) & ~1);
-  float* red = reinterpret_cast<float*>(xch);
+  unsigned char* work = smem_raw + C::TW_BYTES;
+  float* red = reinterpret_cast<float*>(work);
 
   const int tid = threadIdx.x;
   const int g = tid / T;   // group within the CTA
@@ -105,43 +140,73 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   const bool unit_ok = unit < a.unit0 + a.unit_count;
   const int c = unit_ok ? unit / a.units_per_chan : 0;
   const int d = unit_ok ? unit % a.units_per_chan : 0;
-  const long long chan_base = (long long)c * a.chan_stride;
-  const long long unit_first_spec = (long long)d * a.M;
-  const int iters = (a.spc + gps - 1) / gps;
+  const int iters = (a.spc + gps * SPI - 1) / (gps * SPI);
   const float im_sign = a.conj ? -1.0f : 1.0f;
+  const W* const unit_src = reinterpret_cast<const W*>(a.in) + (long long)c * a.chan_stride + (long long)d * a.M * N;
+  auto spec_of = [&](int it) { return s_begin + (gi + it * gps) * SPI; };
 
-  float acc[R][NP];
+  // Accumulators.  Total power: one sum per bin over both lanes.  Four
+  // planes: the two powers as one packed pair (|X0|^2, |X1|^2), the cross
+  // terms Re and Im(X0 X1*) unsigned; Stokes I and Q and the conjugation sign
+  // are linear in these sums and applied after the last spectrum.
+  float tp[NP == 1 ? R : 1];
+  float2 pw[NP == 4 ? R : 1], xr[NP == 4 ? R : 1];
 #pragma unroll
-  for (int m = 0; m < R; ++m)
+  for (int m = 0; m < (NP == 1 ? R : 1); ++m) tp[m] = 0.0f;
 #pragma unroll
-    for (int p = 0; p < NP; ++p) acc[m][p] = 0.0f;
-  // Total power of two polarisations on the packed instructions: one lane
-  // per polarisation, the lanes summed after the last spectrum.
-  constexpr bool kPackedTP = POL == POL_TP && NV == 2 && RSG_PACKED;
-  // Cross products of two polarisations: the two powers as one packed pair
-  // (|X0|^2, |X1|^2), the cross terms Re and Im(X0 X1*) unsigned; Stokes I
-  // and Q and the conjugation sign are linear in these sums and applied
-  // after the last spectrum.
-  constexpr bool kPackedX = POL != POL_TP && NV == 2 && RSG_PACKED;
-  float2 acc2[(kPackedTP || kPackedX) ? R : 1];
-#pragma unroll
-  for (int m = 0; m < ((kPackedTP || kPackedX) ? R : 1); ++m) acc2[m] = make_float2(0.f, 0.f);
+  for (int m = 0; m < (NP == 4 ? R : 1); ++m) pw[m] = xr[m] = make_float2(0.f, 0.f);
 
-  float2* my_xch = xch + (size_t)g * NV * smem_padded_len(N);
+  unsigned char* const raw = work + (size_t)g * C::RAW_GROUP;
+  float2* const xch = reinterpret_cast<float2*>(work + (size_t)G * C::RAW_GROUP) + (size_t)g * C::XCH;
 
-  using W = typename SampleWord<FMT, NV>::type;
-  constexpr bool kVec = T == 1 && (R * sizeof(W)) % 16 == 0;
-  // Words of spectrum `it` of this group (zeros past the unit's end).
-  auto load_words = [&](int it, W (&w)[R]) {
-    const int s_local = s_begin + gi + it * gps;
-    if (!(unit_ok && s_local < s_end)) {
+  // Requests the group's spectra of iteration `it` (those that exist).
+  auto stage = [&](int it) {
+#pragma unroll
+    for (int q = 0; q < SPI; ++q) {
+      const int s = spec_of(it) + q;
+      if (!(unit_ok && s < s_end)) break;
+      const W* src = unit_src + (long long)s * N;
+      unsigned char* dst = raw + q * C::RAW;
+      if (a.vec16) {
+#pragma unroll
+        for (int i = 0; i < N * (int)sizeof(W) / 16; i += T) {
+          if (N * (int)sizeof(W) / 16 % T == 0 || i + j < N * (int)sizeof(W) / 16) {
+            if constexpr (T == 1) cp_async16_l1(dst + (i + j) * 16, reinterpret_cast<const char*>(src) + (i + j) * 16);
+            else cp_async16(dst + (i + j) * 16, reinterpret_cast<const char*>(src) + (i + j) * 16);
+          }
+        }
+      } else {
+#pragma unroll 4
+        for (int i = j; i < N; i += T) reinterpret_cast<W*>(dst)[i] = __ldg(src + i);
+      }
+    }
+  };
+  // Words of the staged spectrum q of this group, or of spectrum s in global
+  // memory (short transforms, one thread each).
+  auto take = [&](int q, W (&w)[R]) {
+    const unsigned char* src = raw + q * C::RAW;
+    if constexpr (T == 1) {
+#pragma unroll
+      for (int i = 0; i < (int)(R * sizeof(W) / 16); ++i) {
+        const uint4 u = reinterpret_cast<const uint4*>(src)[i];
+        memcpy(reinterpret_cast<char*>(w) + 16 * i, &u, 16);
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < R; ++m) w[m] = reinterpret_cast<const W*>(src)[j + m * T];
+    }
+  };
+  constexpr bool kBiased = FMT == FMT_I8;  // 8-bit codes carry kCodeBias into the first pass
+  constexpr bool kVec = (R * sizeof(W)) % 16 == 0;
+  auto fetch = [&](int it, int q, W (&w)[R]) {
+    const int s = spec_of(it) + q;
+    if (!(unit_ok && s < s_end)) {
 #pragma unroll
       for (int m = 0; m < R; ++m) w[m] = W{};
       return;
     }
-    const W* src = reinterpret_cast<const W*>(a.in) + chan_base + (unit_first_spec + s_local) * N + j;
+    const W* src = unit_src + (long long)s * N + j;
     if (kVec && a.vec16) {
-      // one thread per transform: its R contiguous words in 16-byte loads
       const uint4* s4 = reinterpret_cast<const uint4*>(src);
 #pragma unroll
       for (int i = 0; i < (int)(R * sizeof(W) / 16); ++i) {
@@ -153,131 +218,172 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
       for (int m = 0; m < R; ++m) w[m] = __ldg(src + m * T);
     }
   };
-  // The next spectrum's words are requested before the current transform
-  // when the registers allow it (spectra of one thread, or 8 values per
-  // thread); otherwise each spectrum is loaded when it is processed.
-  constexpr bool kPrefetch = T == 1 || (NV == 2 ? R <= 8 : R <= 16);
-  static_assert(kPrefetch || !kVec, "vector loads only on the prefetching path");
-  W wn[kPrefetch ? R : 1];
-  if constexpr (kPrefetch) load_words(0, wn);
+  W wn[SPI][C::STAGED ? 1 : R];
+  if constexpr (C::STAGED) {
+    stage(0);
+    if constexpr (T > 32) {
+      cp_async_wait();
+      group_barrier(1 + g, T);
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < SPI; ++q) fetch(0, q, wn[q]);
+  }
 
   for (int it = 0; it < iters; ++it) {
-    const int s_local = s_begin + gi + it * gps;
+    const int s_local = spec_of(it);
     const bool valid = unit_ok && s_local < s_end;
-    float2 v[NV][R];
-    if constexpr (kPrefetch) {
-      W w[R];
+    const bool valid1 = unit_ok && s_local + 1 < s_end;  // PAIR: the second spectrum
+    cpair v[R];
+    {
+      W w[SPI][R];
+      if constexpr (C::STAGED) {
+        if constexpr (T <= 32) {
+          cp_async_wait();
+          __syncwarp();
+        }
 #pragma unroll
-      for (int m = 0; m < R; ++m) w[m] = wn[m];
-      if (it + 1 < iters) load_words(it + 1, wn);
+        for (int q = 0; q < SPI; ++q) take(q, w[q]);
+        if constexpr (T <= 32) {
+          __syncwarp();
+          stage(it + 1);
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < SPI; ++q) {
+#pragma unroll
+          for (int m = 0; m < R; ++m) w[q][m] = wn[q][m];
+          if (it + 1 < iters) fetch(it + 1, q, wn[q]);
+        }
+      }
 #pragma unroll
       for (int m = 0; m < R; ++m) {
-        float2 smp[NV];
-        Unpack<FMT, NV>::run(w[m], smp);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) v[q][m] = smp[q];
+        if constexpr (kBiased) {
+          uint32_t both = w[0][m];
+          if constexpr (C::PAIR) both |= valid1 ? (uint32_t)w[1][m] << 16 : 0u;
+          v[m] = unpack_biased(both);
+        } else if constexpr (C::PAIR) {
+          float2 s0[1], s1[1];
+          Unpack<FMT, 1>::run(w[0][m], s0);
+          Unpack<FMT, 1>::run(valid1 ? w[1][m] : W{}, s1);
+          v[m] = pack2(s0[0], s1[0]);
+        } else {
+          float2 smp[2];
+          Unpack<FMT, 2>::run(w[0][m], smp);
+          v[m] = pack2(smp[0], smp[1]);
+        }
       }
-    } else if (valid) {
-      const W* src = reinterpret_cast<const W*>(a.in) + chan_base + (unit_first_spec + s_local) * N + j;
-      W w[R];
-#pragma unroll
-      for (int m = 0; m < R; ++m) w[m] = __ldg(src + m * T);
-#pragma unroll
-      for (int m = 0; m < R; ++m) {
-        float2 smp[NV];
-        Unpack<FMT, NV>::run(w[m], smp);
-#pragma unroll
-        for (int q = 0; q < NV; ++q) v[q][m] = smp[q];
+    }
+    // Within a warp: the warp's barrier.  Larger groups request the next
+    // spectrum once everyone has taken the current one, and wait for their
+    // part of it before the transform's last barrier, which publishes it.
+    auto sync = [&](bool first, bool last) {
+      if constexpr (T <= 32) {
+        __syncwarp();
+      } else {
+        if (last) cp_async_wait();
+        group_barrier(1 + g, T);
+        if (first) stage(it + 1);
       }
-    } else {
-#pragma unroll
-      for (int m = 0; m < R; ++m)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) v[q][m] = make_float2(0.f, 0.f);
-    }
-    if constexpr (T > 32) {
-      static_assert(G <= 15, "one named barrier per group");
-      GroupFFT<N, R, NV>::run(v, j, my_xch, smem_padded_len(N), tw_s, GroupSync{1 + g, T});
-    } else {
-      GroupFFT<N, R, NV>::run(v, j, my_xch, smem_padded_len(N), tw_s, WarpSync{});
-    }
+    };
+    static_assert(T <= 32 || FftShape<N, R>::PASSES >= 3, "a group's copies span two exchanges");
+    static_assert(G <= 15 || T <= 32, "one named barrier per group");
+    GroupFFT<N, R, 2>::template run_packed<C::SPLIT, kBiased>(v, j, xch, C::PLANE, tw_s, sync);
     if (valid) {
-      if constexpr (kPackedTP) {
 #pragma unroll
-        for (int m = 0; m < R; ++m) {
-          const cpair x = pack2(v[0][m], v[1][m]);
-          acc2[m] = f2fma(x.im, x.im, f2fma(x.re, x.re, acc2[m]));
-        }
-      } else if constexpr (kPackedX) {
-#pragma unroll
-        for (int m = 0; m < R; ++m) {
-          const float2 x0 = v[0][m], x1 = v[1][m];
-          const cpair x = pack2(x0, x1);
-          acc2[m] = f2fma(x.im, x.im, f2fma(x.re, x.re, acc2[m]));
-          acc[m][2] = __fmaf_rn(x0.y, x1.y, __fmaf_rn(x0.x, x1.x, acc[m][2]));
-          acc[m][3] = __fmaf_rn(-x0.x, x1.y, __fmaf_rn(x0.y, x1.x, acc[m][3]));
-        }
-      } else {
-#pragma unroll
-        for (int m = 0; m < R; ++m) {
-          float2 x[NV];
-#pragma unroll
-          for (int q = 0; q < NV; ++q) x[q] = v[q][m];
-          detect_acc<POL, NV>(acc[m], x, im_sign);
+      for (int m = 0; m < R; ++m) {
+        if constexpr (NP == 1) {
+          tp[m] = __fmaf_rn(v[m].re.x, v[m].re.x, tp[m]);
+          tp[m] = __fmaf_rn(v[m].im.x, v[m].im.x, tp[m]);
+          tp[m] = __fmaf_rn(v[m].re.y, v[m].re.y, tp[m]);
+          tp[m] = __fmaf_rn(v[m].im.y, v[m].im.y, tp[m]);
+        } else {
+          const float2 x0 = lane0(v[m]), x1 = lane1(v[m]);
+          pw[m] = f2fma(v[m].im, v[m].im, f2fma(v[m].re, v[m].re, pw[m]));
+          xr[m].x = __fmaf_rn(x0.y, x1.y, __fmaf_rn(x0.x, x1.x, xr[m].x));
+          xr[m].y = __fmaf_rn(-x0.x, x1.y, __fmaf_rn(x0.y, x1.x, xr[m].y));
         }
       }
-    }
-  }
-  if constexpr (kPackedTP) {
-#pragma unroll
-    for (int m = 0; m < R; ++m) acc[m][0] = acc2[m].x + acc2[m].y;
-  }
-  if constexpr (kPackedX) {
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      if constexpr (POL == POL_FULL) {
-        acc[m][0] = acc2[m].x;
-        acc[m][1] = acc2[m].y;
-      } else {
-        acc[m][0] = acc2[m].x + acc2[m].y;
-        acc[m][1] = acc2[m].x - acc2[m].y;
-      }
-      acc[m][3] *= im_sign;
     }
   }
 
-  // Reduce across the groups of each set: red[g][p][m][j], the groups'
-  // slices padded apart (small_red_stride) so that their writes fall into
-  // different banks (with one thread per transform they would all hit one).
-  constexpr int RS = small_red_stride<N, NP>();
+  // Reduce across the groups of each set: red[g][p][m][j].
+  cp_async_wait();  // nothing lands in the area any more (none is in flight after the last iteration)
   __syncthreads();
 #pragma unroll
-  for (int p = 0; p < NP; ++p)
+  for (int m = 0; m < R; ++m) {
+    float acc[NP];
+    if constexpr (NP == 1) {
+      acc[0] = tp[m];
+    } else {
+      acc[0] = POL == POL_FULL ? pw[m].x : pw[m].x + pw[m].y;
+      acc[1] = POL == POL_FULL ? pw[m].y : pw[m].x - pw[m].y;
+      acc[2] = xr[m].x;
+      acc[3] = xr[m].y * im_sign;
+    }
 #pragma unroll
-    for (int m = 0; m < R; ++m) red[g * RS + (p * R + m) * T + j] = acc[m][p];
+    for (int p = 0; p < NP; ++p) red[g * C::RED + (p * R + m) * T + j] = acc[p];
+  }
   __syncthreads();
 
   const int set_threads = gps * T;
   const int t_in_set = tid - set * set_threads;
-  if (!unit_ok) return;
-  for (int o = t_in_set; o < NP * N; o += set_threads) {
+  auto store = [&](int p, int k, float s) {
+    float* dst = a.out + (((size_t)d * NP + p) * a.Nc + c) * N + out_pos(k, N, a.inverse);
+    if (a.mode == ACC_ADD) *dst = __fmaf_rn(s, a.scale, *dst); else *dst = s * a.scale;
+  };
+  for (int o = unit_ok ? t_in_set : NP * N; o < NP * N; o += set_threads) {
     const int p = o / N;
     const int k = o - p * N;
     const int m = k / T;
     const int jj = k - m * T;
     float s = 0.0f;
-    for (int q = 0; q < gps; ++q) s += red[(set * gps + q) * RS + (p * R + m) * T + jj];
-    if (a.chunks > 1) {
-      a.partial[(((size_t)unit * a.chunks + chunk) * NP + p) * N + k] = s;
-    } else {
-      float* dst = a.out + (((size_t)d * NP + p) * a.Nc + c) * N + out_pos(k, N, a.inverse);
-      if (a.mode == ACC_ADD) *dst = __fmaf_rn(s, a.scale, *dst); else *dst = s * a.scale;
+    for (int q = 0; q < gps; ++q) s += red[(set * gps + q) * C::RED + (p * R + m) * T + jj];
+    if (a.chunks > 1) __stcg(a.partial + (((size_t)unit * a.chunks + chunk) * NP + p) * N + k, s);
+    else store(p, k, s);
+  }
+  if (a.chunks == 1) return;
+
+  // Units spread over CTAs: the last CTA of the block of units to arrive sums
+  // the chunks' partials in chunk order (the same order whichever CTA it is)
+  // and leaves the arrival counter zeroed for the next launch.  A kernel of
+  // its own for this sum cost a launch and a drained GPU, 6-10 us a product.
+  __shared__ int s_last;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    s_last = atomicAdd(a.arrived + ublock, 1u) == (unsigned)a.chunks - 1;
+    if (s_last) a.arrived[ublock] = 0;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (!unit_ok) return;
+  constexpr int V = NP * N % 4 == 0 ? 4 : 1;  // outputs per access
+  for (int o = t_in_set * V; o < NP * N; o += set_threads * V) {
+    const float* src = a.partial + (size_t)unit * a.chunks * NP * N + o;
+    float s[V];
+#pragma unroll
+    for (int i = 0; i < V; ++i) s[i] = 0.0f;
+#pragma unroll 8
+    for (int q = 0; q < a.chunks; ++q) {
+      if constexpr (V == 4) {
+        const float4 f = __ldcg(reinterpret_cast<const float4*>(src + (size_t)q * NP * N));
+        s[0] += f.x;
+        s[1] += f.y;
+        s[2] += f.z;
+        s[3] += f.w;
+      } else {
+        s[0] += __ldcg(src + (size_t)q * NP * N);
+      }
     }
+#pragma unroll
+    for (int i = 0; i < V; ++i) store((o + i) / N, (o + i) % N, s[i]);
   }
 }
 
 template <int N, int FMT, int NV, int POL>
-__global__ void __launch_bounds__(SmallCfg<N, PolOut<POL>::NP>::TPB, SmallCfg<N, PolOut<POL>::NP>::MINB)
+__global__ void __launch_bounds__(SmallCfg<N, FMT, NV, POL>::TPB, SmallCfg<N, FMT, NV, POL>::MINB)
 k_small(const __grid_constant__ SmallLaunch a) {
   small_body<N, FMT, NV, POL>(a, blockIdx.x);
 }
@@ -285,7 +391,7 @@ k_small(const __grid_constant__ SmallLaunch a) {
 // Several launches of one configuration in one grid: CTA b belongs to the
 // launch k whose range [end[k-1], end[k]) holds it.
 template <int N, int FMT, int NV, int POL>
-__global__ void __launch_bounds__(SmallCfg<N, PolOut<POL>::NP>::TPB, SmallCfg<N, PolOut<POL>::NP>::MINB)
+__global__ void __launch_bounds__(SmallCfg<N, FMT, NV, POL>::TPB, SmallCfg<N, FMT, NV, POL>::MINB)
 k_small_group(const __grid_constant__ SmallGroup g) {
   int k = 0;
   while (k + 1 < g.n && (int)blockIdx.x >= g.end[k]) ++k;
@@ -318,162 +424,160 @@ __global__ void k_finalize(FinalizeLaunch a) {
 namespace {
 
 struct SmallInfo {
-  int R, T, TPB, G;
+  int R, T, TPB, G, SPI;
   size_t smem;
 };
-
-template <int N, int NP>
-SmallInfo small_info_np(int nv) {
-  using C = SmallCfg<N, NP>;
-  SmallInfo s{C::R, C::T, C::TPB, C::G, 0};
-  s.smem = nv == 1 ? small_smem_bytes<N, 1, NP>() : small_smem_bytes<N, 2, NP>();
-  return s;
-}
-template <int N>
-SmallInfo small_info(int nv, int pol) {
-  return pol == POL_TP ? small_info_np<N, 1>(nv) : small_info_np<N, 4>(nv);
-}
-
-SmallInfo small_info_dyn(int logN, int nv, int pol) {
-  switch (logN) {
-    case 0: return small_info<1>(nv, pol);
-    case 1: return small_info<2>(nv, pol);
-    case 2: return small_info<4>(nv, pol);
-    case 3: return small_info<8>(nv, pol);
-    case 4: return small_info<16>(nv, pol);
-    case 5: return small_info<32>(nv, pol);
-    case 6: return small_info<64>(nv, pol);
-    case 7: return small_info<128>(nv, pol);
-    case 8: return small_info<256>(nv, pol);
-    case 9: return small_info<512>(nv, pol);
-    case 10: return small_info<1024>(nv, pol);
-    case 11: return small_info<2048>(nv, pol);
-    default: return small_info<4096>(nv, pol);
-  }
-}
 
 int small_grid(const SmallLaunch& L) { return ((L.unit_count + L.sets - 1) / L.sets) * L.chunks; }
 
 // op: 0 launch, 1 allow the dynamic shared memory, 2 also report the
 // resident CTAs per SM in *occ, 3 launch the group *grp (entries of L's
-// configuration).
+// configuration), 4 report the geometry in *info.
 template <int N, int FMT, int NV, int POL>
-cudaError_t launch_t(const SmallLaunch& L, cudaStream_t s, int op, int* occ, const SmallGroup* grp) {
+cudaError_t launch_t(const SmallLaunch& L, cudaStream_t s, int op, int* occ, const SmallGroup* grp, SmallInfo* info) {
+  using C = SmallCfg<N, FMT, NV, POL>;
   auto k = k_small<N, FMT, NV, POL>;
+  if (op == 4) {
+    *info = SmallInfo{C::R, C::T, C::TPB, C::G, C::SPI, C::SMEM};
+    return cudaSuccess;
+  }
   if (op == 3) {
     auto kg = k_small_group<N, FMT, NV, POL>;
     cudaError_t e = cudaFuncSetAttribute(kg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
     if (e != cudaSuccess) return e;
     const int grid = grp->end[grp->n - 1];
     if (grid < 1) return cudaSuccess;
-    kg<<<grid, SmallCfg<N, PolOut<POL>::NP>::TPB, L.smem, s>>>(*grp);
+    kg<<<grid, C::TPB, L.smem, s>>>(*grp);
     return cudaGetLastError();
   }
   if (op != 0) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
     if (e != cudaSuccess || op == 1) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, SmallCfg<N, PolOut<POL>::NP>::TPB, L.smem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, C::TPB, L.smem);
   }
   const int grid = small_grid(L);
   if (grid < 1) return cudaSuccess;
-  k<<<grid, SmallCfg<N, PolOut<POL>::NP>::TPB, L.smem, s>>>(L);
+  k<<<grid, C::TPB, L.smem, s>>>(L);
   return cudaGetLastError();
 }
 
 template <int N, int FMT>
-cudaError_t launch_pol(const SmallLaunch& L, cudaStream_t s, int op, int* occ, const SmallGroup* grp) {
-  if (L.nv == 1) return launch_t<N, FMT, 1, POL_TP>(L, s, op, occ, grp);
+cudaError_t launch_pol(const SmallLaunch& L, cudaStream_t s, int op, int* occ, const SmallGroup* grp, SmallInfo* info) {
+  if (L.nv == 1) return launch_t<N, FMT, 1, POL_TP>(L, s, op, occ, grp, info);
   switch (L.pol) {
-    case POL_FULL: return launch_t<N, FMT, 2, POL_FULL>(L, s, op, occ, grp);
-    case POL_STOKES: return launch_t<N, FMT, 2, POL_STOKES>(L, s, op, occ, grp);
-    default: return launch_t<N, FMT, 2, POL_TP>(L, s, op, occ, grp);
+    case POL_FULL: return launch_t<N, FMT, 2, POL_FULL>(L, s, op, occ, grp, info);
+    case POL_STOKES: return launch_t<N, FMT, 2, POL_STOKES>(L, s, op, occ, grp, info);
+    default: return launch_t<N, FMT, 2, POL_TP>(L, s, op, occ, grp, info);
   }
 }
 
 template <int N>
-cudaError_t launch_fmt(const SmallLaunch& L, cudaStream_t s, int op, int* occ, const SmallGroup* grp) {
-  return L.fmt == FMT_I16 ? launch_pol<N, FMT_I16>(L, s, op, occ, grp) : launch_pol<N, FMT_I8>(L, s, op, occ, grp);
+cudaError_t launch_fmt(const SmallLaunch& L, cudaStream_t s, int op, int* occ, const SmallGroup* grp, SmallInfo* info) {
+  return L.fmt == FMT_I16 ? launch_pol<N, FMT_I16>(L, s, op, occ, grp, info) : launch_pol<N, FMT_I8>(L, s, op, occ, grp, info);
 }
 
 cudaError_t small_dispatch(const SmallLaunch& L, cudaStream_t s, int op, int* occ = nullptr,
-                           const SmallGroup* grp = nullptr) {
+                           const SmallGroup* grp = nullptr, SmallInfo* info = nullptr) {
   switch (L.logN) {
-    case 0: return launch_fmt<1>(L, s, op, occ, grp);
-    case 1: return launch_fmt<2>(L, s, op, occ, grp);
-    case 2: return launch_fmt<4>(L, s, op, occ, grp);
-    case 3: return launch_fmt<8>(L, s, op, occ, grp);
-    case 4: return launch_fmt<16>(L, s, op, occ, grp);
-    case 5: return launch_fmt<32>(L, s, op, occ, grp);
-    case 6: return launch_fmt<64>(L, s, op, occ, grp);
-    case 7: return launch_fmt<128>(L, s, op, occ, grp);
-    case 8: return launch_fmt<256>(L, s, op, occ, grp);
-    case 9: return launch_fmt<512>(L, s, op, occ, grp);
-    case 10: return launch_fmt<1024>(L, s, op, occ, grp);
-    case 11: return launch_fmt<2048>(L, s, op, occ, grp);
-    case 12: return launch_fmt<4096>(L, s, op, occ, grp);
+    case 0: return launch_fmt<1>(L, s, op, occ, grp, info);
+    case 1: return launch_fmt<2>(L, s, op, occ, grp, info);
+    case 2: return launch_fmt<4>(L, s, op, occ, grp, info);
+    case 3: return launch_fmt<8>(L, s, op, occ, grp, info);
+    case 4: return launch_fmt<16>(L, s, op, occ, grp, info);
+    case 5: return launch_fmt<32>(L, s, op, occ, grp, info);
+    case 6: return launch_fmt<64>(L, s, op, occ, grp, info);
+    case 7: return launch_fmt<128>(L, s, op, occ, grp, info);
+    case 8: return launch_fmt<256>(L, s, op, occ, grp, info);
+    case 9: return launch_fmt<512>(L, s, op, occ, grp, info);
+    case 10: return launch_fmt<1024>(L, s, op, occ, grp, info);
+    case 11: return launch_fmt<2048>(L, s, op, occ, grp, info);
+    case 12: return launch_fmt<4096>(L, s, op, occ, grp, info);
     default: return cudaErrorInvalidValue;
   }
 }
 
-// Chunks per unit: at least c_min (the parallelism asked for), raised while
-// that makes the grid fill its last wave of resident CTAs markedly better
-// (all CTAs of a launch take about the same time, so a grid of 2.1 waves
-// runs as long as one of 3).  Units processed whole (c_min = 1) stay whole:
-// splitting them would add a finalisation pass.
-#ifndef RSG_SMALL_WAVEFIT
-#define RSG_SMALL_WAVEFIT 1
-#endif
-int fit_chunks(int M, int ublocks, int c_min, int max_chunks, int slots) {
-  auto actual = [&](int c) { const int spc = (M + c - 1) / c; return (M + spc - 1) / spc; };
-  auto eff = [&](int c) {
-    const double w = (double)ublocks * actual(c) / slots;
-    return w / std::ceil(w);
-  };
-  int best = std::max(1, std::min(c_min, max_chunks));
-  if (!RSG_SMALL_WAVEFIT || slots <= 0 || best == 1) return best;
-  for (int c = best + 1; c <= std::min(max_chunks, 2 * best); ++c)
-    if (eff(c) > eff(best) + 0.05) best = c;
+// Chunks per unit: the split with the shortest schedule.  A launch lasts as
+// long as its most loaded SM: ceil(CTAs / SMs) CTAs of `iters` iterations each
+// (an SM with fewer CTAs resident than it holds loses little, so a split over
+// occupancy slots would be the wrong measure: 1024 CTAs of N = 64 run in
+// 127 us, 512 twice as long ones in 143, 2560 in 124), plus about 0.6
+// iterations for a CTA's start and reduction; a CTA alone on its SM is bound
+// by its own latency, about 1.5 times its share of a full one.  Split units
+// add an arrival and a sum at the end (about 2 us) and the traffic of the
+// partial sums.  All times in microseconds.
+struct SplitCost {
+  double unit;     // SM time of one iteration of a CTA
+  double partial;  // traffic of one chunk's partial sums of every unit
+  int sms, occ;
+};
+int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k) {
+  int best = c_lo;
+  double best_cost = 1e300;
+  for (int c = c_lo; c <= c_hi; ++c) {
+    const int per = (turns + c - 1) / c;
+    if (c > c_lo && (turns + per - 1) / per != c) continue;
+    const double per_sm = std::ceil((double)ublocks * c / k.sms);
+    const double load = std::max(per_sm, 1.5 * std::ceil(per_sm / k.occ));
+    const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + (c > 1 ? 2.0 + c * k.partial : 0.0);
+    if (cost < best_cost * 0.99) {
+      best_cost = cost;
+      best = c;
+    }
+  }
   return best;
 }
 
 }  // namespace
 
-int small_radix(int logN, int pol) { return small_info_dyn(logN, 2, pol).R; }
+int small_radix(int logN, int pol) { return small_r(1 << logN, pol == POL_TP ? 1 : 4); }
 
-int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int pipe_groups) {
+int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int pipe_groups, size_t max_partial,
+                    int max_arrivals) {
   if (L.logN < 0 || L.logN > 12 || L.M < 1 || L.n_units < 1) return -1;
-  const SmallInfo si = small_info_dyn(L.logN, L.nv, L.pol);
+  SmallInfo si{};
+  if (small_dispatch(L, nullptr, 4, nullptr, nullptr, &si) != cudaSuccess) return -1;
   L.tpb = si.TPB;
   L.smem = si.smem;
   const int G = si.G;
   const int np = L.pol == POL_TP ? 1 : 4;
   auto pow2_floor = [](int x) { int p = 1; while (p * 2 <= x) p *= 2; return p; };
-  // Groups per unit: at most one per spectrum, and few enough that every
-  // thread of a set has an output to reduce (gps <= |P| * R).
-  int gps = std::min(G, std::min(pow2_floor(np * si.R), pow2_floor(L.M)));
+  // Groups per unit: at most one per spectrum (or pair of them), and few
+  // enough that every thread of a set has an output to reduce (gps <= |P| * R).
+  const int turns = (L.M + si.SPI - 1) / si.SPI;  // iterations of a unit on one group
+  int gps = std::min(G, std::min(pow2_floor(np * si.R), pow2_floor(turns)));
   L.sets = G / gps;
   const int ublocks = (L.n_units + L.sets - 1) / L.sets;
-  const int max_chunks = (L.M + gps - 1) / gps;
+  const int max_chunks = (turns + gps - 1) / gps;
   // resident CTAs on the device
   int occ = 0, sms = 0, dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
       cudaSuccess || small_dispatch(L, nullptr, 2, &occ) != cudaSuccess)
     occ = 0;
-  const int slots = occ * sms;
-  const int chunks = fit_chunks(L.M, ublocks, (target_ctas + ublocks - 1) / ublocks, max_chunks, slots);
-  L.spc = (L.M + chunks - 1) / chunks;
-  L.chunks = (L.M + L.spc - 1) / L.spc;
+  // The split of `units` units: spectra per chunk, and the chunks that makes.
+  auto split = [&](int units, int* spc, int* chunks) {
+    const int ub = (units + L.sets - 1) / L.sets;
+    const int aim = std::max(1, (target_ctas + ub - 1) / ub);  // chunks that fill the GPU
+    // partial sums that fit the limit and the arrival counters
+    const long long floats = (long long)L.n_units * np << L.logN;
+    int most = (int)std::min<long long>(max_chunks, std::max(8, 4 * aim));
+    if (max_partial) most = (int)std::min<long long>(most, std::max<long long>(1, (long long)max_partial / floats));
+    if (max_arrivals && ublocks > max_arrivals) most = 1;
+    // a sample of both lanes takes about 2.3 ps of the GPU; partial sums are
+    // written and read at about 4 TB/s
+    const SplitCost cost{si.TPB * si.R * sms * 2.3e-6, (double)ub * L.sets * np * (1 << L.logN) * 2e-6, sms, occ};
+    const int c = occ > 0 ? fit_chunks(turns, gps, ub, std::min(most, std::max(1, aim / 4)), std::max(1, most), cost)
+                          : std::max(1, std::min(aim, most));
+    const int per = (turns + c - 1) / c;  // iterations' worth of spectra per chunk
+    *spc = std::min(L.M, per * si.SPI);
+    *chunks = (turns + per - 1) / per;
+  };
+  split(L.n_units, &L.spc, &L.chunks);
   L.grid = ublocks * L.chunks;
   // the same for a launch over 1/pipe_groups of the units
-  {
-    const int gunits = std::max(1, L.n_units / std::max(1, pipe_groups));
-    const int gublocks = (gunits + L.sets - 1) / L.sets;
-    const int c2 = fit_chunks(L.M, gublocks, (target_ctas + gublocks - 1) / gublocks, max_chunks, slots);
-    L.spc_pipe = (L.M + c2 - 1) / c2;
-    L.chunks_pipe = (L.M + L.spc_pipe - 1) / L.spc_pipe;
-  }
+  split(std::max(1, L.n_units / std::max(1, pipe_groups)), &L.spc_pipe, &L.chunks_pipe);
   const int cmax = std::max(L.chunks, L.chunks_pipe);
   *partial_floats = cmax > 1 ? (size_t)L.n_units * cmax * np * ((size_t)1 << L.logN) : 0;
+  L.arrivals = cmax > 1 ? ublocks : 0;
   L.unit0 = 0;
   L.unit_count = L.n_units;
   const long long wbytes = (L.fmt == FMT_I16 ? 4 : 2) * L.nv;

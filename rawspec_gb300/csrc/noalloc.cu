@@ -6,8 +6,8 @@
 // other stream of the process), or a host framework that owns all device
 // memory through its own pool and budget.  This entry point takes the input
 // and output as caller-provided device pointers and keeps its only scratch --
-// the per-chunk partial sums of the fused small-FFT kernel and its twiddle
-// table -- in the file-scope array below, which every GPU that loads the
+// the per-chunk partial sums of the fused small-FFT kernel, its twiddle table
+// and its arrival counters -- in the file-scope array below, which every GPU that loads the
 // library holds until the process exits.
 #include <cstdint>
 #include <cstdio>
@@ -20,12 +20,14 @@ namespace {
 
 constexpr size_t kPartialFloats = size_t(1) << 20;  // 4 MiB of partial sums
 constexpr int kMaxNt = 4096;                        // twiddle table capacity
-constexpr size_t kScratchFloats = kPartialFloats + 2 * (size_t)kMaxNt;
+constexpr int kArrivals = 8192;                     // arrival counters of split units, zero between calls
+constexpr size_t kScratchFloats = kPartialFloats + 2 * (size_t)kMaxNt + kArrivals;
 constexpr int kMaxDevices = 64;
 
 }  // namespace
 
-// The shared scratch: partial sums [0, kPartialFloats), twiddles after them.
+// The shared scratch (zero when the library is loaded): partial sums [0,
+// kPartialFloats), twiddles after them, then the arrival counters.
 static __device__ __align__(256) float g_noalloc_scratch[kScratchFloats];
 
 namespace {
@@ -119,6 +121,7 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
   L.out = d_out;
   L.tw = tw;
   L.partial = scratch;
+  L.arrived = reinterpret_cast<unsigned*>(scratch + kPartialFloats + 2 * (size_t)kMaxNt);
   L.mode = ACC_WRITE;
   L.inverse = fft_dir <= 0 ? 1 : 0;
   L.conj = input_conjugated ? 1 : 0;
@@ -129,14 +132,12 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
   int dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Split units over CTAs only as far as the partial sums fit the scratch.
+  // Units are split over CTAs only as far as the partial sums and the arrival
+  // counters fit the scratch.
   size_t need = 0;
-  for (int target = sms * 4;; target /= 2) {
-    if (small_configure(L, target, &need) != 0) {
-      fprintf(stderr, "rawspec_gb300_product_noalloc: unsupported configuration\n");
-      return 1;
-    }
-    if (need <= kPartialFloats || target <= 1) break;
+  if (small_configure(L, sms * 4, &need, 1, kPartialFloats, kArrivals) != 0) {
+    fprintf(stderr, "rawspec_gb300_product_noalloc: unsupported configuration\n");
+    return 1;
   }
   if (need > kPartialFloats) {
     fprintf(stderr, "rawspec_gb300_product_noalloc: partial sums exceed the %zu-float scratch\n", kPartialFloats);
@@ -145,21 +146,6 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
   cudaError_t e = stockham_twiddle_fill(tw, (int)Nt, small_radix(L.logN, L.pol), s);
   if (e == cudaSuccess) e = small_prepare(L);
   if (e == cudaSuccess) e = small_launch(L, s);
-  if (e == cudaSuccess && L.chunks > 1) {
-    FinalizeLaunch F;
-    F.partial = scratch;
-    F.out = d_out;
-    F.n_units = L.n_units;
-    F.chunks = L.chunks;
-    F.np = npol == 1 ? 1 : 4;
-    F.N = (int)Nt;
-    F.Nc = (int)Nc;
-    F.units_per_chan = L.units_per_chan;
-    F.mode = ACC_WRITE;
-    F.inverse = L.inverse;
-    F.scale = L.scale;
-    e = finalize_launch(F, s);
-  }
   if (e != cudaSuccess) {
     fprintf(stderr, "rawspec_gb300_product_noalloc: %s\n", cudaGetErrorName(e));
     return 1;

@@ -75,6 +75,7 @@ struct Product {
   int* d_ctl = nullptr;    // control words of the fused kernel (error word first) or the tc error word
   int* h_err = nullptr;    // pinned copy of the error word, refreshed after every fused or tc launch
   float* d_partial = nullptr;  // per-chunk partial sums of this product
+  unsigned* d_arrived = nullptr;  // k_small: arrival counters of its split units
   bool kahan = false;          // compensated integration across buffers
   float* d_stage = nullptr;    // this buffer's sums (out_bytes), folded into d_out by k_kahan_merge
   float* d_comp = nullptr;     // running compensation of d_out (out_bytes)
@@ -211,22 +212,21 @@ bool graphs_wanted(const GpuCtx* g) {
 }
 
 // Which products of 8-bit input run their DFT on the tensor cores (k_tc)
-// rather than in k_small: by default the total-power products of N = 1024,
-// where k_tc is faster alone (227 against 233 us per 256 MiB buffer) and
-// leaves FMA and issue slots to concurrent CUDA-core kernels.  Since k_small
-// runs both polarisations on the packed f32x2 instructions it is the faster
-// one at N = 4096 (299 against 339 us) and N = 256; the cross-pol modes stay
-// on k_small (k_tc is as fast alone but slows a mixed step with the fused
-// kernel).  RAWSPEC_GB300_TENSOR_DFT=1 at
-// initialisation selects k_tc for every case it supports (N = 256, 1024,
-// 4096, all modes up to 1024), =0 for none.  Without the variable, a
-// tuning-table entry's dft= decides before the default.
-bool tensor_dft_wanted(int logN, int pol, const rawspec_gb300_tune& t) {
+// rather than in k_small: by default the 1024-point total-power products of
+// buffers of at most 2^18 time samples over all channels, where the launch is
+// the time and k_tc, which splits a unit further, is not the slower one
+// (4 channels x 16384 samples 7.8 against 8.0 us a buffer, 1 x 65536 8.0
+// against 10.8; 8 x 65536 9.9 against 8.8, 64 x 262144 59 against 42).
+// RAWSPEC_GB300_TENSOR_DFT=1 at initialisation selects k_tc for every case it
+// supports (N = 256, 1024, 4096, all modes up to 1024), =0 for none.  Without
+// the variable, a tuning-table entry's dft= decides before the default.
+constexpr long long kMaxTensorSamples = 1ll << 18;
+bool tensor_dft_wanted(int logN, int pol, const rawspec_gb300_tune& t, long long samples) {
   const char* v = getenv("RAWSPEC_GB300_TENSOR_DFT");
   if (v && v[0] == '0') return false;
   if (v && v[0] == '1') return true;
   if (t.dft >= 0) return t.dft == 1;
-  return logN == 10 && pol == POL_TP;
+  return logN == 10 && pol == POL_TP && samples <= kMaxTensorSamples;
 }
 
 // Tuning-table entry of product i of a validated context (unset values if
@@ -567,7 +567,7 @@ struct DeferredSmall {
 // Queues product i's kernels for the channels [c0, c1) of the buffer.  With
 // compensated integration the buffers after an integration's first write
 // their sums to the staging plane.  With `defer`, a k_small launch over all
-// channels is recorded there instead (with its finalisation).
+// channels is recorded there instead.
 int launch_product(rawspec_context* ctx, GpuCtx* g, int i, int mode, int inverse, int c0, int c1,
                    std::vector<DeferredSmall>* defer = nullptr) {
   Product& P = g->prod[i];
@@ -615,9 +615,6 @@ int launch_product(rawspec_context* ctx, GpuCtx* g, int i, int mode, int inverse
       RSG_CUDA(small_launch(L, P.stream));
       g->launches++;
     }
-    if (L.chunks > 1 &&
-        launch_finalize(ctx, g, P, out, L.unit0, L.unit_count, L.chunks, L.units_per_chan, mode, inverse, L.scale))
-      return 1;
   } else {
     LargeLaunch L = P.ll;
     L.out = out;
@@ -746,8 +743,7 @@ int process_buffer(rawspec_context* ctx, GpuCtx* g, int fft_dir, int ngroups, co
 // Queues the deferred k_small launches of several contexts: launches of the
 // same kernel configuration share one grid (up to kSmallGroupMax), issued on
 // the first one's product stream after every member's stream has reached
-// it; each member's stream then continues after the shared launch with its
-// own finalisation.
+// it; each member's stream then continues after the shared launch.
 int launch_deferred(std::vector<DeferredSmall>& d) {
   std::vector<char> done(d.size(), 0);
   for (size_t a = 0; a < d.size(); a++) {
@@ -787,10 +783,6 @@ int launch_deferred(std::vector<DeferredSmall>& d) {
       DeferredSmall& e = d[m];
       e.g->launches++;  // every member's context counts the launch it took part in
       if (mem.size() > 1) e.g->shared_launches++;
-      Product& P = e.g->prod[e.product];
-      if (e.L.chunks > 1 && launch_finalize(e.ctx, e.g, P, e.out, e.L.unit0, e.L.unit_count, e.L.chunks,
-                                            e.L.units_per_chan, e.L.mode, e.L.inverse, e.L.scale))
-        return 1;
     }
   }
   return 0;
@@ -823,7 +815,7 @@ int plan_device_bytes(const rawspec_context* ctx, bool expanded, int sm_count, s
     if (kahan_wanted(ctx->Nas[i], Nis)) t += 2 * ctx->h_pwrbuf_size[i];
     if (ctx->incoherently_sum) t += ctx->h_pwrbuf_size[i] / ctx->Nant;
     const bool large = logN > 12;
-    if (!large && tensor_dft_wanted(logN, pol, tune) && tc_supported(logN, fmt, (int)ctx->Np, pol, M)) {
+    if (!large && tensor_dft_wanted(logN, pol, tune, (long long)ctx->Nb * ctx->Ntpb * ctx->Nc) && tc_supported(logN, fmt, (int)ctx->Np, pol, M)) {
       TcLaunch L;
       L.logN = logN;
       L.pol = pol;
@@ -847,7 +839,8 @@ int plan_device_bytes(const rawspec_context* ctx, bool expanded, int sm_count, s
       L.chan_stride = (long long)ctx->Nb * ctx->Ntpb;
       size_t pf = 0;
       if (small_configure(L, target_ctas, &pf, groups)) return 1;
-      t += pf * sizeof(float) + (size_t)std::max(stockham_table_size(N, small_radix(logN, pol)), 1) * sizeof(float2);
+      t += pf * sizeof(float) + (size_t)L.arrivals * sizeof(unsigned) +
+           (size_t)std::max(stockham_table_size(N, small_radix(logN, pol)), 1) * sizeof(float2);
     } else {
       LargeLaunch L;
       L.logN = logN;
@@ -1059,7 +1052,7 @@ int rawspec_initialize(rawspec_context* ctx) {
     }
 
     P.large = P.logN > 12;
-    P.tc = !P.large && tensor_dft_wanted(P.logN, pol, tune) && tc_supported(P.logN, g->fmt, (int)ctx->Np, pol, M);
+    P.tc = !P.large && tensor_dft_wanted(P.logN, pol, tune, (long long)ctx->Nb * ctx->Ntpb * ctx->Nc) && tc_supported(P.logN, g->fmt, (int)ctx->Np, pol, M);
     if (P.tc) {
       TcLaunch& L = P.tl;
       L.logN = P.logN;
@@ -1108,6 +1101,11 @@ int rawspec_initialize(rawspec_context* ctx) {
         FAIL();
       }
       if (pf && dev_alloc(g, &P.d_partial, pf * sizeof(float))) FAIL();
+      if (L.arrivals) {
+        if (dev_alloc(g, &P.d_arrived, (size_t)L.arrivals * sizeof(unsigned))) FAIL();
+        CK(cudaMemsetAsync(P.d_arrived, 0, (size_t)L.arrivals * sizeof(unsigned), g->stream));
+        L.arrived = P.d_arrived;
+      }
       const int R = small_radix(P.logN, pol);
       const size_t ntw = (size_t)std::max(stockham_table_size(P.N, R), 1);
       if (dev_alloc(g, &P.d_tw, ntw * sizeof(float2))) FAIL();
@@ -1246,6 +1244,7 @@ void rawspec_cleanup(rawspec_context* ctx) {
     dfree(g->prod[i].d_ctl);
     pinned_free(g->prod[i].h_err, sizeof(int));
     dfree(g->prod[i].d_partial);
+    dfree(g->prod[i].d_arrived);
     dfree(g->prod[i].d_scratch);
     dfree(g->prod[i].d_stage);
     dfree(g->prod[i].d_comp);
