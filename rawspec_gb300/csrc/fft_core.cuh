@@ -165,11 +165,17 @@ __host__ __device__ constexpr int bitrev(int x, int bits) {
 }
 
 // In-register DFT over the RP elements v[off + s*STRIDE] (RP <= 32), natural
-// order in and out.  tw: the pass's twiddle entries for this butterfly,
-// `tstride` apart (entry i of stage L = 2: i = 0; of stage L >= 4: i = L/4 +
-// q, q < L/4); TW = false: no input factors.
-template <int RP, int STRIDE, bool TW, typename E, int R>
-__device__ __forceinline__ void dft_subset(cx<E> (&v)[R], int off, const float2* __restrict__ tw, int tstride) {
+// order in and out.  tw(i): twiddle entry i of the pass for this butterfly
+// (stage L = 2: i = 0; stage L >= 4: i = L/4 + q, q < L/4); NoTwiddle: no
+// input factors.
+struct NoTwiddle {};
+struct TableTwiddle {  // entries `stride` apart
+  const float2* __restrict__ p;
+  int stride;
+  __device__ __forceinline__ float2 operator()(int i) const { return p[i * stride]; }
+};
+template <int RP, int STRIDE, typename Tw, typename E, int R>
+__device__ __forceinline__ void dft_subset(cx<E> (&v)[R], int off, const Tw& tw) {
   if constexpr (RP > 1) {
     constexpr int LOG = ilog2(RP);
     cx<E> t[RP];
@@ -178,11 +184,11 @@ __device__ __forceinline__ void dft_subset(cx<E> (&v)[R], int off, const float2*
 #pragma unroll
     for (int l = 1; l <= LOG; ++l) {
       const int len = 1 << l, half = len >> 1;
-      if constexpr (TW) {
+      if constexpr (!std::is_same_v<Tw, NoTwiddle>) {
         const int nq = len >= 4 ? len / 4 : 1;
 #pragma unroll
         for (int q = 0; q < nq; ++q) {
-          const float2 ct = tw[(len >= 4 ? len / 4 + q : 0) * tstride];
+          const float2 ct = tw(len >= 4 ? len / 4 + q : 0);
 #pragma unroll
           for (int i = 0; i < RP; i += len) {
             bfly_tab(t[i + q], t[i + q + half], ct, false);
@@ -283,7 +289,7 @@ struct GroupFFT {
 
   template <bool BIASED>
   static __device__ __forceinline__ void first_pass(cx<E> (&v)[R]) {
-    dft_subset<R, 1, false>(v, 0, nullptr, 0);
+    dft_subset<R, 1>(v, 0, NoTwiddle{});
     if constexpr (BIASED) {
       v[0].re = esubk(v[0].re, R * kCodeBias);
       v[0].im = esubk(v[0].im, R * kCodeBias);
@@ -308,7 +314,7 @@ struct GroupFFT {
           first_pass<BIASED>(v);
         } else {
           const int k = j & (Ns - 1);
-          dft_subset<R, 1, true>(v, 0, tw + stockham_tw_offset(N, R, p) + k, Ns);
+          dft_subset<R, 1>(v, 0, TableTwiddle{tw + stockham_tw_offset(N, R, p) + k, Ns});
         }
         const bool last = (p == S::FULL - 1) && (S::RLAST == 1);
         if (!last) {
@@ -360,7 +366,7 @@ struct GroupFFT {
         constexpr int NSL = N / RL;
         const float2* twl = tw + stockham_tw_offset(N, R, S::FULL) + j;
 #pragma unroll
-        for (int qb = 0; qb < Q; ++qb) dft_subset<RL, Q, true>(v, qb, twl + qb * T, NSL);
+        for (int qb = 0; qb < Q; ++qb) dft_subset<RL, Q>(v, qb, TableTwiddle{twl + qb * T, NSL});
       }
     }
   }

@@ -185,8 +185,7 @@ cudaError_t large_prepare(const LargeLaunch& L);
 // launch; each launch leaves them zeroed for the next, the error word apart).
 bool large_fused_supported(const LargeLaunch& L);
 cudaError_t large_fused_plan(LargeLaunch& L);
-int large_fused_row_radix(int pol);  // radix of the row tiles (twiddle table of twN1)
-int large_fused_col_radix();         // radix of the column tiles (tables twN2 and twM)
+int large_fused_radix(const LargeLaunch& L);  // radix of its tiles (twiddle tables twN1, twN2 and twM)
 int large_fused_ctl_ints(const LargeLaunch& L);
 int large_fused_twj_entries(const LargeLaunch& L);  // size of the twJ table
 cudaError_t large_fused_prepare(LargeLaunch& L);

@@ -44,7 +44,18 @@ namespace rsg {
 
 namespace {
 
-constexpr int kFusedTPB = 256;
+// Values per thread and CTA size.  With columns of 1024 points (2^19, 2^20),
+// 32 values per thread: one exchange per transform instead of two, by CTAs of
+// 128 threads (two an SM, 255 registers).  2^20 points, 256 MiB buffer: 16
+// values and 256 threads 698 us total power and 1010 four planes, 32 and 128
+// 626 and 961 (16 and 128: 712 and 1271).  Shorter columns would leave a warp
+// less than a block of ring rows to store (2^16 points, four planes: 825 us
+// with 16 and 256, 1122 with 32 and 128; 2^19 in four planes 855 and 884),
+// 2048 points two rows to a CTA.
+__host__ __device__ constexpr int fused_radix(int N1, int N2, int pol) {
+  return N2 == 1024 && (N1 == 1024 || (N1 == 512 && pol == POL_TP)) ? 32 : 16;
+}
+__host__ __device__ constexpr int fused_tpb(int N1, int N2, int pol) { return fused_radix(N1, N2, pol) == 32 ? 128 : 256; }
 // Row tiles of slab s are queued after the column tiles of slab s + lag, and
 // a slot of the intermediate ring is reused `ring` slabs later (ring > lag
 // keeps every wait pointed at earlier items).  Both distances are chosen at
@@ -68,20 +79,6 @@ static_assert(fused_k<POL_TP>() >= 2 && fused_k<POL_FULL>() >= 2, "an item must 
 constexpr long long kSpinLimit = 1ll << 24;         // polls of a counter (~2 s with back-off)
 constexpr long long kMbarCycles = 4000000000ll;     // ~2 s of SM clocks for a stage copy
 
-// Radix (values per thread per transform) of the column and row tiles.
-#ifndef RSG_FUSED_RA
-#define RSG_FUSED_RA 16
-#endif
-#ifndef RSG_FUSED_RB_TP
-#define RSG_FUSED_RB_TP 16
-#endif
-#ifndef RSG_FUSED_RB_X
-#define RSG_FUSED_RB_X 16
-#endif
-__host__ __device__ constexpr int fused_ra() { return RSG_FUSED_RA; }
-template <int POL>
-__host__ __device__ constexpr int fused_rb() { return POL == POL_TP ? RSG_FUSED_RB_TP : RSG_FUSED_RB_X; }
-
 // Shared-memory distance between the exchange buffers of neighbouring
 // interleaved sub-FFTs, chosen so that the C sub-FFTs served by one
 // half-warp land on disjoint banks, and even (16-byte aligned rows for the
@@ -98,8 +95,9 @@ __host__ __device__ constexpr int round16(int x) { return (x + 15) & ~15; }
 
 template <int N1, int N2, int POL>
 struct FusedCfg {
-  static constexpr int RA = fused_ra(), TA = N2 / RA, CA = kFusedTPB / TA;
-  static constexpr int RB = fused_rb<POL>(), TB = N1 / RB, CB = kFusedTPB / TB;
+  static constexpr int TPB = fused_tpb(N1, N2, POL);
+  static constexpr int RA = fused_radix(N1, N2, POL), TA = N2 / RA, CA = TPB / TA;
+  static constexpr int RB = RA, TB = N1 / RB, CB = TPB / TB;
   static constexpr int TWA = stockham_tw_size(N2, RA), TWB = stockham_tw_size(N1, RB);
   static constexpr int GSA = group_stride(N2, CA), GSB = group_stride(N1, CB);
   // column-tile words: boxes of BOXR rows x CW words (CW >= 4: 16-byte rows)
@@ -131,7 +129,7 @@ struct FusedCfg {
   static constexpr unsigned BYTES_A = (unsigned)N2 * CW * 4;
   static constexpr unsigned BYTES_TW = (unsigned)(TA + RA) * CA * 8;
   static constexpr unsigned BYTES_B = (unsigned)CB * N1 * 8;
-  static_assert(TA * CA == kFusedTPB && TB * CB == kFusedTPB, "sub-FFT threads must tile the CTA");
+  static_assert(TA * CA == TPB && TB * CB == TPB, "sub-FFT threads must tile the CTA");
   static_assert((size_t)BYTES_A <= (size_t)XCH * sizeof(float2), "column words must fit a stage buffer");
   static_assert(N2 % BOXR == 0 && CA % 2 == 0, "tensor boxes must tile the column");
   static_assert(N1 % (2 * BOXO) == 0, "output boxes must not straddle the FFT shift");
@@ -350,7 +348,7 @@ __device__ __forceinline__ Item decode_item(long long item, int S, int lag, int 
 // transforms, F::TMA_OUT); otherwise per-thread stores (and loads of the
 // accumulator in accumulate mode).
 template <int N1, int N2, int POL, bool TOUT>
-__global__ void __launch_bounds__(kFusedTPB, 2)
+__global__ void __launch_bounds__(fused_tpb(N1, N2, POL), 2)
 k_large_fused(const __grid_constant__ LargeLaunch a) {
   using F = FusedCfg<N1, N2, POL>;
   static_assert(!TOUT || F::TMA_OUT, "tensor-store outputs need one plane and 16-byte rows");
@@ -393,8 +391,8 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
     s_abort = 0;
     s_issued[0] = s_issued[1] = 0;
   }
-  for (int i = tid; i < F::TWA; i += kFusedTPB) twA[i] = a.twN2[i];
-  for (int i = tid; i < F::TWB; i += kFusedTPB) twB[i] = a.twN1[i];
+  for (int i = tid; i < F::TWA; i += F::TPB) twA[i] = a.twN2[i];
+  for (int i = tid; i < F::TWB; i += F::TPB) twB[i] = a.twN1[i];
   __syncthreads();
 
   // Stage copies (issued by thread 0).  Column stage t of an item: the C_A
@@ -505,15 +503,13 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
         cpair v[R];
 #pragma unroll
         for (int m = 0; m < R; ++m) {
-          float2 smp[2];
-          Unpack<FMT_I8, 2>::run(words[(j + T * m) * F::CW], smp);
-          v[m] = pack2(smp[0], smp[1]);
+          v[m] = unpack_biased(words[(j + T * m) * F::CW]);
         }
         __syncthreads();  // the buffer becomes the exchange buffer; tile t-1 is done
         if (t > 0) refill(t - 1);
         const float2 w0 = tw[j * C + col];  // W_N^(n1 j)
         float2* dst = scr;
-        GroupFFT<N2, R, 2>::template run_packed<true>(v, j, sb + (size_t)col * F::GSA, 0, twA, Sync{});
+        GroupFFT<N2, R, 2>::template run_packed<true, true>(v, j, sb + (size_t)col * F::GSA, 0, twA, Sync{});
 #pragma unroll
         for (int m = 0; m < R; ++m) {
           const int k2 = j + m * T;
@@ -600,13 +596,13 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
             const char* blk = reinterpret_cast<const char*>(scr + (size_t)2 * tile * C * N1);
             constexpr int kLines = 2 * F::BYTES_B / 128;
 #pragma unroll 1
-            for (int l = tid; l < kLines; l += kFusedTPB) discard_l2(blk + (size_t)l * 128);
+            for (int l = tid; l < kLines; l += F::TPB) discard_l2(blk + (size_t)l * 128);
           } else {
             const char* rows0 = reinterpret_cast<const char*>(scr + (size_t)tile * C * N1);
             const char* rows1 = reinterpret_cast<const char*>(scr + ((size_t)N2 + (size_t)tile * C) * N1);
             constexpr int kLines = F::BYTES_B / 128;
 #pragma unroll 1
-            for (int l = tid; l < kLines; l += kFusedTPB) {
+            for (int l = tid; l < kLines; l += F::TPB) {
               discard_l2(rows0 + (size_t)l * 128);
               discard_l2(rows1 + (size_t)l * 128);
             }
@@ -706,7 +702,7 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
   __syncthreads();
   if (s_last) {
     __threadfence();
-    for (int i = tid; i < 1 + 2 * S; i += kFusedTPB) next[i] = 0;
+    for (int i = tid; i < 1 + 2 * S; i += F::TPB) next[i] = 0;
     if (tid == 0) *exited = 0;
     __threadfence();
   }
@@ -732,7 +728,7 @@ cudaError_t fused_t(const LargeLaunch& L, cudaStream_t s, int mode_op, int* ctas
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kFusedTPB, F::SMEM);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, F::TPB, F::SMEM);
     if (e != cudaSuccess) return e;
     *ctas_out = std::max(1, per_sm) * sms;
     return cudaSuccess;
@@ -749,7 +745,7 @@ cudaError_t fused_t(const LargeLaunch& L, cudaStream_t s, int mode_op, int* ctas
     ctas_out[8] = fused_k<POL>();
     return cudaSuccess;
   }
-  k<<<L.fused_ctas, kFusedTPB, F::SMEM, s>>>(L);
+  k<<<L.fused_ctas, F::TPB, F::SMEM, s>>>(L);
   return cudaGetLastError();
 }
 
@@ -828,9 +824,7 @@ cudaError_t large_fused_plan(LargeLaunch& L) {
   return L.ring > L.lag ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-int large_fused_row_radix(int pol) { return pol == POL_TP ? fused_rb<POL_TP>() : fused_rb<POL_FULL>(); }
-
-int large_fused_col_radix() { return fused_ra(); }
+int large_fused_radix(const LargeLaunch& L) { return fused_radix(1 << L.logN1, 1 << L.logN2, L.pol); }
 
 int large_fused_ctl_ints(const LargeLaunch& L) { return 3 + 2 * L.Nc * L.Nss; }
 
@@ -855,7 +849,7 @@ cudaError_t encode_2d(CUtensorMap* map, const void* base, CUtensorMapDataType ty
 }  // namespace
 
 int large_fused_twj_entries(const LargeLaunch& L) {
-  return (1 << L.logN1) * ((1 << L.logN2) / fused_ra());
+  return (1 << L.logN1) * ((1 << L.logN2) / large_fused_radix(L));
 }
 
 cudaError_t large_fused_prepare(LargeLaunch& L) {

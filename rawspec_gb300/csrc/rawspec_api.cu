@@ -866,8 +866,8 @@ int plan_device_bytes(const rawspec_context* ctx, bool expanded, int sm_count, s
       }
       t += sf * sizeof(float2) + pf * sizeof(float);
       const int n1 = 1 << L.logN1, n2 = 1 << L.logN2;
-      const int RA = fused ? large_fused_col_radix() : large_pass_a_radix();
-      const int RB = fused ? large_fused_row_radix(pol) : large_pass_b_radix(pol);
+      const int RA = fused ? large_fused_radix(L) : large_pass_a_radix();
+      const int RB = fused ? large_fused_radix(L) : large_pass_b_radix(pol);
       const size_t ta = (size_t)stockham_table_size(n2, RA), tb = (size_t)stockham_table_size(n1, RB);
       const size_t nlo = (size_t)1 << L.h, nhi = (size_t)1 << (L.logN - L.h), nm = (size_t)RA * n1;
       const size_t nj = fused ? (size_t)large_fused_twj_entries(L) : 0;
@@ -1151,8 +1151,8 @@ int rawspec_initialize(rawspec_context* ctx) {
       if (sf && dev_alloc(g, &P.d_scratch, sf * sizeof(float2))) FAIL();
       if (pf && dev_alloc(g, &P.d_partial, pf * sizeof(float))) FAIL();
       const int n1 = 1 << L.logN1, n2 = 1 << L.logN2;
-      const int RA = P.fused ? large_fused_col_radix() : large_pass_a_radix();
-      const int RB = P.fused ? large_fused_row_radix(pol) : large_pass_b_radix(pol);
+      const int RA = P.fused ? large_fused_radix(L) : large_pass_a_radix();
+      const int RB = P.fused ? large_fused_radix(L) : large_pass_b_radix(pol);
       // tables at 256-byte aligned offsets (the fused kernel copies twM and
       // twJ with the tensor copy engine)
       auto al = [](size_t n) { return (n + 31) & ~size_t(31); };
