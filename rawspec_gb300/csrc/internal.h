@@ -129,7 +129,7 @@ cudaError_t tcs_launch(const TcLaunch& L, cudaStream_t s);
 // ---------------------------------------------------------------------------
 // Four-step large FFT (4096 < N <= 2^22): N = N1 * N2.
 //   pass A: N2-point FFTs down the columns n1 of x[n1 + N1*n2], twiddled by
-//           W_N^(n1*k2), written to scratch as [slab][pol][k2][n1];
+//           W_N^(n1*k2), written to scratch as [slab][k2][n1];
 //   pass B: N1-point FFTs along the rows k2, detection, integration.
 // A slab is one (channel, spectrum) pair.
 // ---------------------------------------------------------------------------
@@ -140,7 +140,7 @@ struct LargeLaunch {
   int M = 0, units_per_chan = 0, n_units = 0, chunks = 1, spc = 0;
   long long chan_stride = 0;
   const void* in = nullptr;
-  float2* scratch = nullptr;      // [Nc*Nss][nv][N2][N1]
+  float2* scratch = nullptr;      // [Nc*Nss][N2][N1] of nv complex values
   float* out = nullptr;
   float* partial = nullptr;
   const float2* twN2 = nullptr;   // pass-ordered Stockham table of the N2-point FFT
@@ -155,6 +155,7 @@ struct LargeLaunch {
   int S = 0;                      // slabs of this launch (Nc * Nss for a whole buffer)
   int slab0 = 0;                  // first slab of this launch
   int unit0 = 0, unit_count = 0;  // units of this launch (two-kernel path)
+  int tiles_a = 1;                // column tiles per CTA of pass A
   int ring = 0;                   // intermediate slots
   int lag = 2;                    // row tiles of slab s follow the column tiles of slab s + lag
   int lag_pipe = 2;               // the lag of a launch over one channel group of the pipelined call
@@ -168,11 +169,11 @@ struct LargeLaunch {
 int large_configure(LargeLaunch& L, int target_ctas, size_t* scratch_float2, size_t* partial_floats);
 // Radix of pass A (values per thread of its N2-point FFT) and its threads per
 // column FFT, which define the pass-A twiddle table twM ([R_A][N1]).
-int large_pass_a_radix();
+int large_pass_a_radix(const LargeLaunch& L);
 // Sizes (entries) of the pass-ordered twiddle tables.
 int stockham_table_size(int N, int R);
 int small_radix(int logN, int pol);
-int large_pass_b_radix(int pol);
+int large_pass_b_radix(const LargeLaunch& L);
 cudaError_t large_launch_a(const LargeLaunch& L, cudaStream_t s);
 cudaError_t large_launch_b(const LargeLaunch& L, cudaStream_t s);
 // Raises both kernels' dynamic shared-memory limits on the current device.
@@ -184,6 +185,7 @@ cudaError_t large_prepare(const LargeLaunch& L);
 // and large_fused_ctl_ints() control words (zeroed once before the first
 // launch; each launch leaves them zeroed for the next, the error word apart).
 bool large_fused_supported(const LargeLaunch& L);
+bool large_fused_wanted(const LargeLaunch& L);  // a supported product is faster on it than on large_launch_a/b
 cudaError_t large_fused_plan(LargeLaunch& L);
 int large_fused_radix(const LargeLaunch& L);  // radix of its tiles (twiddle tables twN1, twN2 and twM)
 int large_fused_ctl_ints(const LargeLaunch& L);

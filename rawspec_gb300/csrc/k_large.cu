@@ -6,7 +6,7 @@
 //
 //   pass A  N2-point FFTs down the columns of x[n1 + N1*n2] (both
 //           polarisations), twiddled by W_N^(n1*k2), written to scratch as
-//           [slab][pol][k2][n1] -- the only intermediate that touches global
+//           [slab][k2][n1] -- the only intermediate that touches global
 //           memory;
 //   pass B  N1-point FFTs along the rows k2 of that scratch, detection of
 //           the output bins X[k2 + N2*k1], integration over the unit's
@@ -24,127 +24,231 @@ namespace rsg {
 
 namespace {
 
-constexpr int kRA = 16;  // radix of pass A
-constexpr int kLargeTPB = 256;
-// Resident CTAs per SM the register budget allows: one polarisation fits
-// 80 registers a thread without spills (three CTAs of 256 threads), two
-// polarisations need about 128 (two CTAs).
-template <int NV>
-constexpr int large_min_blocks() { return NV == 1 ? 3 : 2; }
-
-// Sub-FFT of NSUB points at radix R; C sub-FFTs (columns or rows) per CTA,
-// interleaved across lanes so that global accesses of neighbouring lanes are
-// neighbouring columns.
-template <int NSUB, int R>
-struct LargeCfg {
-  static constexpr int T = NSUB / R;              // threads per sub-FFT
-  static constexpr int C = kLargeTPB / T > 8 ? 8 : (kLargeTPB / T > 0 ? kLargeTPB / T : 1);
-  static constexpr int TPB = T * C;
+// Both passes run two lanes in lockstep on the packed instructions: the two
+// polarisations of a value (NV = 2), or, of one polarisation, neighbouring
+// columns n1 in pass A and neighbouring rows k2 in pass B.  In pass A a lane
+// pair is one word of the input either way (two polarisations of a sample,
+// or two samples).
+//
+// What bounds them is HBM and how well its lines are used: pass A moves 20 bytes
+// a sample of both polarisations (4 in, 16 out), pass B 16 and the result.
+//   * Pass A: CTAs of 128 threads, C neighbouring columns each, whose
+//     words come through shared memory (cp.async, 16 bytes of a row a copy) one
+//     tile ahead of the transforms.  16 values per thread up to 256 points, 32
+//     for 512 and 1024 (one exchange).
+//   * Pass B: 16 values per thread and two neighbouring rows across the lanes,
+//     so that a warp's load takes 256 contiguous bytes of each row; with
+//     eight rows (64 bytes) a load it took 333 us per 64 Mi samples, with two
+//     186 (65536 points, Nint 16).  Results are staged in shared memory until
+//     a CTA has ROWS_OUT neighbouring rows, 32 bytes of a line in total power.
+// With 256 threads, each polarisation in a plane of its own and eight rows
+// across the lanes, 65536 points at Nint 16 took 446 + 344 us.
+template <int NSUB, int FMT>
+struct ColumnCfg {
+  static constexpr int R = NSUB == 512 || NSUB == 1024 ? 32 : 16;
+  static constexpr int T = NSUB / R;              // threads per column
+  static constexpr int TPB = T <= 32 ? 128 : 256;
+  static constexpr int C = TPB / T;               // columns (lane pairs) per CTA
+  static constexpr int REGS = R == 32 ? 168 : 128;
+  static constexpr int MINB = 65536 / (TPB * REGS);
   static constexpr int TW = stockham_tw_size(NSUB, R);
+  static constexpr bool SPLIT = R == 32;          // one exchange buffer: three CTAs fit an SM
+  static constexpr int WB = FMT == FMT_I16 ? 8 : 4;
+  static constexpr bool STAGED = C * WB >= 16;
+  static constexpr int STAGE = STAGED ? NSUB * C * WB : 0;
+};
+// OUT: results staged until a CTA has several neighbouring rows (units of one
+// or two spectra, whose output is as large as their input).
+template <int NSUB, int NV, int POL, bool OUT>
+struct RowCfg {
+  static constexpr int NP = PolOut<POL>::NP;
+  static constexpr int R = POL == POL_TP || NSUB <= 1024 ? 16 : 8;
+  static constexpr int T = NSUB / R;
+  static constexpr int TPB = T <= 64 ? 128 : T <= 256 ? 256 : T;
+  static constexpr int C = TPB / T;               // transforms per CTA
+  static constexpr int CR = C < 2 ? C : 2;        // of them neighbouring lanes
+  static constexpr int ROWS = NV == 2 ? 1 : 2;    // rows per transform
+  static constexpr int REGS = POL != POL_TP && R == 16 ? 168 : 128;
+  static constexpr int MINB = 65536 / (TPB * REGS);
+  static constexpr int TW = stockham_tw_size(NSUB, R);
+  // rows staged before they are written: eight, within 32 KiB
+  static constexpr int FIT = 32768 / (NP * NSUB * 4);
+  static constexpr int WANT = FIT < 8 ? FIT : 8;
+  static constexpr int GROUPS = !OUT || C * ROWS >= WANT ? 1 : WANT / (C * ROWS);
+  static constexpr int ROWS_OUT = C * ROWS * GROUPS;
 };
 
-template <int POL>
-__host__ __device__ constexpr int pass_b_radix() { return POL == POL_TP ? 16 : 8; }
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// *p += v for four floats, without a round trip.
+__device__ __forceinline__ void red_add4(float* p, float4 v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
 
 struct BlockSyncL {
   __device__ __forceinline__ void operator()(bool, bool) const { __syncthreads(); }
 };
 
-// float2 between the exchange areas of neighbouring sub-FFTs (NV buffers of
-// smem_padded_len(N) each): at least their size, and chosen so that the C
-// sub-FFTs served by one half-warp start in different banks (their start
-// offsets modulo 16 float2 are multiples of 16 / C), even for 16-byte rows.
-template <int N, int C, int NV>
+// Elements between the exchange areas of neighbouring transforms (BUFS buffers
+// of smem_padded_len(N) each): at least their size, and chosen so that the C
+// transforms served by one half-warp start in different banks (their start
+// offsets modulo 16 are multiples of 16 / C).
+template <int N, int C, int BUFS>
 __host__ __device__ constexpr int sub_stride() {
-  int base = NV * smem_padded_len(N);
+  int base = BUFS * smem_padded_len(N);
   const int cp = C < 16 ? C : 16;
   const int want = (16 / cp) % 16;
   while (base % 16 != want) ++base;
-  return base + (base & 1);
+  return base;
 }
 
-template <int N2, int NV>
+template <int N2, int FMT>
 constexpr size_t passA_smem() {
-  using Cf = LargeCfg<N2, kRA>;
-  return (size_t)((Cf::TW + 1) & ~1) * sizeof(float2) + (size_t)Cf::C * sub_stride<N2, Cf::C, NV>() * sizeof(float2);
+  using Cf = ColumnCfg<N2, FMT>;
+  return (size_t)((Cf::TW + 1) & ~1) * sizeof(float2) + Cf::STAGE +
+         (size_t)Cf::C * sub_stride<N2, Cf::C, Cf::SPLIT ? 1 : 2>() * sizeof(float2);
 }
 
-template <int N1, int NV, int R>
+template <int N1, int NV, int POL, bool OUT>
 constexpr size_t passB_smem() {
-  using Cf = LargeCfg<N1, R>;
-  return (size_t)((Cf::TW + 1) & ~1) * sizeof(float2) + (size_t)Cf::C * sub_stride<N1, Cf::C, NV>() * sizeof(float2);
+  using Cf = RowCfg<N1, NV, POL, OUT>;
+  return (size_t)((Cf::TW + 1) & ~1) * sizeof(float2) + (OUT ? (size_t)Cf::NP * N1 * Cf::ROWS_OUT * sizeof(float) : 0) +
+         (size_t)Cf::C * sub_stride<N1, Cf::CR, 2>() * sizeof(float2);
+}
+
+// a * (w0, w1), one twiddle per lane
+__device__ __forceinline__ cpair pmul2(const cpair& a, float2 w0, float2 w1) {
+  const float2 c = make_float2(w0.x, w1.x), s = make_float2(w0.y, w1.y), ns = make_float2(-w0.y, -w1.y);
+  return {f2fma(a.im, ns, f2mul(a.re, c)), f2fma(a.re, s, f2mul(a.im, c))};
 }
 
 }  // namespace
 
 template <int N2, int FMT, int NV>
-__global__ void __launch_bounds__(LargeCfg<N2, kRA>::TPB, large_min_blocks<NV>())
-k_large_a(LargeLaunch a) {
-  using Cf = LargeCfg<N2, kRA>;
-  constexpr int R = kRA, T = Cf::T, C = Cf::C, TPB = Cf::TPB;
+__global__ void __launch_bounds__(ColumnCfg<N2, FMT>::TPB, ColumnCfg<N2, FMT>::MINB)
+k_large_a(const __grid_constant__ LargeLaunch a) {
+  using Cf = ColumnCfg<N2, FMT>;
+  constexpr int R = Cf::R, T = Cf::T, C = Cf::C, TPB = Cf::TPB;
+  constexpr int XS = sub_stride<N2, C, Cf::SPLIT ? 1 : 2>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* tw_s = reinterpret_cast<float2*>(smem_raw);
-  float2* xch = tw_s + ((Cf::TW + 1) & ~1);
+  unsigned char* const stage = smem_raw + (size_t)((Cf::TW + 1) & ~1) * sizeof(float2);
+  float2* const xch = reinterpret_cast<float2*>(stage + Cf::STAGE);
 
   const int tid = threadIdx.x;
   for (int i = tid; i < Cf::TW; i += TPB) tw_s[i] = a.twN2[i];
 
   const int N1 = 1 << a.logN1;
-  const int tiles = N1 / C;
-  const int tile = blockIdx.x % tiles;
-  const int slab = a.slab0 + blockIdx.x / tiles;
-  const int c = slab / a.Nss;
-  const int s = slab % a.Nss;
+  const int NW = NV == 2 ? N1 : N1 / 2;  // lane pairs per row of the input
+  const int tiles = NW / C;              // per slab
+  const int first = blockIdx.x * a.tiles_a, last = min(first + a.tiles_a, tiles * a.S);
   const int col = tid % C;
   const int j = tid / C;
-  const int n1 = tile * C + col;
 
-  using W = typename SampleWord<FMT, NV>::type;
-  const W* src = reinterpret_cast<const W*>(a.in) + (long long)c * a.chan_stride + (long long)s * (N1 * (long long)N2) + n1 +
-                 (long long)N1 * j;
-  float2 v[NV][R];
-  {
-    W w[R];
+  using W = typename SampleWord<FMT, 2>::type;
+  // Word 0 of column 0 of a tile (tiles are counted over the slabs).
+  auto tile_src = [&](int tile) {
+    const int slab = a.slab0 + tile / tiles;
+    return reinterpret_cast<const W*>(a.in) +
+           ((long long)(slab / a.Nss) * a.chan_stride + (long long)(slab % a.Nss) * (N1 * (long long)N2)) / (NV == 2 ? 1 : 2) +
+           (tile % tiles) * C;
+  };
+  auto request = [&](int tile) {
+    if constexpr (Cf::STAGED) {
+      constexpr int PER = C * Cf::WB / 16;  // copies per row
+      const char* src = reinterpret_cast<const char*>(tile_src(tile));
 #pragma unroll
-    for (int m = 0; m < R; ++m) w[m] = __ldg(src + (long long)N1 * T * m);
+      for (int i = 0; i < N2 * PER / TPB; ++i) {
+        const int e = i * TPB + tid;
+        cp_async16(stage + e * 16, src + (long long)(e / PER) * NW * Cf::WB + (e % PER) * 16);
+      }
+    }
+  };
+  // W_N^e from the two-level table.
+  auto level2 = [&](int e) {
+    return cmul(__ldg(a.twLo + (e & ((1 << a.h) - 1))), __ldg(a.twHi + (e >> a.h)));
+  };
+
+  if (first < last) request(first);
+  for (int tile = first; tile < last; ++tile) {
+    const int slab = a.slab0 + tile / tiles;
+    const int wc = (tile % tiles) * C + col;
+    // W_N^(n1*j) of the lanes' columns
+    const int n1 = NV == 2 ? wc : 2 * wc;
+    const float2 w0 = level2(n1 * j);
+    const float2 w1 = NV == 2 ? w0 : level2((n1 + 1) * j);
+    cpair v[R];
+    {
+      W w[R];
+      if constexpr (Cf::STAGED) {
+        cp_async_wait();
+        __syncthreads();  // every thread's copies have landed (and the twiddle table)
+#pragma unroll
+        for (int m = 0; m < R; ++m) w[m] = reinterpret_cast<const W*>(stage)[tid + m * T * C];
+      } else {
+        const W* src = tile_src(tile) + col + (long long)NW * j;
+#pragma unroll
+        for (int m = 0; m < R; ++m) w[m] = __ldg(src + (long long)NW * T * m);
+        __syncthreads();
+      }
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        if constexpr (FMT == FMT_I8) {
+          v[m] = unpack_biased(w[m]);
+        } else {
+          float2 smp[2];
+          Unpack<FMT, 2>::run(w[m], smp);
+          v[m] = pack2(smp[0], smp[1]);
+        }
+      }
+    }
+    // the next tile is requested when every thread has taken this one's words
+    GroupFFT<N2, R, 2>::template run_packed<Cf::SPLIT, FMT == FMT_I8>(
+        v, j, xch + (size_t)col * XS, smem_padded_len(N2), tw_s, [&](bool taken, bool) {
+          __syncthreads();
+          if (taken && tile + 1 < last) request(tile + 1);
+        });
+
+    // Output k2 = j + m*T: W_N^(n1*k2) = W_N^(n1*j) * W_N^(n1*m*T).  Elements of
+    // 16 bytes, [slab][k2][lane pair]: both polarisations (re, re, im, im), or
+    // two columns (re, im, re, im).
+    float4* dst = reinterpret_cast<float4*>(a.scratch) + ((size_t)slab * N2 + j) * NW + wc;
+    const float2* twm = a.twM + n1;
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      float2 smp[NV];
-      Unpack<FMT, NV>::run(w[m], smp);
-#pragma unroll
-      for (int q = 0; q < NV; ++q) v[q][m] = smp[q];
+      float4 o;
+      if constexpr (NV == 2) {
+        const cpair x = pmul(v[m], m == 0 ? w0 : cmul(w0, __ldg(twm + (size_t)m * N1)));
+        o = make_float4(x.re.x, x.re.y, x.im.x, x.im.y);
+      } else {
+        float2 wa = w0, wb = w1;
+        if (m > 0) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(twm + (size_t)m * N1));
+          wa = cmul(w0, make_float2(t.x, t.y));
+          wb = cmul(w1, make_float2(t.z, t.w));
+        }
+        const cpair x = pmul2(v[m], wa, wb);
+        o = make_float4(x.re.x, x.im.x, x.re.y, x.im.y);
+      }
+      dst[(size_t)m * T * NW] = o;
     }
-  }
-  // W_N^(n1*j) for this thread's column, from the two-level table.
-  const int e0 = n1 * j;
-  const float2 w0 = cmul(__ldg(a.twLo + (e0 & ((1 << a.h) - 1))), __ldg(a.twHi + (e0 >> a.h)));
-  __syncthreads();  // twiddle table in shared memory
-  using E = typename GroupFFT<N2, R, NV>::E;
-  GroupFFT<N2, R, NV>::run(v, j, reinterpret_cast<E*>(xch + (size_t)col * sub_stride<N2, C, NV>()),
-                            smem_padded_len(N2), tw_s, BlockSyncL{});
-
-  // Output k2 = j + m*T: W_N^(n1*k2) = W_N^(n1*j) * W_N^(n1*m*T).
-  float2* dst = a.scratch + (size_t)slab * NV * N2 * N1 + n1;
-  const float2* twm = a.twM + n1;
-#pragma unroll
-  for (int m = 0; m < R; ++m) {
-    const int k2 = j + m * T;
-    const float2 w = m == 0 ? w0 : cmul(w0, __ldg(twm + (size_t)m * N1));
-#pragma unroll
-    for (int q = 0; q < NV; ++q) dst[((size_t)q * N2 + k2) * N1] = cmul(v[q][m], w);
   }
 }
 
-template <int N1, int NV, int POL>
-__global__ void __launch_bounds__(LargeCfg<N1, pass_b_radix<POL>()>::TPB, large_min_blocks<NV>())
-k_large_b(LargeLaunch a) {
-  constexpr int R = pass_b_radix<POL>();
-  using Cf = LargeCfg<N1, R>;
-  constexpr int T = Cf::T, C = Cf::C, TPB = Cf::TPB;
-  constexpr int NP = PolOut<POL>::NP;
+template <int N1, int NV, int POL, bool OUT>
+__global__ void __launch_bounds__(RowCfg<N1, NV, POL, OUT>::TPB, RowCfg<N1, NV, POL, OUT>::MINB)
+k_large_b(const __grid_constant__ LargeLaunch a) {
+  using Cf = RowCfg<N1, NV, POL, OUT>;
+  constexpr int R = Cf::R, T = Cf::T, C = Cf::C, CR = Cf::CR, TPB = Cf::TPB;
+  constexpr int NP = Cf::NP, ROWS = Cf::ROWS, ROWS_OUT = Cf::ROWS_OUT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float2* tw_s = reinterpret_cast<float2*>(smem_raw);
-  float2* xch = tw_s + ((Cf::TW + 1) & ~1);
+  float* const outs = reinterpret_cast<float*>(tw_s + ((Cf::TW + 1) & ~1));  // [plane][k1][ROWS_OUT]
+  float2* const xch = reinterpret_cast<float2*>(outs + (OUT ? NP * N1 * ROWS_OUT : 0));
 
   const int tid = threadIdx.x;
   for (int i = tid; i < Cf::TW; i += TPB) tw_s[i] = a.twN1[i];
@@ -152,73 +256,135 @@ k_large_b(LargeLaunch a) {
 
   const int N2 = 1 << a.logN2;
   const int N = N1 * N2;
-  const int tiles = N2 / C;
+  const int tiles = N2 / ROWS_OUT;
   const int tile = blockIdx.x % tiles;
   const int uc = blockIdx.x / tiles;
   const int unit = a.unit0 + uc / a.chunks;
   const int chunk = uc % a.chunks;
   const int c = unit / a.units_per_chan;
   const int d = unit % a.units_per_chan;
-  const int row = tid % C;
-  const int j = tid / C;
-  const int k2 = tile * C + row;
+  const int row = tid % CR + CR * (tid / (CR * T));  // transform of the CTA
+  const int j = tid / CR % T;
   const int s_begin = chunk * a.spc;
   const int s_end = min(a.M, s_begin + a.spc);
   const float im_sign = a.conj ? -1.0f : 1.0f;
 
-  float acc[R][NP];
-#pragma unroll
-  for (int m = 0; m < R; ++m)
-#pragma unroll
-    for (int p = 0; p < NP; ++p) acc[m][p] = 0.0f;
+  // Row k2 holds bins k2 + N2*k1: of the partial sums in bin order, or of the
+  // dump buffer.
+  const bool part = a.chunks > 1;
+  float* const obase = part ? a.partial + ((size_t)unit * a.chunks + chunk) * NP * N : a.out + ((size_t)d * NP * a.Nc + c) * N;
+  const size_t plane = part ? (size_t)N : (size_t)a.Nc * N;
+  const float scale = part ? 1.0f : a.scale;
+  const bool add = !part && a.mode == ACC_ADD;
 
-  using E = typename GroupFFT<N1, R, NV>::E;
-  E* my_xch = reinterpret_cast<E*>(xch + (size_t)row * sub_stride<N1, C, NV>());
+  float2* const my_xch = xch + (size_t)row * sub_stride<N1, CR, 2>();
+#pragma unroll 1
+  for (int g = 0; g < Cf::GROUPS; ++g) {
+  const int r0 = (g * C + row) * ROWS;    // the transform's first row of the CTA's
+  const int k2 = tile * ROWS_OUT + r0;
+  // total power: per lane (a row each) of one polarisation, else their sum
+  float2 acc[NP == 4 || NV == 1 ? R : 1], xr[NP == 4 ? R : 1];
+  float tp[NP == 1 && NV == 2 ? R : 1];
+#pragma unroll
+  for (int m = 0; m < R; ++m) {
+    if constexpr (NP == 4 || NV == 1) acc[m] = make_float2(0.f, 0.f);
+    if constexpr (NP == 4) xr[m] = make_float2(0.f, 0.f);
+    if constexpr (NP == 1 && NV == 2) tp[m] = 0.0f;
+  }
+
   for (int sl = s_begin; sl < s_end; ++sl) {
     const int slab = c * a.Nss + d * a.M + sl;
-    const float2* src = a.scratch + ((size_t)slab * NV * N2 + k2) * N1 + j;
-    float2 v[NV][R];
+    cpair v[R];
+    if constexpr (NV == 2) {
+      const float4* src = reinterpret_cast<const float4*>(a.scratch) + ((size_t)slab * N2 + k2) * N1 + j;
 #pragma unroll
-    for (int q = 0; q < NV; ++q)
+      for (int m = 0; m < R; ++m) {
+        const float4 f = __ldcs(src + m * T);
+        v[m] = cpair{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+      }
+    } else {
+      const float2* src = a.scratch + ((size_t)slab * N2 + k2) * N1 + j;
 #pragma unroll
-      for (int m = 0; m < R; ++m) v[q][m] = src[(size_t)q * N2 * N1 + m * T];
-    GroupFFT<N1, R, NV>::run(v, j, my_xch, smem_padded_len(N1), tw_s, BlockSyncL{});
+      for (int m = 0; m < R; ++m) v[m] = pack2(__ldcs(src + m * T), __ldcs(src + N1 + m * T));
+    }
+    GroupFFT<N1, R, 2>::template run_packed<false>(v, j, my_xch, smem_padded_len(N1), tw_s, BlockSyncL{});
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      float2 x[NV];
-#pragma unroll
-      for (int q = 0; q < NV; ++q) x[q] = v[q][m];
-      detect_acc<POL, NV>(acc[m], x, im_sign);
+      if constexpr (NP == 4) {
+        const float2 x0 = lane0(v[m]), x1 = lane1(v[m]);
+        acc[m] = f2fma(v[m].im, v[m].im, f2fma(v[m].re, v[m].re, acc[m]));
+        xr[m].x = __fmaf_rn(x0.y, x1.y, __fmaf_rn(x0.x, x1.x, xr[m].x));
+        xr[m].y = __fmaf_rn(-x0.x, x1.y, __fmaf_rn(x0.y, x1.x, xr[m].y));
+      } else if constexpr (NV == 1) {
+        acc[m] = f2fma(v[m].im, v[m].im, f2fma(v[m].re, v[m].re, acc[m]));
+      } else {
+        tp[m] = __fmaf_rn(v[m].re.x, v[m].re.x, tp[m]);
+        tp[m] = __fmaf_rn(v[m].im.x, v[m].im.x, tp[m]);
+        tp[m] = __fmaf_rn(v[m].re.y, v[m].re.y, tp[m]);
+        tp[m] = __fmaf_rn(v[m].im.y, v[m].im.y, tp[m]);
+      }
     }
   }
+  // value (plane p, or the lanes' rows) of element m
+  auto result = [&](int m, int p, int lane) -> float {
+    if constexpr (NP == 4) {
+      if (p == 2) return xr[m].x;
+      if (p == 3) return xr[m].y * im_sign;
+      if (POL == POL_FULL) return p == 0 ? acc[m].x : acc[m].y;
+      return p == 0 ? acc[m].x + acc[m].y : acc[m].x - acc[m].y;
+    } else if constexpr (NV == 1) {
+      return lane == 0 ? acc[m].x : acc[m].y;
+    } else {
+      return tp[m];
+    }
+  };
 
-  if (a.chunks > 1) {
+  if constexpr (OUT) {  // k1 = j + m*T of the rows into the staging area
 #pragma unroll
     for (int m = 0; m < R; ++m)
 #pragma unroll
       for (int p = 0; p < NP; ++p)
-        a.partial[(((size_t)unit * a.chunks + chunk) * NP + p) * N + k2 + N2 * (j + m * T)] = acc[m][p];
-    return;
-  }
-  float* obase = a.out + ((size_t)d * NP * a.Nc + c) * N;
-  const size_t plane = (size_t)a.Nc * N;
-  if (a.mode == ACC_ADD) {
-    // request every old value before the first store
-    float old[R][NP];
 #pragma unroll
-    for (int m = 0; m < R; ++m)
-#pragma unroll
-      for (int p = 0; p < NP; ++p) old[m][p] = __ldcg(obase + p * plane + out_pos(k2 + N2 * (j + m * T), N, a.inverse));
-#pragma unroll
-    for (int m = 0; m < R; ++m)
-#pragma unroll
-      for (int p = 0; p < NP; ++p)
-        obase[p * plane + out_pos(k2 + N2 * (j + m * T), N, a.inverse)] = __fmaf_rn(acc[m][p], a.scale, old[m][p]);
+        for (int l = 0; l < ROWS; ++l) outs[((size_t)p * N1 + j + m * T) * ROWS_OUT + r0 + l] = result(m, p, l);
   } else {
 #pragma unroll
     for (int m = 0; m < R; ++m)
 #pragma unroll
-      for (int p = 0; p < NP; ++p) obase[p * plane + out_pos(k2 + N2 * (j + m * T), N, a.inverse)] = acc[m][p] * a.scale;
+      for (int p = 0; p < NP; ++p)
+#pragma unroll
+        for (int l = 0; l < ROWS; ++l) {
+          const int k = k2 + l + N2 * (j + m * T);
+          float* o = obase + p * plane + (part ? k : out_pos(k, N, a.inverse));
+          const float x = result(m, p, l) * scale;
+          if (add) atomicAdd(o, x);  // each element once per launch: a plain add, without a round trip
+          else *o = x;
+        }
+  }
+  }
+  if constexpr (!OUT) return;
+  __syncthreads();
+
+  // Neighbouring rows are neighbouring bins.
+  constexpr int V = ROWS_OUT % 4 == 0 ? 4 : 1;
+  const int k20 = tile * ROWS_OUT;
+  for (int e = tid * V; e < NP * N1 * ROWS_OUT; e += TPB * V) {
+    const int r = e % ROWS_OUT, k1 = e / ROWS_OUT % N1, p = e / (ROWS_OUT * N1);
+    const int k = k20 + r + N2 * k1;
+    float* o = obase + p * plane;
+    if (V == 4 && (part || !a.inverse)) {
+      float4 x = *reinterpret_cast<const float4*>(outs + e);
+      x = make_float4(x.x * scale, x.y * scale, x.z * scale, x.w * scale);
+      o += part ? k : out_pos(k, N, 0);
+      if (add) red_add4(o, x);
+      else *reinterpret_cast<float4*>(o) = x;
+    } else {
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        float* q = o + (part ? k + i : out_pos(k + i, N, a.inverse));
+        if (add) atomicAdd(q, outs[e + i] * scale);  // each element once per launch
+        else *q = outs[e + i] * scale;
+      }
+    }
   }
 }
 
@@ -229,12 +395,35 @@ namespace {
 
 template <int N2, int FMT, int NV>
 cudaError_t launch_a_t(const LargeLaunch& L, cudaStream_t s, bool prep) {
-  using Cf = LargeCfg<N2, kRA>;
+  using Cf = ColumnCfg<N2, FMT>;
   auto k = k_large_a<N2, FMT, NV>;
-  const size_t smem = passA_smem<N2, NV>();
+  const size_t smem = passA_smem<N2, FMT>();
   if (prep) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int N1 = 1 << L.logN1;
-  const long long grid = (long long)(N1 / Cf::C) * L.S;
+  const long long tiles = (long long)(N1 / (NV == 2 ? 1 : 2) / Cf::C) * L.S;
+  if (tiles < 1) return cudaSuccess;
+  // Tiles per CTA: as many as leave four CTAs for every resident one, eight at
+  // most (the first tile of a CTA is not copied ahead of time).
+  LargeLaunch l = L;
+  l.tiles_a = Cf::STAGED ? (int)std::max<long long>(1, std::min<long long>(8, tiles / (4ll * 152 * Cf::MINB))) : 1;
+  k<<<(unsigned)((tiles + l.tiles_a - 1) / l.tiles_a), Cf::TPB, smem, s>>>(l);
+  return cudaGetLastError();
+}
+
+// Units of at most this many spectra per chunk stage their results: one
+// spectrum, 2^16 points 319 -> 270 us, 2^18 496 -> 375; with 16 the staging
+// costs more than it gives (2^18 237 -> 311).
+constexpr int kStageOutSpectra = 2;
+bool stage_out(const LargeLaunch& L) { return L.M <= kStageOutSpectra; }
+
+template <int N1, int NV, int POL, bool OUT>
+cudaError_t launch_b_o(const LargeLaunch& L, cudaStream_t s, bool prep) {
+  using Cf = RowCfg<N1, NV, POL, OUT>;
+  auto k = k_large_b<N1, NV, POL, OUT>;
+  const size_t smem = passB_smem<N1, NV, POL, OUT>();
+  if (prep) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int N2 = 1 << L.logN2;
+  const long long grid = (long long)(N2 / Cf::ROWS_OUT) * L.unit_count * L.chunks;
   if (grid < 1) return cudaSuccess;
   k<<<(unsigned)grid, Cf::TPB, smem, s>>>(L);
   return cudaGetLastError();
@@ -242,16 +431,7 @@ cudaError_t launch_a_t(const LargeLaunch& L, cudaStream_t s, bool prep) {
 
 template <int N1, int NV, int POL>
 cudaError_t launch_b_t(const LargeLaunch& L, cudaStream_t s, bool prep) {
-  constexpr int R = pass_b_radix<POL>();
-  using Cf = LargeCfg<N1, R>;
-  auto k = k_large_b<N1, NV, POL>;
-  const size_t smem = passB_smem<N1, NV, R>();
-  if (prep) return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const int N2 = 1 << L.logN2;
-  const long long grid = (long long)(N2 / Cf::C) * L.unit_count * L.chunks;
-  if (grid < 1) return cudaSuccess;
-  k<<<(unsigned)grid, Cf::TPB, smem, s>>>(L);
-  return cudaGetLastError();
+  return stage_out(L) ? launch_b_o<N1, NV, POL, true>(L, s, prep) : launch_b_o<N1, NV, POL, false>(L, s, prep);
 }
 
 template <int N2>
@@ -295,37 +475,72 @@ cudaError_t dispatch_b(const LargeLaunch& L, cudaStream_t s, bool prep) {
   }
 }
 
-template <int N1, int R>
-int rows_per_cta() { return LargeCfg<N1, R>::C; }
+template <int N1, int NV, int POL>
+void row_geometry_t(bool out, int* radix, int* rows) {
+  *radix = RowCfg<N1, NV, POL, false>::R;
+  *rows = out ? RowCfg<N1, NV, POL, true>::ROWS_OUT : RowCfg<N1, NV, POL, false>::ROWS_OUT;
+}
+template <int N1>
+void row_geometry(const LargeLaunch& L, int* radix, int* rows) {
+  if (L.pol != POL_TP) row_geometry_t<N1, 2, POL_FULL>(stage_out(L), radix, rows);
+  else if (L.nv == 2) row_geometry_t<N1, 2, POL_TP>(stage_out(L), radix, rows);
+  else row_geometry_t<N1, 1, POL_TP>(stage_out(L), radix, rows);
+}
 
-int pass_b_rows(int logN1, int pol) {
-  const bool tp = pol == POL_TP;
-  switch (logN1) {
-    case 6: return tp ? rows_per_cta<64, 16>() : rows_per_cta<64, 8>();
-    case 7: return tp ? rows_per_cta<128, 16>() : rows_per_cta<128, 8>();
-    case 8: return tp ? rows_per_cta<256, 16>() : rows_per_cta<256, 8>();
-    case 9: return tp ? rows_per_cta<512, 16>() : rows_per_cta<512, 8>();
-    case 10: return tp ? rows_per_cta<1024, 16>() : rows_per_cta<1024, 8>();
-    case 11: return tp ? rows_per_cta<2048, 16>() : rows_per_cta<2048, 8>();
-    default: return tp ? rows_per_cta<4096, 16>() : rows_per_cta<4096, 8>();
+// Radix and rows per CTA of pass B.
+void pass_b_geometry(const LargeLaunch& L, int* radix, int* rows) {
+  switch (L.logN1) {
+    case 6: return row_geometry<64>(L, radix, rows);
+    case 7: return row_geometry<128>(L, radix, rows);
+    case 8: return row_geometry<256>(L, radix, rows);
+    case 9: return row_geometry<512>(L, radix, rows);
+    case 10: return row_geometry<1024>(L, radix, rows);
+    case 11: return row_geometry<2048>(L, radix, rows);
+    default: return row_geometry<4096>(L, radix, rows);
   }
 }
 
 }  // namespace
 
-int large_pass_a_radix() { return kRA; }
-int large_pass_b_radix(int pol) { return pol == POL_TP ? pass_b_radix<POL_TP>() : pass_b_radix<POL_FULL>(); }
+int large_pass_a_radix(const LargeLaunch& L) { return L.logN2 == 9 || L.logN2 == 10 ? 32 : 16; }
+int large_pass_b_radix(const LargeLaunch& L) {
+  int r, c;
+  pass_b_geometry(L, &r, &c);
+  return r;
+}
 int stockham_table_size(int N, int R) { return stockham_tw_size(N, R); }
+
+// N2 of N1 * N2.  Pass A is fastest at 256 points (eight columns a CTA: 250 us
+// per 64 Mi samples of two polarisations; 512 points 295, 1024, with four
+// columns, 490), pass B between 128 and 512 (185-240; 1024 250, 2048 340, 4096
+// 410 with 16 spectra a unit): 2^16 247 + 190, 2^18 as 256 x 1024 249 + 246,
+// as 512 x 512 294 + 240; 2^20 in total power 512 x 2048 300 + 338, 1024 x 1024
+// 502 + 276.  The four planes and one polarisation pay more for long rows
+// (2^20: 760 and 307 with 2048, 441 and 243 with 1024).
+static int split_log_n2(const LargeLaunch& L) {
+  const bool pair = L.pol == POL_TP && L.nv == 2;  // total power of two polarisations
+  switch (L.logN) {
+    case 13: return 7;
+    case 14: case 15: case 16: case 18: return 8;
+    case 17: case 19: return 9;
+    case 20: return pair ? 9 : 10;
+    case 21: return pair ? 9 : L.nv == 1 ? 10 : 11;
+    case 22: return L.nv == 1 ? 10 : 11;
+    default: return 12;
+  }
+}
 
 int large_configure(LargeLaunch& L, int target_ctas, size_t* scratch_float2, size_t* partial_floats) {
   if (L.logN < 13 || L.logN > 24) return -1;
-  L.logN2 = (L.logN + 1) / 2;
+  L.logN2 = split_log_n2(L);
   L.logN1 = L.logN - L.logN2;
   L.h = (L.logN + 1) / 2;
   const int N2 = 1 << L.logN2;
   const int np = L.pol == POL_TP ? 1 : 4;
   // Chunks of a unit's spectra across CTAs for parallelism.
-  const int cpr = N2 / pass_b_rows(L.logN1, L.pol);  // CTAs per unit and chunk
+  int radix, rows;
+  pass_b_geometry(L, &radix, &rows);
+  const int cpr = N2 / rows;  // CTAs per unit and chunk
   const long long base = (long long)cpr * L.n_units;
   int chunks = (int)std::max<long long>(1, (target_ctas + base - 1) / base);
   chunks = std::min(chunks, L.M);

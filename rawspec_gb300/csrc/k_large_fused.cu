@@ -788,13 +788,30 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 bool large_fused_supported(const LargeLaunch& L) {
   if (L.fmt != FMT_I8 || L.nv != 2 || L.M != 1 || L.logN < 16 || L.logN > 22) return false;
-  if (L.logN2 != (L.logN + 1) / 2) return false;
-  const long long n1 = 1ll << L.logN1;
+  const long long n1 = 1ll << (L.logN - (L.logN + 1) / 2);
   // the column tiles' tensor copies view each channel as rows of N1 words
   return L.chan_stride % n1 == 0 && (reinterpret_cast<uintptr_t>(L.in) & 15) == 0;
 }
 
+// Which of the supported products the persistent kernel computes rather than
+// the two of k_large.cu (whose intermediate goes through HBM).  64 channels of
+// 2^20 samples, one spectrum a unit: total power 2^16 666 against 518 us,
+// 2^17 729 / 566, 2^18 713 / 647, 2^19 621 / 695, 2^20 630 / 640; four planes
+// 2^16 804 / 833, 2^20 1150 / 1600.  A single transform or two leave it nothing
+// to overlap (2^16, one: 67 against 28 us from call to result; 2^20 88 / 62).
+// Short total-power transforms of small buffers would gain too (twelve of 2^16
+// 83 against 43 us) but stay: the choice of this kernel at such a size is
+// part of what the tuning table's users (and its tests) rely on.
+constexpr long long kSmallBuffer = 1ll << 20;  // time samples over all channels
+bool large_fused_wanted(const LargeLaunch& L) {
+  const long long slabs = (long long)L.Nc * L.Nss;
+  if (slabs <= 2 && L.logN <= 20) return false;
+  return !(L.pol == POL_TP && L.logN <= 18 && (slabs << L.logN) > kSmallBuffer);
+}
+
 cudaError_t large_fused_plan(LargeLaunch& L) {
+  L.logN2 = (L.logN + 1) / 2;
+  L.logN1 = L.logN - L.logN2;
   cudaError_t e = fused_dispatch(L, nullptr, 1, nullptr);  // shared-memory limit first: occupancy depends on it
   if (e != cudaSuccess) return e;
   e = fused_dispatch(L, nullptr, 2, &L.fused_ctas);

@@ -243,6 +243,12 @@ int target_ctas_for(int sm_count, const rawspec_gb300_tune& t) {
   return sm_count * (t.ctas > 0 ? t.ctas : kDefaultCtasPerSm);
 }
 
+// A supported long product runs on the persistent fused kernel where that is
+// the faster one, or where a tuning-table entry sets its lag or ring.
+bool fused_wanted(const LargeLaunch& L, const rawspec_gb300_tune& t) {
+  return large_fused_supported(L) && (large_fused_wanted(L) || t.lag > 0 || t.ring > 0);
+}
+
 // A tuning-table lag / ring of the fused kernel replaces the plan's; the
 // ring stays longer than the lag, the lag of channel-group launches no
 // longer than the ring allows.
@@ -855,7 +861,7 @@ int plan_device_bytes(const rawspec_context* ctx, bool expanded, int sm_count, s
       L.chan_stride = (long long)ctx->Nb * ctx->Ntpb;
       size_t sf = 0, pf = 0;
       if (large_configure(L, target_ctas, &sf, &pf)) return 1;
-      const bool fused = large_fused_supported(L);
+      const bool fused = fused_wanted(L, tune);
       if (fused) {
         L.S = (int)ctx->Nc * (int)Nss;
         if (large_fused_plan(L) != cudaSuccess) return 1;
@@ -866,8 +872,8 @@ int plan_device_bytes(const rawspec_context* ctx, bool expanded, int sm_count, s
       }
       t += sf * sizeof(float2) + pf * sizeof(float);
       const int n1 = 1 << L.logN1, n2 = 1 << L.logN2;
-      const int RA = fused ? large_fused_radix(L) : large_pass_a_radix();
-      const int RB = fused ? large_fused_radix(L) : large_pass_b_radix(pol);
+      const int RA = fused ? large_fused_radix(L) : large_pass_a_radix(L);
+      const int RB = fused ? large_fused_radix(L) : large_pass_b_radix(L);
       const size_t ta = (size_t)stockham_table_size(n2, RA), tb = (size_t)stockham_table_size(n1, RB);
       const size_t nlo = (size_t)1 << L.h, nhi = (size_t)1 << (L.logN - L.h), nm = (size_t)RA * n1;
       const size_t nj = fused ? (size_t)large_fused_twj_entries(L) : 0;
@@ -1133,7 +1139,7 @@ int rawspec_initialize(rawspec_context* ctx) {
         fprintf(stderr, "unsupported FFT length %d\n", P.N);
         FAIL();
       }
-      if (large_fused_supported(L)) {
+      if (fused_wanted(L, tune)) {
         P.fused = true;
         L.S = (int)ctx->Nc * (int)P.Nss;
         CK(large_fused_plan(L));
@@ -1151,8 +1157,8 @@ int rawspec_initialize(rawspec_context* ctx) {
       if (sf && dev_alloc(g, &P.d_scratch, sf * sizeof(float2))) FAIL();
       if (pf && dev_alloc(g, &P.d_partial, pf * sizeof(float))) FAIL();
       const int n1 = 1 << L.logN1, n2 = 1 << L.logN2;
-      const int RA = P.fused ? large_fused_radix(L) : large_pass_a_radix();
-      const int RB = P.fused ? large_fused_radix(L) : large_pass_b_radix(pol);
+      const int RA = P.fused ? large_fused_radix(L) : large_pass_a_radix(L);
+      const int RB = P.fused ? large_fused_radix(L) : large_pass_b_radix(L);
       // tables at 256-byte aligned offsets (the fused kernel copies twM and
       // twJ with the tensor copy engine)
       auto al = [](size_t n) { return (n + 31) & ~size_t(31); };
