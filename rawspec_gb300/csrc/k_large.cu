@@ -15,6 +15,7 @@
 //
 // X[k2 + N2 k1] = sum_n1 W_N1^(n1 k1) W_N^(n1 k2) sum_n2 x[n1 + N1 n2] W_N2^(n2 k2).
 #include <algorithm>
+#include <cmath>
 
 #include "detect.cuh"
 #include "fft_core.cuh"
@@ -520,8 +521,8 @@ int stockham_table_size(int N, int R) { return stockham_tw_size(N, R); }
 static int split_log_n2(const LargeLaunch& L) {
   const bool pair = L.pol == POL_TP && L.nv == 2;  // total power of two polarisations
   switch (L.logN) {
-    case 13: return 7;
-    case 14: case 15: case 16: case 18: return 8;
+    case 13: case 14: return 7;
+    case 15: case 16: case 18: return 8;
     case 17: case 19: return 9;
     case 20: return pair ? 9 : 10;
     case 21: return pair ? 9 : L.nv == 1 ? 10 : 11;
@@ -537,13 +538,26 @@ int large_configure(LargeLaunch& L, int target_ctas, size_t* scratch_float2, siz
   L.h = (L.logN + 1) / 2;
   const int N2 = 1 << L.logN2;
   const int np = L.pol == POL_TP ? 1 : 4;
-  // Chunks of a unit's spectra across CTAs for parallelism.
+  // Chunks of a unit's spectra across CTAs: where a unit's spectra one after
+  // another (about 1.5 us each in a CTA) would take longer than the pass's
+  // traffic, by more than the sum of the partials costs (a launch and its
+  // traffic: 21 channels x 16384 points, Nint 8: whole units 39 us, halves
+  // 35 + 14; 8 channels, Nint 32: whole 50, quarters 23 + 6).
   int radix, rows;
   pass_b_geometry(L, &radix, &rows);
-  const int cpr = N2 / rows;  // CTAs per unit and chunk
-  const long long base = (long long)cpr * L.n_units;
-  int chunks = (int)std::max<long long>(1, (target_ctas + base - 1) / base);
-  chunks = std::min(chunks, L.M);
+  const long long base = (long long)(N2 / rows) * L.n_units;  // CTAs per chunk
+  const double bytes = (double)L.n_units * L.M * ((size_t)8 * L.nv << L.logN);
+  const double partial_us = (double)L.n_units * np * ((size_t)8 << L.logN) / 4e6;
+  int chunks = 1;
+  double best = 1e300;
+  for (int c = 1; c <= L.M && (c == 1 || base * c <= 2ll * target_ctas); ++c) {
+    const double serial = std::ceil((double)L.M / c) * 1.5 * std::max(1.0, (double)base * c / target_ctas);
+    const double t = std::max(bytes / 5.5e6, serial) + (c > 1 ? 6.0 + c * partial_us : 0.0);
+    if (t < best * 0.95) {
+      best = t;
+      chunks = c;
+    }
+  }
   L.spc = (L.M + chunks - 1) / chunks;
   L.chunks = (L.M + L.spc - 1) / L.spc;
   *scratch_float2 = (size_t)L.Nc * L.Nss * L.nv * ((size_t)1 << L.logN);
