@@ -102,7 +102,7 @@ struct TcLaunch {
   float* out = nullptr;          // [units_per_chan][|P|][Nc][N], FFT-shifted
   float* partial = nullptr;      // [n_units][chunks][|P|][N] (chunks > 1)
   const void* tab = nullptr;     // tc_table_bytes(logN) bytes from tc_table_fill
-  int* err = nullptr;            // set to 1 if a bounded wait for the tensor cores timed out
+  int* err = nullptr;            // pinned host word, set to 1 if a bounded wait for the tensor cores timed out
   int mode = ACC_WRITE, inverse = 0, conj = 0;
   float scale = 1.0f;
   int unit0 = 0, unit_count = 0;
@@ -159,7 +159,8 @@ struct LargeLaunch {
   int ring = 0;                   // intermediate slots
   int lag = 2;                    // row tiles of slab s follow the column tiles of slab s + lag
   int lag_pipe = 2;               // the lag of a launch over one channel group of the pipelined call
-  int* ctl = nullptr;             // [0] error, [1] CTAs finished, [2] item counter, [3..3+S) A done, [3+S..3+2S) B done
+  int* ctl = nullptr;             // [0] CTAs finished, [1] item counter, [2..2+S) A done, [2+S..2+2S) B done
+  int* err = nullptr;             // pinned host word: code of a bounded wait that ran out
   int fused_ctas = 0;             // persistent grid size
   // fused kernel: tensor maps of the input (rows of N1 words), of the
   // twiddle tables twJ and twM and of the dump buffer (rows of N2 floats)
@@ -183,7 +184,7 @@ cudaError_t large_prepare(const LargeLaunch& L);
 // spectrum.  large_fused_plan() sets the grid size, the lag and the number of
 // intermediate slabs (ring); the launch needs ring * 2 * N float2 of scratch
 // and large_fused_ctl_ints() control words (zeroed once before the first
-// launch; each launch leaves them zeroed for the next, the error word apart).
+// launch; each launch leaves them zeroed for the next).
 bool large_fused_supported(const LargeLaunch& L);
 bool large_fused_wanted(const LargeLaunch& L);  // a supported product is faster on it than on large_launch_a/b
 cudaError_t large_fused_plan(LargeLaunch& L);

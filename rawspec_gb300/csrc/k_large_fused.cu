@@ -163,7 +163,7 @@ __device__ __forceinline__ int load_acquire(const int* p) {
 // wait, finishes its current work item on whatever the buffers hold (all
 // accesses stay in bounds), drains the copies already in flight and exits.
 __device__ __forceinline__ void set_abort(int* err, int code, int* abort_flag) {
-  atomicExch(err, code);
+  atomicExch_system(err, code);
   *reinterpret_cast<volatile int*>(abort_flag) = 1;
 }
 __device__ __forceinline__ bool aborted(const int* abort_flag) {
@@ -373,11 +373,11 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
   static_assert(tilesA % K == 0 && tilesB % K == 0, "items must cover whole tiles");
   constexpr int itemsA = tilesA / K, itemsB = tilesB / K;
   const long long total = (long long)S * (itemsA + itemsB);
-  int* err = a.ctl;  // sticky error word (never reset by a launch)
-  int* exited = a.ctl + 1;  // CTAs of this launch that have finished
-  int* next = a.ctl + 2;
-  int* doneA = a.ctl + 3;
-  int* doneB = a.ctl + 3 + S;
+  int* err = a.err;         // error word in host memory (never reset by a launch)
+  int* exited = a.ctl;      // CTAs of this launch that have finished
+  int* next = a.ctl + 1;
+  int* doneA = a.ctl + 2;
+  int* doneB = a.ctl + 2 + S;
   const float im_sign = a.conj ? -1.0f : 1.0f;
   const unsigned long long pol_first = policy_evict_first();
   const unsigned long long pol_last = policy_evict_last();
@@ -688,11 +688,11 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
   // mbarrier complete in order, so the earlier ones are then complete too).
   if (tid == 0) {
     for (int b = 0; b < 2; ++b)
-      if (s_issued[b] > 0 && !mbar_wait_bounded(&mbar[b], (s_issued[b] - 1) & 1u)) atomicExch(err, 4);
+      if (s_issued[b] > 0 && !mbar_wait_bounded(&mbar[b], (s_issued[b] - 1) & 1u)) atomicExch_system(err, 4);
   }
   if (TOUT && tid == 0) bulk_wait_all();
   // The last CTA to finish zeroes the counters for the next launch (every
-  // other CTA has stopped reading them); the error word stays.
+  // other CTA has stopped reading them).
   __shared__ int s_last;
   __syncthreads();
   if (tid == 0) {
@@ -843,7 +843,7 @@ cudaError_t large_fused_plan(LargeLaunch& L) {
 
 int large_fused_radix(const LargeLaunch& L) { return fused_radix(1 << L.logN1, 1 << L.logN2, L.pol); }
 
-int large_fused_ctl_ints(const LargeLaunch& L) { return 3 + 2 * L.Nc * L.Nss; }
+int large_fused_ctl_ints(const LargeLaunch& L) { return 2 + 2 * L.Nc * L.Nss; }
 
 namespace {
 

@@ -15,6 +15,7 @@
 // Nothing but the raw voltages is read and nothing but integrated spectra is
 // written.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "detect.cuh"
@@ -527,6 +528,36 @@ int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitC
   return best;
 }
 
+// Resident CTAs per SM of the configuration and SMs of the current device, with
+// the kernel's dynamic shared-memory limit raised; asked of the runtime once
+// per configuration and device (it takes longer than a small launch).  0
+// CTAs if it cannot say.
+void resident_ctas(const SmallLaunch& L, int* occ, int* sms) {
+  constexpr int kDevices = 64, kConfigs = 13 * 2 * 4;
+  static std::atomic<int> known[kDevices][kConfigs];  // occ + 1
+  static std::atomic<int> known_sms[kDevices];
+  *occ = *sms = 0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return;
+  const int mode = L.nv == 1 ? 0 : L.pol == POL_FULL ? 1 : L.pol == POL_STOKES ? 2 : 3;
+  const int key = (L.logN * 2 + (L.fmt == FMT_I16 ? 1 : 0)) * 4 + mode;
+  const bool cached = dev < kDevices;
+  if (cached && known[dev][key].load() > 0) {
+    *occ = known[dev][key].load() - 1;
+    *sms = known_sms[dev].load();
+    return;
+  }
+  if (cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      small_dispatch(L, nullptr, 2, occ) != cudaSuccess) {
+    *occ = 0;
+    return;
+  }
+  if (cached) {
+    known_sms[dev].store(*sms);
+    known[dev][key].store(*occ + 1);
+  }
+}
+
 }  // namespace
 
 int small_radix(int logN, int pol) { return small_r(1 << logN, pol == POL_TP ? 1 : 4); }
@@ -548,11 +579,8 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   L.sets = G / gps;
   const int ublocks = (L.n_units + L.sets - 1) / L.sets;
   const int max_chunks = (turns + gps - 1) / gps;
-  // resident CTAs on the device
-  int occ = 0, sms = 0, dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
-      cudaSuccess || small_dispatch(L, nullptr, 2, &occ) != cudaSuccess)
-    occ = 0;
+  int occ = 0, sms = 0;
+  resident_ctas(L, &occ, &sms);
   // The split of `units` units: spectra per chunk, and the chunks that makes.
   auto split = [&](int units, int* spc, int* chunks) {
     const int ub = (units + L.sets - 1) / L.sets;

@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(TcCfg<S>::THREADS, TcCfg<S>::MINB) k_tc(const 
   __syncthreads();
   tc::fence_after_sync();
   if (warp == 0) tc::tmem_dealloc(tmem, C::TMEM_COLS);
-  if (bad) atomicExch(a.err, 1);
+  if (bad) atomicExch_system(a.err, 1);
 }
 
 // Plan-time tables in the byte layout of the kernel's shared memory: the DFT

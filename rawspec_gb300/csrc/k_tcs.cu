@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(TcsCfg<N>::THREADS) k_tcs(const __grid_constan
   __syncthreads();
   tc::fence_after_sync();
   if (warp == 0) tc::tmem_dealloc(tmem, C::TMEM_COLS);
-  if (tid == 0 && *abort_flag) atomicExch(a.err, 1);
+  if (tid == 0 && *abort_flag) atomicExch_system(a.err, 1);
 }
 
 // The DFT operand in the byte layout of the kernel's shared memory: rows

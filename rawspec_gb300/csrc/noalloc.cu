@@ -6,8 +6,8 @@
 // other stream of the process), or a host framework that owns all device
 // memory through its own pool and budget.  This entry point takes the input
 // and output as caller-provided device pointers and keeps its only scratch --
-// the per-chunk partial sums of the fused small-FFT kernel, its twiddle table
-// and its arrival counters -- in the file-scope array below, which every GPU that loads the
+// the per-chunk partial sums of the fused small-FFT kernel, its twiddle tables
+// and its arrival counters -- in the file-scope arrays below, which every GPU that loads the
 // library holds until the process exits.
 #include <cstdint>
 #include <cstdio>
@@ -19,40 +19,83 @@
 namespace {
 
 constexpr size_t kPartialFloats = size_t(1) << 20;  // 4 MiB of partial sums
-constexpr int kMaxNt = 4096;                        // twiddle table capacity
+constexpr int kMaxLogNt = 12;
+constexpr int kMaxNt = 1 << kMaxLogNt;              // twiddle table capacity of one call
 constexpr int kArrivals = 8192;                     // arrival counters of split units, zero between calls
+constexpr int kTableEntries = 3 * kMaxNt;           // the tables of every FFT length and mode
 constexpr size_t kScratchFloats = kPartialFloats + 2 * (size_t)kMaxNt + kArrivals;
 constexpr int kMaxDevices = 64;
 
 }  // namespace
 
 // The shared scratch (zero when the library is loaded): partial sums [0,
-// kPartialFloats), twiddles after them, then the arrival counters.
+// kPartialFloats), one call's twiddles after them, then the arrival counters.
 static __device__ __align__(256) float g_noalloc_scratch[kScratchFloats];
+// Twiddle tables of every FFT length, for total power and for the four
+// planes, filled by the first call on a device outside a stream capture.
+static __device__ __align__(256) float2 g_noalloc_tables[kTableEntries];
 
 namespace {
 
 std::mutex g_mu;
 float* g_scratch_ptr[kMaxDevices] = {nullptr};
+float2* g_table_ptr[kMaxDevices] = {nullptr};
+bool g_tables_filled[kMaxDevices] = {false};
 
 // Device address of the scratch array on the current device, looked up once
 // per device.  In host code the array's name is only a host-side stand-in.
 // The address belongs to the device's primary context (the one the CUDA
 // runtime uses); it is not looked up again after cudaDeviceReset.
-float* scratch_for_current_device() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+float* scratch_for_device(int dev) {
   std::lock_guard<std::mutex> lock(g_mu);
   if (!g_scratch_ptr[dev]) {
     float* p = nullptr;
-    const cudaError_t rc = cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_noalloc_scratch);
+    float2* t = nullptr;
+    cudaError_t rc = cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_noalloc_scratch);
+    if (rc == cudaSuccess) rc = cudaGetSymbolAddress(reinterpret_cast<void**>(&t), g_noalloc_tables);
     if (rc != cudaSuccess) {
       fprintf(stderr, "rawspec_gb300_product_noalloc: cudaGetSymbolAddress failed: %s\n", cudaGetErrorName(rc));
       return nullptr;
     }
+    g_table_ptr[dev] = t;
     g_scratch_ptr[dev] = p;
   }
   return g_scratch_ptr[dev];
+}
+
+// The twiddle table of an FFT length and mode on the current device, or null
+// where it has to be filled for the call (a first call inside a stream
+// capture, or an error).  The first call outside one fills all of them and
+// waits for that: filling a call's own table was a launch of FP64 sines
+// before every call's kernel (14.3 of its 18 us at 5 channels x 256 points).
+const float2* twiddles_for(int dev, int logN, int pol, cudaStream_t s) {
+  using namespace rsg;
+  std::lock_guard<std::mutex> lock(g_mu);
+  int offset[2][kMaxLogNt + 1], total = 0;
+  for (int m = 0; m < 2; ++m)
+    for (int l = 0; l <= kMaxLogNt; ++l) {
+      offset[m][l] = total;
+      total += (stockham_table_size(1 << l, small_radix(l, m == 0 ? POL_TP : POL_FULL)) + 1) & ~1;
+    }
+  if (total > kTableEntries) return nullptr;
+  if (!g_tables_filled[dev]) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    cudaError_t e = cudaSuccess;
+    for (int m = 0; m < 2 && e == cudaSuccess; ++m)
+      for (int l = 0; l <= kMaxLogNt && e == cudaSuccess; ++l)
+        e = stockham_twiddle_fill(g_table_ptr[dev] + offset[m][l], 1 << l, small_radix(l, m == 0 ? POL_TP : POL_FULL), s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    g_tables_filled[dev] = true;
+  }
+  return g_table_ptr[dev] + offset[pol == POL_TP ? 0 : 1][logN];
 }
 
 bool pow2(unsigned x) { return x && !(x & (x - 1)); }
@@ -100,9 +143,10 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
             samples_per_channel / span);
     return 1;
   }
-  float* scratch = scratch_for_current_device();
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 1;
+  float* scratch = scratch_for_device(dev);
   if (!scratch) return 1;
-  float2* tw = reinterpret_cast<float2*>(scratch + kPartialFloats);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 
   const int npol = Npolout;
@@ -119,7 +163,6 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
   L.chan_stride = (long long)samples_per_channel;
   L.in = d_in;
   L.out = d_out;
-  L.tw = tw;
   L.partial = scratch;
   L.arrived = reinterpret_cast<unsigned*>(scratch + kPartialFloats + 2 * (size_t)kMaxNt);
   L.mode = ACC_WRITE;
@@ -129,8 +172,6 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
   L.scale = 1.0f / (snorm_d * snorm_d);
 
   int sms = 152;
-  int dev = 0;
-  cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // Units are split over CTAs only as far as the partial sums and the arrival
   // counters fit the scratch.
@@ -143,8 +184,13 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
     fprintf(stderr, "rawspec_gb300_product_noalloc: partial sums exceed the %zu-float scratch\n", kPartialFloats);
     return 1;
   }
-  cudaError_t e = stockham_twiddle_fill(tw, (int)Nt, small_radix(L.logN, L.pol), s);
-  if (e == cudaSuccess) e = small_prepare(L);
+  cudaError_t e = cudaSuccess;
+  L.tw = twiddles_for(dev, L.logN, L.pol, s);
+  if (!L.tw) {
+    float2* tw = reinterpret_cast<float2*>(scratch + kPartialFloats);
+    L.tw = tw;
+    e = stockham_twiddle_fill(tw, (int)Nt, small_radix(L.logN, L.pol), s);
+  }
   if (e == cudaSuccess) e = small_launch(L, s);
   if (e != cudaSuccess) {
     fprintf(stderr, "rawspec_gb300_product_noalloc: %s\n", cudaGetErrorName(e));

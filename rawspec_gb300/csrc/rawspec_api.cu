@@ -72,8 +72,9 @@ struct Product {
   int chunks = 1;
   bool fused = false;      // persistent fused four-step kernel
   bool tc = false;         // tensor-core DFT kernel instead of k_small
-  int* d_ctl = nullptr;    // control words of the fused kernel (error word first) or the tc error word
-  int* h_err = nullptr;    // pinned copy of the error word, refreshed after every fused or tc launch
+  int* d_ctl = nullptr;    // control words of the fused kernel
+  int* h_err = nullptr;    // error word of the fused and tc kernels: pinned host memory they write if a wait
+                           // runs out (a copy behind every launch cost a DMA operation each)
   float* d_partial = nullptr;  // per-chunk partial sums of this product
   unsigned* d_arrived = nullptr;  // k_small: arrival counters of its split units
   bool kahan = false;          // compensated integration across buffers
@@ -599,7 +600,6 @@ int launch_product(rawspec_context* ctx, GpuCtx* g, int i, int mode, int inverse
     if (L.chunks > 1 &&
         launch_finalize(ctx, g, P, out, L.unit0, L.unit_count, L.chunks, L.units_per_chan, mode, inverse, L.scale))
       return 1;
-    RSG_CUDA(cudaMemcpyAsync(P.h_err, P.d_ctl, sizeof(int), cudaMemcpyDeviceToHost, P.stream));
     return 0;
   }
   if (!P.large) {
@@ -638,9 +638,6 @@ int launch_product(rawspec_context* ctx, GpuCtx* g, int i, int mode, int inverse
         RSG_CUDA(large_fused_launch(L, P.stream));
         g->launches++;
       }
-      // the error word follows the launch to the host, so that a wait needs no
-      // synchronous copy
-      RSG_CUDA(cudaMemcpyAsync(P.h_err, P.d_ctl, sizeof(int), cudaMemcpyDeviceToHost, P.stream));
       return 0;
     }
     {
@@ -831,7 +828,7 @@ int plan_device_bytes(const rawspec_context* ctx, bool expanded, int sm_count, s
       L.n_units = (int)ctx->Nc * upc;
       size_t pf = 0;
       if (tc_configure(L, &pf, groups)) return 1;
-      t += pf * sizeof(float) + ((tc_table_bytes(logN) + 15) & ~size_t(15)) + sizeof(int);
+      t += pf * sizeof(float) + ((tc_table_bytes(logN) + 15) & ~size_t(15));
     } else if (!large) {
       SmallLaunch L;
       L.logN = logN;
@@ -1082,11 +1079,9 @@ int rawspec_initialize(rawspec_context* ctx) {
       if (dev_alloc(g, &P.d_tw, (tb + 15) & ~size_t(15))) FAIL();
       CK(tc_table_fill(P.d_tw, P.logN, g->stream));
       L.tab = P.d_tw;
-      if (dev_alloc(g, &P.d_ctl, sizeof(int))) FAIL();
-      CK(cudaMemsetAsync(P.d_ctl, 0, sizeof(int), g->stream));
       CK(pinned_alloc((void**)&P.h_err, sizeof(int)));
       *P.h_err = 0;
-      L.err = P.d_ctl;
+      L.err = P.h_err;
     } else if (!P.large) {
       SmallLaunch& L = P.sl;
       L.logN = P.logN;
@@ -1153,6 +1148,7 @@ int rawspec_initialize(rawspec_context* ctx) {
         CK(pinned_alloc((void**)&P.h_err, sizeof(int)));
         *P.h_err = 0;
         L.ctl = P.d_ctl;
+        L.err = P.h_err;
       }
       if (sf && dev_alloc(g, &P.d_scratch, sf * sizeof(float2))) FAIL();
       if (pf && dev_alloc(g, &P.d_partial, pf * sizeof(float))) FAIL();
@@ -1502,7 +1498,7 @@ int rawspec_wait_for_completion(rawspec_context* ctx) {
   if (cudaStreamSynchronize(g->stream) != cudaSuccess) return 1;
   for (unsigned i = 0; i < ctx->No; i++) {
     if (!g->prod[i].h_err) continue;
-    const int err = *g->prod[i].h_err;  // copied behind every fused or tc launch, ordered before the join
+    const int err = *static_cast<volatile int*>(g->prod[i].h_err);  // written before the launch that failed completed
     if (err) {
       if (g->prod[i].tc)
         fprintf(stderr, "rawspec: product %u: a bounded wait for the tensor cores timed out\n", i);
