@@ -218,6 +218,17 @@ struct Expand4Launch {
 };
 cudaError_t expand4_launch(const Expand4Launch& L, cudaStream_t s);
 
+// Corner turn of num_blocks page-locked host blocks into the device input
+// buffer, 4-bit samples expanded.
+constexpr int kGatherBlocks = 16;
+struct GatherLaunch {
+  const void* src[kGatherBlocks] = {};  // [Nc][row_bytes] each
+  void* dst = nullptr;                  // [Nc][Nb][row_bytes], twice that if expanded
+  long long row_bytes = 0;              // bytes of a channel in a host block
+  int Nc = 0, Nb = 0, dst_block = 0, num_blocks = 0, expand = 0;
+};
+cudaError_t gather_launch(const GatherLaunch& L, cudaStream_t s);
+
 // Weighted incoherent sum over antennas of FFT-shifted spectra:
 // ics[d][p][c][f] = sum_a w[a] * pwr[d][p][a*Nca + c][f] (sequential in a).
 struct IcsLaunch {

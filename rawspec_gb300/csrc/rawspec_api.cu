@@ -23,6 +23,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -101,6 +102,7 @@ struct EventPair {
 struct GpuCtx {
   int device = 0;
   int sm_count = 152;
+  std::vector<std::pair<const char*, const char*>> host_blocks;  // blocks this context page-locked, device addresses
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;     // host-to-device copies of the pipelined path
   cudaEvent_t ev_ready[kMaxCopyGroups] = {nullptr};  // per channel group: its copy has landed
@@ -791,6 +793,93 @@ int launch_deferred(std::vector<DeferredSmall>& d) {
   return 0;
 }
 
+// Copies of at most this many host bytes are done by a kernel, larger ones by
+// the copy engines.  The corner turn, one product and its dump, us: 0.5 MiB in
+// 8 blocks 53 by the engines, 23 by the kernel; 2 MiB in 8 blocks 52 and 35; 4
+// MiB in one block 58 and 48 with the call alone, 35 both ways back to back; 8
+// MiB 77 and 74, 55 both ways; 16 MiB 130 both ways: the link's rate.
+constexpr size_t kGatherBytes = size_t(8) << 20;
+
+// Queues the corner turn of a small copy as one kernel if it can be one: few
+// blocks, distinct destinations, and every block one that this context
+// page-locked (a caller may have put other memory in its place).  *done tells.
+int queue_gather(rawspec_context* ctx, GpuCtx* g, off_t src_idx, off_t dst_idx, size_t num_blocks, size_t row, bool expand,
+                 bool* done) {
+  *done = false;
+  if (num_blocks == 0 || num_blocks > (size_t)kGatherBlocks || num_blocks > ctx->Nb || src_idx < 0 || dst_idx < 0 ||
+      ctx->Nc > 65535 || row * ctx->Nc * num_blocks > kGatherBytes ||
+      row * (expand ? 2 : 1) * ctx->Nc * ctx->Nb > g->in_bytes)
+    return 0;
+  GatherLaunch L;
+  for (size_t b = 0; b < num_blocks; b++) {
+    const size_t i = (size_t)((src_idx + (off_t)b) % ctx->Nb_host);
+    if (i >= g->host_blocks.size() || !ctx->h_blkbufs[i] || g->host_blocks[i].first != ctx->h_blkbufs[i]) return 0;
+    L.src[b] = g->host_blocks[i].second;
+  }
+  L.dst = g->d_in;
+  L.row_bytes = (long long)row;
+  L.Nc = (int)ctx->Nc;
+  L.Nb = (int)ctx->Nb;
+  L.dst_block = (int)(dst_idx % ctx->Nb);
+  L.num_blocks = (int)num_blocks;
+  L.expand = expand ? 1 : 0;
+  ProfScope ps(g, RAWSPEC_GB300_K_H2D);
+  RSG_CUDA(gather_launch(L, g->stream));
+  g->launches++;
+  *done = true;
+  return 0;
+}
+
+// Queues the copy of num_blocks host blocks into the device buffer on the
+// context stream.
+int queue_copy(rawspec_context* ctx, GpuCtx* g, off_t src_idx, off_t dst_idx, size_t num_blocks) {
+  const size_t blk_chan = (size_t)ctx->Ntpb * ctx->Np * 2 * (ctx->Nbps / 8);
+  bool done = false;
+  if (queue_gather(ctx, g, src_idx, dst_idx, num_blocks, blk_chan, false, &done)) return 1;
+  if (done) return 0;
+  ProfScope ps(g, RAWSPEC_GB300_K_H2D);
+  for (size_t b = 0; b < num_blocks; b++) {
+    const off_t sblk = (src_idx + (off_t)b) % ctx->Nb_host;
+    const off_t dblk = (dst_idx + (off_t)b) % ctx->Nb;
+    RSG_CUDA(cudaMemcpy2DAsync((char*)g->d_in + dblk * blk_chan, ctx->Nb * blk_chan, ctx->h_blkbufs[sblk], blk_chan,
+                               blk_chan, ctx->Nc, cudaMemcpyHostToDevice, g->stream));
+  }
+  return 0;
+}
+
+// The same for packed 4-bit blocks, expanded to 8 bits.
+int queue_copy4(rawspec_context* ctx, GpuCtx* g, off_t src_idx, off_t dst_idx, size_t num_blocks) {
+  const size_t blk_packed = (size_t)ctx->Ntpb * ctx->Np;  // bytes per channel per block
+  bool done = false;
+  if (queue_gather(ctx, g, src_idx, dst_idx, num_blocks, blk_packed, true, &done)) return 1;
+  if (done) return 0;
+  if (!g->d_in4) {
+    g->in4_bytes = g->in_bytes / 2;
+    if (dev_alloc(g, &g->d_in4, g->in4_bytes)) return 1;
+  }
+  {
+    ProfScope ps(g, RAWSPEC_GB300_K_H2D);
+    for (size_t b = 0; b < num_blocks; b++) {
+      const off_t sblk = (src_idx + (off_t)b) % ctx->Nb_host;
+      const off_t dblk = (dst_idx + (off_t)b) % ctx->Nb;
+      RSG_CUDA(cudaMemcpy2DAsync(g->d_in4 + dblk * blk_packed, ctx->Nb * blk_packed, ctx->h_blkbufs[sblk],
+                                 blk_packed, blk_packed, ctx->Nc, cudaMemcpyHostToDevice, g->stream));
+    }
+  }
+  Expand4Launch E;
+  E.packed = g->d_in4;
+  E.out = reinterpret_cast<int8_t*>(g->d_in);
+  E.Nc = (int)ctx->Nc;
+  E.Nb = (int)ctx->Nb;
+  E.blk_bytes_packed = (long long)blk_packed;
+  E.dst_block = (int)(dst_idx % ctx->Nb);
+  E.num_blocks = (int)num_blocks;
+  ProfScope ps(g, RAWSPEC_GB300_K_EXPAND4);
+  RSG_CUDA(expand4_launch(E, g->stream));
+  g->launches++;
+  return 0;
+}
+
 }  // namespace
 
 // Device bytes rawspec_initialize() allocates for a validated context: the
@@ -999,6 +1088,17 @@ int rawspec_initialize(rawspec_context* ctx) {
       }
       g->registered = i + 1;
     }
+  }
+
+  // The blocks page-locked above, as kernels see them: kernels read no others.
+  g->host_blocks.assign(ctx->Nb_host, {nullptr, nullptr});
+  for (unsigned i = 0; i < ctx->Nb_host; i++) {
+    if (g->caller_managed && !g->locked_here[i]) continue;
+    void* dev = nullptr;
+    if (cudaHostGetDevicePointer(&dev, ctx->h_blkbufs[i], 0) == cudaSuccess)
+      g->host_blocks[i] = {ctx->h_blkbufs[i], static_cast<const char*>(dev)};
+    else
+      cudaGetLastError();
   }
 
   // Device input buffer.
@@ -1274,16 +1374,7 @@ void rawspec_cleanup(rawspec_context* ctx) {
 int rawspec_copy_blocks_to_gpu(rawspec_context* ctx, off_t src_idx, off_t dst_idx, size_t num_blocks) {
   GpuCtx* g = G(ctx);
   if (!g) return 1;
-  const size_t blk_chan = (size_t)ctx->Ntpb * ctx->Np * 2 * (ctx->Nbps / 8);
-  {
-    ProfScope ps(g, RAWSPEC_GB300_K_H2D);
-    for (size_t b = 0; b < num_blocks; b++) {
-      const off_t sblk = (src_idx + (off_t)b) % ctx->Nb_host;
-      const off_t dblk = (dst_idx + (off_t)b) % ctx->Nb;
-      RSG_CUDA(cudaMemcpy2DAsync((char*)g->d_in + dblk * blk_chan, ctx->Nb * blk_chan, ctx->h_blkbufs[sblk],
-                                 blk_chan, blk_chan, ctx->Nc, cudaMemcpyHostToDevice, g->stream));
-    }
-  }
+  if (queue_copy(ctx, g, src_idx, dst_idx, num_blocks)) return 1;
   RSG_CUDA(cudaStreamSynchronize(g->stream));
   return 0;
 }
@@ -1296,33 +1387,7 @@ int rawspec_copy_blocks_to_gpu_expanding_complex4(rawspec_context* ctx, off_t sr
     fprintf(stderr, "%s: num_blocks (%zu) > Nb (%u)\n", __FUNCTION__, num_blocks, ctx->Nb);
     return 1;
   }
-  const size_t blk_packed = (size_t)ctx->Ntpb * ctx->Np;  // bytes per channel per block
-  if (!g->d_in4) {
-    g->in4_bytes = g->in_bytes / 2;
-    if (dev_alloc(g, &g->d_in4, g->in4_bytes)) return 1;
-  }
-  {
-    ProfScope ps(g, RAWSPEC_GB300_K_H2D);
-    for (size_t b = 0; b < num_blocks; b++) {
-      const off_t sblk = (src_idx + (off_t)b) % ctx->Nb_host;
-      const off_t dblk = (dst_idx + (off_t)b) % ctx->Nb;
-      RSG_CUDA(cudaMemcpy2DAsync(g->d_in4 + dblk * blk_packed, ctx->Nb * blk_packed, ctx->h_blkbufs[sblk],
-                                 blk_packed, blk_packed, ctx->Nc, cudaMemcpyHostToDevice, g->stream));
-    }
-  }
-  Expand4Launch E;
-  E.packed = g->d_in4;
-  E.out = reinterpret_cast<int8_t*>(g->d_in);
-  E.Nc = (int)ctx->Nc;
-  E.Nb = (int)ctx->Nb;
-  E.blk_bytes_packed = (long long)blk_packed;
-  E.dst_block = (int)(dst_idx % ctx->Nb);
-  E.num_blocks = (int)num_blocks;
-  {
-    ProfScope ps(g, RAWSPEC_GB300_K_EXPAND4);
-    RSG_CUDA(expand4_launch(E, g->stream));
-    g->launches++;
-  }
+  if (queue_copy4(ctx, g, src_idx, dst_idx, num_blocks)) return 1;
   RSG_CUDA(cudaStreamSynchronize(g->stream));
   return 0;
 }
@@ -1426,10 +1491,19 @@ int rawspec_copy_blocks_to_gpu_and_start_processing(rawspec_context* ctx, size_t
   if (!g) return 1;
   const int ngroups = std::min<int>(kMaxCopyGroups, (int)ctx->Nc);
   if (num_blocks != ctx->Nb || ngroups < 2 || g->in_bytes < kMinPipelinedBytes) {
-    const int rc = expand4bps_to8bps ? rawspec_copy_blocks_to_gpu_expanding_complex4(ctx, 0, 0, num_blocks)
-                                     : rawspec_copy_blocks_to_gpu(ctx, 0, 0, num_blocks);
-    if (rc) return rc;
-    return rawspec_start_processing(ctx, fft_dir);
+    // The processing is queued behind the copy; the call returns once the copy
+    // has left the host blocks.
+    if (expand4bps_to8bps && num_blocks > ctx->Nb)
+      return rawspec_copy_blocks_to_gpu_expanding_complex4(ctx, 0, 0, num_blocks);  // refused there
+    int rc = expand4bps_to8bps ? queue_copy4(ctx, g, 0, 0, num_blocks) : queue_copy(ctx, g, 0, 0, num_blocks);
+    if (rc) {
+      cudaStreamSynchronize(g->stream);
+      return rc;
+    }
+    RSG_CUDA(cudaEventRecord(g->ev_free, g->stream));
+    rc = rawspec_start_processing(ctx, fft_dir);
+    RSG_CUDA(cudaEventSynchronize(g->ev_free));
+    return rc;
   }
   const bool packed = expand4bps_to8bps != 0;
   if (packed && !g->d_in4) {
