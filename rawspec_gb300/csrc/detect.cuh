@@ -11,6 +11,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fft_core.cuh"
 #include "internal.h"
 
 namespace rsg {
@@ -20,34 +21,23 @@ struct PolOut {
   static constexpr int NP = (POL == POL_TP) ? 1 : 4;
 };
 
-template <int POL, int NV>
-__device__ __forceinline__ void detect_acc(float (&a)[PolOut<POL>::NP], const float2 (&x)[NV],
-                                           float im_sign) {
-  if constexpr (POL == POL_TP) {
-    float s = a[0];
-    s = __fmaf_rn(x[0].x, x[0].x, s);
-    s = __fmaf_rn(x[0].y, x[0].y, s);
-    if constexpr (NV == 2) {
-      s = __fmaf_rn(x[1].x, x[1].x, s);
-      s = __fmaf_rn(x[1].y, x[1].y, s);
-    }
-    a[0] = s;
-  } else {
-    static_assert(NV == 2, "cross-pol products need two polarisations");
-    const float p0 = __fmaf_rn(x[0].x, x[0].x, x[0].y * x[0].y);
-    const float p1 = __fmaf_rn(x[1].x, x[1].x, x[1].y * x[1].y);
-    const float re = __fmaf_rn(x[0].x, x[1].x, x[0].y * x[1].y);
-    const float im = __fmaf_rn(x[0].y, x[1].x, -(x[0].x * x[1].y));
-    if constexpr (POL == POL_FULL) {
-      a[0] += p0;
-      a[1] += p1;
-    } else {
-      a[0] += p0 + p1;
-      a[1] += p0 - p1;
-    }
-    a[2] += re;
-    a[3] = __fmaf_rn(im_sign, im, a[3]);
-  }
+// |X|^2 of both lanes, and their sum.  A spectrum's power is formed first and
+// enters a sum over spectra with one rounding.
+__device__ __forceinline__ float2 powers(const cpair& v) { return f2fma(v.re, v.re, f2mul(v.im, v.im)); }
+__device__ __forceinline__ float both_powers(const cpair& v) {
+  return __fmaf_rn(v.im.y, v.im.y, __fmaf_rn(v.re.y, v.re.y, __fmaf_rn(v.im.x, v.im.x, v.re.x * v.re.x)));
+}
+
+// Adds one spectrum's bin of both polarisations to the sums of the four
+// planes: pw the planes 0 and 1, xr Re and Im of X0 X1* (its sign for
+// conjugated input comes after the last spectrum, being linear).  Stokes Q is summed as the
+// difference of every spectrum, not as the difference of two large sums.
+template <int POL>
+__device__ __forceinline__ void add_planes(const cpair& v, float2& pw, float2& xr) {
+  const float2 p = powers(v);
+  pw = f2add(pw, POL == POL_STOKES ? make_float2(p.x + p.y, p.x - p.y) : p);
+  const float2 x0 = lane0(v), x1 = lane1(v);
+  xr = f2add(xr, make_float2(__fmaf_rn(x0.x, x1.x, x0.y * x1.y), __fmaf_rn(x0.y, x1.x, -(x0.x * x1.y))));
 }
 
 // Position of forward-FFT bin k in the FFT-shifted output of an N-point

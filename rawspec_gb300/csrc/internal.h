@@ -35,6 +35,7 @@ struct SmallLaunch {
   int pol = POL_TP;  // PolMode
   // geometry (filled by small_configure)
   int tpb = 0, sets = 1, chunks = 1, spc = 0, grid = 0;
+  int sms = 0;       // of the device (0: units are not summed within clusters)
   size_t smem = 0;
   // problem
   int Nc = 0, M = 0, units_per_chan = 0, n_units = 0;

@@ -312,17 +312,11 @@ k_large_b(const __grid_constant__ LargeLaunch a) {
 #pragma unroll
     for (int m = 0; m < R; ++m) {
       if constexpr (NP == 4) {
-        const float2 x0 = lane0(v[m]), x1 = lane1(v[m]);
-        acc[m] = f2fma(v[m].im, v[m].im, f2fma(v[m].re, v[m].re, acc[m]));
-        xr[m].x = __fmaf_rn(x0.y, x1.y, __fmaf_rn(x0.x, x1.x, xr[m].x));
-        xr[m].y = __fmaf_rn(-x0.x, x1.y, __fmaf_rn(x0.y, x1.x, xr[m].y));
+        add_planes<POL>(v[m], acc[m], xr[m]);
       } else if constexpr (NV == 1) {
-        acc[m] = f2fma(v[m].im, v[m].im, f2fma(v[m].re, v[m].re, acc[m]));
+        acc[m] = f2add(acc[m], powers(v[m]));
       } else {
-        tp[m] = __fmaf_rn(v[m].re.x, v[m].re.x, tp[m]);
-        tp[m] = __fmaf_rn(v[m].im.x, v[m].im.x, tp[m]);
-        tp[m] = __fmaf_rn(v[m].re.y, v[m].re.y, tp[m]);
-        tp[m] = __fmaf_rn(v[m].im.y, v[m].im.y, tp[m]);
+        tp[m] += both_powers(v[m]);
       }
     }
   }
@@ -331,8 +325,7 @@ k_large_b(const __grid_constant__ LargeLaunch a) {
     if constexpr (NP == 4) {
       if (p == 2) return xr[m].x;
       if (p == 3) return xr[m].y * im_sign;
-      if (POL == POL_FULL) return p == 0 ? acc[m].x : acc[m].y;
-      return p == 0 ? acc[m].x + acc[m].y : acc[m].x - acc[m].y;
+      return p == 0 ? acc[m].x : acc[m].y;
     } else if constexpr (NV == 1) {
       return lane == 0 ? acc[m].x : acc[m].y;
     } else {

@@ -24,6 +24,18 @@
 
 namespace rsg {
 
+// Whether a launch of `ctas` CTAs whose units are spread over `chunks` of them
+// runs these as a cluster.  Up to 8 (what every GPU takes) while every CTA has
+// an SM of its own, else pairs: a larger cluster waits for that many places in
+// one cluster of SMs.  Four units of 8 x 2048 points in four planes: 28 us
+// without, 27 with pairs, 12 with 8; 64 Mi samples of 2048 points in four
+// planes, 1024 CTAs: 278 without, 256 with pairs, 259 with 4, 267 with 8; four
+// products in four planes, 4096 to 8 points: 108, 110, 110, 121.
+constexpr int kSmallCluster = 8;
+inline bool small_clustered(int chunks, int ctas, int sms) {
+  return chunks == 2 || (chunks > 1 && chunks <= kSmallCluster && ctas <= sms);
+}
+
 __host__ __device__ constexpr int small_r(int N, int NP) {
   const int most = NP == 1 && (N == 32 || N == 512 || N == 1024) ? 32 : 16;
   return N < most ? N : most;
@@ -92,6 +104,24 @@ __device__ __forceinline__ void group_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The cluster's size, its barrier, and a float of CTA `rank`'s shared memory.
+__device__ __forceinline__ uint32_t cluster_ctas() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+  return n;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float cluster_load(uint32_t addr, uint32_t rank) {
+  float f;
+  asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.f32 %0, [r];\n\t}"
+               : "=f"(f)
+               : "r"(addr), "r"(rank)
+               : "memory");
+  return f;
+}
+
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
                "l"(src)
@@ -100,6 +130,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 // The same through L1 (neighbouring copies share a 32-byte sector).
 __device__ __forceinline__ void cp_async16_l1(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+// 8 bytes (twiddle tables need not start or end on 16).
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
                "l"(src)
                : "memory");
 }
@@ -123,10 +159,10 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   const int g = tid / T;   // group within the CTA
   const int j = tid % T;   // thread within the group
 
-  if constexpr (C::TW > 0) {
-    for (int i = tid; i < C::TW; i += TPB) tw_s[i] = a.tw[i];
-    __syncthreads();
-  }
+  // The twiddle table and the first spectra are requested together: one trip
+  // to memory before the first transform, not two.
+#pragma unroll 4
+  for (int i = tid; i < C::TW; i += TPB) cp_async8(tw_s + i, a.tw + i);
 
   // Which unit / spectra this group works on.  The CTA covers `sets` units
   // (gps groups each) and one chunk of spc spectra of each of them.
@@ -147,9 +183,8 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   auto spec_of = [&](int it) { return s_begin + (gi + it * gps) * SPI; };
 
   // Accumulators.  Total power: one sum per bin over both lanes.  Four
-  // planes: the two powers as one packed pair (|X0|^2, |X1|^2), the cross
-  // terms Re and Im(X0 X1*) unsigned; Stokes I and Q and the conjugation sign
-  // are linear in these sums and applied after the last spectrum.
+  // planes: the first two as one packed pair, the cross terms Re and Im(X0
+  // X1*) as another.
   float tp[NP == 1 ? R : 1];
   float2 pw[NP == 4 ? R : 1], xr[NP == 4 ? R : 1];
 #pragma unroll
@@ -222,11 +257,12 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   W wn[SPI][C::STAGED ? 1 : R];
   if constexpr (C::STAGED) {
     stage(0);
-    if constexpr (T > 32) {
+    if constexpr (C::TW > 0) {
       cp_async_wait();
-      group_barrier(1 + g, T);
+      __syncthreads();
     }
   } else {
+    static_assert(C::TW == 0, "unstaged transforms use no table");
 #pragma unroll
     for (int q = 0; q < SPI; ++q) fetch(0, q, wn[q]);
   }
@@ -294,15 +330,9 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
 #pragma unroll
       for (int m = 0; m < R; ++m) {
         if constexpr (NP == 1) {
-          tp[m] = __fmaf_rn(v[m].re.x, v[m].re.x, tp[m]);
-          tp[m] = __fmaf_rn(v[m].im.x, v[m].im.x, tp[m]);
-          tp[m] = __fmaf_rn(v[m].re.y, v[m].re.y, tp[m]);
-          tp[m] = __fmaf_rn(v[m].im.y, v[m].im.y, tp[m]);
+          tp[m] += both_powers(v[m]);
         } else {
-          const float2 x0 = lane0(v[m]), x1 = lane1(v[m]);
-          pw[m] = f2fma(v[m].im, v[m].im, f2fma(v[m].re, v[m].re, pw[m]));
-          xr[m].x = __fmaf_rn(x0.y, x1.y, __fmaf_rn(x0.x, x1.x, xr[m].x));
-          xr[m].y = __fmaf_rn(-x0.x, x1.y, __fmaf_rn(x0.y, x1.x, xr[m].y));
+          add_planes<POL>(v[m], pw[m], xr[m]);
         }
       }
     }
@@ -317,8 +347,8 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     if constexpr (NP == 1) {
       acc[0] = tp[m];
     } else {
-      acc[0] = POL == POL_FULL ? pw[m].x : pw[m].x + pw[m].y;
-      acc[1] = POL == POL_FULL ? pw[m].y : pw[m].x - pw[m].y;
+      acc[0] = pw[m].x;
+      acc[1] = pw[m].y;
       acc[2] = xr[m].x;
       acc[3] = xr[m].y * im_sign;
     }
@@ -327,25 +357,57 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   }
   __syncthreads();
 
+  const bool clustered = cluster_ctas() > 1;
   const int set_threads = gps * T;
   const int t_in_set = tid - set * set_threads;
   auto store = [&](int p, int k, float s) {
     float* dst = a.out + (((size_t)d * NP + p) * a.Nc + c) * N + out_pos(k, N, a.inverse);
     if (a.mode == ACC_ADD) *dst = __fmaf_rn(s, a.scale, *dst); else *dst = s * a.scale;
   };
-  for (int o = unit_ok ? t_in_set : NP * N; o < NP * N; o += set_threads) {
+  // (a cluster's CTA of one group has its sums where they belong)
+  for (int o = unit_ok && !(clustered && gps == 1) ? t_in_set : NP * N; o < NP * N; o += set_threads) {
     const int p = o / N;
     const int k = o - p * N;
     const int m = k / T;
     const int jj = k - m * T;
     float s = 0.0f;
-    for (int q = 0; q < gps; ++q) s += red[(set * gps + q) * C::RED + (p * R + m) * T + jj];
-    if (a.chunks > 1) __stcg(a.partial + (((size_t)unit * a.chunks + chunk) * NP + p) * N + k, s);
+    float* const slot = red + set * gps * C::RED + (p * R + m) * T + jj;
+    for (int q = 0; q < gps; ++q) s += slot[q * C::RED];
+    if (clustered) *slot = s;
+    else if (a.chunks > 1) __stcg(a.partial + (((size_t)unit * a.chunks + chunk) * NP + p) * N + k, s);
     else store(p, k, s);
   }
   if (a.chunks == 1) return;
 
-  // Units spread over CTAs: the last CTA of the block of units to arrive sums
+  // Units spread over the CTAs of a cluster: every CTA keeps its sums where
+  // the first group's were, and sums a share of the outputs over the chunks,
+  // in chunk order, from the others' shared memory.  By the last CTA alone
+  // (below) four units of 8 x 2048 points in four planes take 27.7 us, so
+  // 11.3; 64 Mi samples of 4096 points in four planes 390, so 353.
+  if (clustered) {
+    cluster_sync();
+    for (int o = unit_ok ? t_in_set + chunk * set_threads : NP * N; o < NP * N; o += set_threads * a.chunks) {
+      const int p = o / N;
+      const int k = o - p * N;
+      const int m = k / T;
+      const int jj = k - m * T;
+      const uint32_t slot =
+          static_cast<uint32_t>(__cvta_generic_to_shared(red + set * gps * C::RED + (p * R + m) * T + jj));
+      float f[kSmallCluster], s = 0.0f;
+#pragma unroll
+      for (int q = 0; q < kSmallCluster; ++q)
+        if (q < a.chunks) f[q] = cluster_load(slot, q);
+#pragma unroll
+      for (int q = 0; q < kSmallCluster; ++q)
+        if (q < a.chunks) s += f[q];
+      store(p, k, s);
+    }
+    cluster_sync();  // no CTA leaves before its sums are read
+    return;
+  }
+
+  // Units spread over more CTAs than a cluster holds, and the launches that
+  // share a grid: the last CTA of the block of units to arrive sums
   // the chunks' partials in chunk order (the same order whichever CTA it is)
   // and leaves the arrival counter zeroed for the next launch.  A kernel of
   // its own for this sum cost a launch and a drained GPU, 6-10 us a product.
@@ -360,26 +422,46 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   if (!s_last) return;
   __threadfence();
   if (!unit_ok) return;
-  constexpr int V = NP * N % 4 == 0 ? 4 : 1;  // outputs per access
-  for (int o = t_in_set * V; o < NP * N; o += set_threads * V) {
-    const float* src = a.partial + (size_t)unit * a.chunks * NP * N + o;
-    float s[V];
+  // U accesses of V outputs a thread and Q chunks at a time: the sum is a
+  // chain of trips to L2 otherwise (four planes of 4096 points in 4 chunks: 64
+  // trips, 12 us).
+  constexpr int V = NP * N % 4 == 0 ? 4 : 1, U = NP * N >= 2048 ? 4 : 1, Q = U == 4 ? 2 : 8;
+  const int step = set_threads * V;
+  const float* const base = a.partial + (size_t)unit * a.chunks * NP * N;
+  for (int o = t_in_set * V; o < NP * N; o += step * U) {
+    float s[U][V] = {};
+    for (int q0 = 0; q0 < a.chunks; q0 += Q) {
+      float f[Q][U][V];
 #pragma unroll
-    for (int i = 0; i < V; ++i) s[i] = 0.0f;
-#pragma unroll 8
-    for (int q = 0; q < a.chunks; ++q) {
-      if constexpr (V == 4) {
-        const float4 f = __ldcg(reinterpret_cast<const float4*>(src + (size_t)q * NP * N));
-        s[0] += f.x;
-        s[1] += f.y;
-        s[2] += f.z;
-        s[3] += f.w;
-      } else {
-        s[0] += __ldcg(src + (size_t)q * NP * N);
+      for (int q = 0; q < Q; ++q) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (q0 + q >= a.chunks || o + u * step >= NP * N) continue;
+          const float* src = base + (size_t)(q0 + q) * NP * N + o + u * step;
+          if constexpr (V == 4) {
+            const float4 w = __ldcg(reinterpret_cast<const float4*>(src));
+            f[q][u][0] = w.x, f[q][u][1] = w.y, f[q][u][2] = w.z, f[q][u][3] = w.w;
+          } else {
+            f[q][u][0] = __ldcg(src);
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (q0 + q >= a.chunks) break;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+          for (int i = 0; i < V; ++i) s[u][i] += f[q][u][i];
+        }
       }
     }
 #pragma unroll
-    for (int i = 0; i < V; ++i) store((o + i) / N, (o + i) % N, s[i]);
+    for (int u = 0; u < U; ++u) {
+      if (o + u * step >= NP * N) break;
+#pragma unroll
+      for (int i = 0; i < V; ++i) store((o + u * step + i) / N, (o + u * step + i) % N, s[u][i]);
+    }
   }
 }
 
@@ -458,6 +540,20 @@ cudaError_t launch_t(const SmallLaunch& L, cudaStream_t s, int op, int* occ, con
   }
   const int grid = small_grid(L);
   if (grid < 1) return cudaSuccess;
+  if (small_clustered(L.chunks, grid, L.sms)) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(C::TPB);
+    cfg.dynamicSmemBytes = L.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = L.chunks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, L);
+  }
   k<<<grid, C::TPB, L.smem, s>>>(L);
   return cudaGetLastError();
 }
@@ -503,12 +599,14 @@ cudaError_t small_dispatch(const SmallLaunch& L, cudaStream_t s, int op, int* oc
 // occupancy slots would be the wrong measure: 1024 CTAs of N = 64 run in
 // 127 us, 512 twice as long ones in 143, 2560 in 124), plus about 0.6
 // iterations for a CTA's start and reduction; a CTA alone on its SM is bound
-// by its own latency, about 1.5 times its share of a full one.  Split units
-// add an arrival and a sum at the end (about 2 us) and the traffic of the
-// partial sums.  All times in microseconds.
+// by its own latency, about 1.5 times its share of a full one.  A unit split
+// within a cluster adds about 1.5 us; one split over more CTAs an arrival, the
+// traffic of the partial sums and their sum by one CTA (120 GB/s).  All times
+// in microseconds.
 struct SplitCost {
   double unit;     // SM time of one iteration of a CTA
   double partial;  // traffic of one chunk's partial sums of every unit
+  double serial;   // the last CTA's reading of one chunk's partial sums
   int sms, occ;
 };
 int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k) {
@@ -519,7 +617,8 @@ int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitC
     if (c > c_lo && (turns + per - 1) / per != c) continue;
     const double per_sm = std::ceil((double)ublocks * c / k.sms);
     const double load = std::max(per_sm, 1.5 * std::ceil(per_sm / k.occ));
-    const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + (c > 1 ? 2.0 + c * k.partial : 0.0);
+    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : 2.0 + c * (k.partial + k.serial);
+    const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + sum;
     if (cost < best_cost * 0.99) {
       best_cost = cost;
       best = c;
@@ -581,6 +680,7 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   const int max_chunks = (turns + gps - 1) / gps;
   int occ = 0, sms = 0;
   resident_ctas(L, &occ, &sms);
+  L.sms = sms;
   // The split of `units` units: spectra per chunk, and the chunks that makes.
   auto split = [&](int units, int* spc, int* chunks) {
     const int ub = (units + L.sets - 1) / L.sets;
@@ -592,7 +692,8 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
     if (max_arrivals && ublocks > max_arrivals) most = 1;
     // a sample of both lanes takes about 2.3 ps of the GPU; partial sums are
     // written and read at about 4 TB/s
-    const SplitCost cost{si.TPB * si.R * sms * 2.3e-6, (double)ub * L.sets * np * (1 << L.logN) * 2e-6, sms, occ};
+    const SplitCost cost{si.TPB * si.R * sms * 2.3e-6, (double)ub * L.sets * np * (1 << L.logN) * 2e-6,
+                         (double)L.sets * np * (1 << L.logN) * 5e-5, sms, occ};
     const int c = occ > 0 ? fit_chunks(turns, gps, ub, std::min(most, std::max(1, aim / 4)), std::max(1, most), cost)
                           : std::max(1, std::min(aim, most));
     const int per = (turns + c - 1) / c;  // iterations' worth of spectra per chunk
