@@ -60,15 +60,11 @@ __device__ __forceinline__ float2 f2sub(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 f2dup(float x) { return make_float2(x, x); }
 
-// Elements of the engine: float (one vector) or float2 (two in lockstep),
-// with sums, differences and a multiply-add by a factor common to the lanes.
-__device__ __forceinline__ float eadd(float a, float b) { return __fadd_rn(a, b); }
+// Elements of the engine (two vectors in lockstep): sums, differences and a
+// multiply-add by a factor common to the lanes.
 __device__ __forceinline__ float2 eadd(float2 a, float2 b) { return f2add(a, b); }
-__device__ __forceinline__ float esub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float2 esub(float2 a, float2 b) { return f2sub(a, b); }
-__device__ __forceinline__ float esubk(float a, float k) { return __fadd_rn(a, -k); }
 __device__ __forceinline__ float2 esubk(float2 a, float k) { return f2add(a, f2dup(-k)); }
-__device__ __forceinline__ float efma(float a, float k, float c) { return __fmaf_rn(a, k, c); }
 __device__ __forceinline__ float2 efma(float2 a, float k, float2 c) { return f2fma(a, f2dup(k), c); }
 
 template <typename E>
@@ -259,33 +255,12 @@ __host__ __device__ constexpr int stockham_tw_size(int N, int R) {
 // the im parts) of smem_padded_len(N) elements each, `sm_stride` elements
 // apart.  SYNC is a functor performing the barrier required between the
 // group's threads.
-template <int N, int R, int NV>
+template <int N, int R>
 struct GroupFFT {
   using S = FftShape<N, R>;
   static constexpr int T = S::T;
   static constexpr int PS = R >= 32 ? 5 : 4;
-  using E = std::conditional_t<NV == 2, float2, float>;
-
-  template <typename Sync>
-  static __device__ __forceinline__ void run(float2 (&v)[NV][R], int j, E* sm, int sm_stride,
-                                             const float2* __restrict__ tw, Sync sync) {
-    cx<E> p[R];
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      if constexpr (NV == 2) p[m] = pack2(v[0][m], v[1][m]);
-      else p[m] = {v[0][m].x, v[0][m].y};
-    }
-    run_packed(p, j, sm, sm_stride, tw, sync);
-#pragma unroll
-    for (int m = 0; m < R; ++m) {
-      if constexpr (NV == 2) {
-        v[0][m] = lane0(p[m]);
-        v[1][m] = lane1(p[m]);
-      } else {
-        v[0][m] = make_float2(p[m].re, p[m].im);
-      }
-    }
-  }
+  using E = float2;
 
   template <bool BIASED>
   static __device__ __forceinline__ void first_pass(cx<E> (&v)[R]) {
@@ -298,9 +273,9 @@ struct GroupFFT {
 
   // SPLIT: one exchange buffer only (sm_stride unused), the re parts and then
   // the im parts passing through it (twice the barriers, half the shared
-  // memory).  BIASED: the input values carry kCodeBias.  sync(first, last) is told whether the barrier is the
-  // transform's first (every thread of the group has taken its input) or its
-  // last.
+  // memory).  BIASED: the input values carry kCodeBias.  sync(first, last) is
+  // told whether the barrier is the transform's first (every thread of the
+  // group has taken its input) or its last.
   template <bool SPLIT = false, bool BIASED = false, typename Sync>
   static __device__ __forceinline__ void run_packed(cx<E> (&v)[R], int j, E* sm, int sm_stride,
                                                     const float2* __restrict__ tw, Sync sync) {

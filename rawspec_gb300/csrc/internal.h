@@ -34,7 +34,7 @@ struct SmallLaunch {
   int nv = 2;        // input polarisations
   int pol = POL_TP;  // PolMode
   // geometry (filled by small_configure)
-  int tpb = 0, sets = 1, chunks = 1, spc = 0, grid = 0;
+  int sets = 1, chunks = 1, spc = 0;
   int sms = 0;       // of the device (0: units are not summed within clusters)
   size_t smem = 0;
   // problem

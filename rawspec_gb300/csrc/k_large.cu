@@ -208,7 +208,7 @@ k_large_a(const __grid_constant__ LargeLaunch a) {
       }
     }
     // the next tile is requested when every thread has taken this one's words
-    GroupFFT<N2, R, 2>::template run_packed<Cf::SPLIT, FMT == FMT_I8>(
+    GroupFFT<N2, R>::template run_packed<Cf::SPLIT, FMT == FMT_I8>(
         v, j, xch + (size_t)col * XS, smem_padded_len(N2), tw_s, [&](bool taken, bool) {
           __syncthreads();
           if (taken && tile + 1 < last) request(tile + 1);
@@ -308,7 +308,7 @@ k_large_b(const __grid_constant__ LargeLaunch a) {
 #pragma unroll
       for (int m = 0; m < R; ++m) v[m] = pack2(__ldcs(src + m * T), __ldcs(src + N1 + m * T));
     }
-    GroupFFT<N1, R, 2>::template run_packed<false>(v, j, my_xch, smem_padded_len(N1), tw_s, BlockSyncL{});
+    GroupFFT<N1, R>::template run_packed<false>(v, j, my_xch, smem_padded_len(N1), tw_s, BlockSyncL{});
 #pragma unroll
     for (int m = 0; m < R; ++m) {
       if constexpr (NP == 4) {

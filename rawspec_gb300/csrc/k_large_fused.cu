@@ -509,7 +509,7 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
         if (t > 0) refill(t - 1);
         const float2 w0 = tw[j * C + col];  // W_N^(n1 j)
         float2* dst = scr;
-        GroupFFT<N2, R, 2>::template run_packed<true, true>(v, j, sb + (size_t)col * F::GSA, 0, twA, Sync{});
+        GroupFFT<N2, R>::template run_packed<true, true>(v, j, sb + (size_t)col * F::GSA, 0, twA, Sync{});
 #pragma unroll
         for (int m = 0; m < R; ++m) {
           const int k2 = j + m * T;
@@ -612,7 +612,7 @@ k_large_fused(const __grid_constant__ LargeLaunch a) {
           if (TOUT && tid == 0) bulk_wait_read();
           __syncthreads();  // both stage buffers are read
           refill(2 * t);
-          GroupFFT<N1, R, 2>::template run_packed<true>(vp, j, sb1 + (size_t)row * F::GSB, 0, twB, Sync{});
+          GroupFFT<N1, R>::template run_packed<true>(vp, j, sb1 + (size_t)row * F::GSB, 0, twB, Sync{});
           refill(2 * t + 1);
           if constexpr (POL == POL_TP) {
 #pragma unroll

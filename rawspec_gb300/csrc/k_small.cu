@@ -325,7 +325,7 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     };
     static_assert(T <= 32 || FftShape<N, R>::PASSES >= 3, "a group's copies span two exchanges");
     static_assert(G <= 15 || T <= 32, "one named barrier per group");
-    GroupFFT<N, R, 2>::template run_packed<C::SPLIT, kBiased>(v, j, xch, C::PLANE, tw_s, sync);
+    GroupFFT<N, R>::template run_packed<C::SPLIT, kBiased>(v, j, xch, C::PLANE, tw_s, sync);
     if (valid) {
 #pragma unroll
       for (int m = 0; m < R; ++m) {
@@ -666,7 +666,6 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   if (L.logN < 0 || L.logN > 12 || L.M < 1 || L.n_units < 1) return -1;
   SmallInfo si{};
   if (small_dispatch(L, nullptr, 4, nullptr, nullptr, &si) != cudaSuccess) return -1;
-  L.tpb = si.TPB;
   L.smem = si.smem;
   const int G = si.G;
   const int np = L.pol == POL_TP ? 1 : 4;
@@ -701,7 +700,6 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
     *chunks = (turns + per - 1) / per;
   };
   split(L.n_units, &L.spc, &L.chunks);
-  L.grid = ublocks * L.chunks;
   // the same for a launch over 1/pipe_groups of the units
   split(std::max(1, L.n_units / std::max(1, pipe_groups)), &L.spc_pipe, &L.chunks_pipe);
   const int cmax = std::max(L.chunks, L.chunks_pipe);
