@@ -171,13 +171,17 @@ int rawspec_gb300_device_bytes_estimate(const rawspec_context *ctx, size_t *byte
  *            rawspec_start_processing() dumps for such a product
  *   stream   cudaStream_t to queue the work on (0 = legacy default stream)
  *
- * Scratch: a file-scope device array of 4 MiB of partial sums plus a 4096-entry
- * twiddle table (4.03 MiB), held by every GPU that loads the library until the
+ * Scratch: file-scope device arrays of 4 MiB of partial sums, a 4096-entry
+ * twiddle table, arrival counters and the twiddle tables of every FFT length
+ * (4.16 MiB in all), held by every GPU that loads the library until the
  * process exits.  The partial-sum split is limited to what fits; FFT lengths
  * above 4096 are rejected with an error.  The first call on a device looks up
- * the array's device address (make that first call before any stream capture
- * on that device).  Every call shares the array and it keeps the last call's
- * contents; everything a call reads from it is written by the same call first.
+ * the arrays' device addresses, fills the twiddle tables on its stream and
+ * waits for that (make that first call before any stream capture on that
+ * device; until a call outside a capture has filled them, a captured call
+ * fills a table of its own).  Every call shares the arrays and they keep the
+ * last call's contents: the tables, which stay, and sums, which every call
+ * writes before it reads them.
  * The looked-up address belongs to the device's primary context (the CUDA
  * runtime's); after cudaDeviceReset the library must be reloaded before this
  * entry point is used again.

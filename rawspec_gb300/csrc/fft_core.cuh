@@ -4,13 +4,13 @@
 //   * dft_regs<R>: an R-point DFT (R a power of two <= 32) held entirely in
 //     registers; radix-2 decimation in time, natural order in and out, every
 //     twiddle multiplication fused into its butterfly.
-//   * GroupFFT<N, R, NV>: an N-point FFT computed by a group of T = N/R
-//     threads, each holding R values of NV independent vectors (the two
-//     polarisations share every twiddle).  Stockham auto-sort passes of radix
-//     R (a smaller radix for the last pass when N is not a power of R), with
-//     one shared-memory exchange between passes.  On entry thread j holds
-//     x[j + m*T] in v[.][m]; on exit it holds X[j + m*T].  The formulation is
-//     the classic per-thread Stockham iteration (Govindaraju et al., SC08).
+//   * GroupFFT<N, R>: an N-point FFT computed by a group of T = N/R threads,
+//     each holding R values of two vectors in lockstep, which share every
+//     twiddle.  Stockham auto-sort passes of radix R (a smaller radix for the
+//     last pass when N is not a power of R), with one shared-memory exchange
+//     between passes.  On entry thread j holds x[j + m*T] in v[m]; on exit it
+//     holds X[j + m*T].  The formulation is the classic per-thread Stockham
+//     iteration (Govindaraju et al., SC08).
 //
 // All FFTs here are forward, exp(-2 pi i k n / N), unnormalised; the inverse
 // transform is obtained by the index reversal X_inv[k] = X_fwd[(N-k) mod N]
@@ -30,7 +30,8 @@
 // 6 operations per butterfly and R/2 table entries (16 points: 192 operations
 // and 8 entries; separate factors: 228 and 15).
 //
-// Two vectors in lockstep (NV = 2, the two polarisations) run on the packed
+// Two vectors in lockstep (the two polarisations of a spectrum, or two
+// spectra, columns or rows of one polarisation) run on the packed
 // FP32 instructions of sm_100 and later (add/sub/fma .f32x2, each lane
 // rounded exactly as the scalar _rn operation): element m of both vectors is
 // held as a cpair {re: (x0.re, x1.re), im: (x0.im, x1.im)}, so that one

@@ -181,7 +181,7 @@ cudaError_t expand4_launch(const Expand4Launch& Lin, cudaStream_t s) {
 // Corner turn of a small buffer straight from the page-locked host blocks: row
 // (channel, block) goes to its place in the device buffer, 4-bit samples
 // expanded on the way.  Bound by the latency of the first load over the link,
-// then by the link (290 GB/s at 8 MiB, the copy engines' rate).  One launch in
+// then by the link, at the copy engines' rate from 4 MiB on.  One launch in
 // place of a pitched copy per block and an expansion, each 2 to 5 us of host
 // and engine: 8 channels, 8 blocks of 256 samples, 8 KiB each, with two spectra
 // of 2048 and the dump 74 -> 48 us.  Rows off the 16-byte grid go bytewise, a

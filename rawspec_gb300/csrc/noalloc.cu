@@ -7,8 +7,8 @@
 // memory through its own pool and budget.  This entry point takes the input
 // and output as caller-provided device pointers and keeps its only scratch --
 // the per-chunk partial sums of the fused small-FFT kernel, its twiddle tables
-// and its arrival counters -- in the file-scope arrays below, which every GPU that loads the
-// library holds until the process exits.
+// and its arrival counters -- in the file-scope arrays below, which every GPU
+// that loads the library holds until the process exits.
 #include <cstdint>
 #include <cstdio>
 #include <mutex>

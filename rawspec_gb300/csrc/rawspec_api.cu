@@ -797,7 +797,7 @@ int launch_deferred(std::vector<DeferredSmall>& d) {
 // the copy engines.  The corner turn, one product and its dump, us: 0.5 MiB in
 // 8 blocks 53 by the engines, 23 by the kernel; 2 MiB in 8 blocks 52 and 35; 4
 // MiB in one block 58 and 48 with the call alone, 35 both ways back to back; 8
-// MiB 77 and 74, 55 both ways; 16 MiB 130 both ways: the link's rate.
+// MiB 77 and 74, 55 both ways; 16 MiB 130 both ways.
 constexpr size_t kGatherBytes = size_t(8) << 20;
 
 // Queues the corner turn of a small copy as one kernel if it can be one: few
