@@ -609,7 +609,7 @@ struct SplitCost {
   double serial;   // the last CTA's reading of one chunk's partial sums
   int sms, occ;
 };
-int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k) {
+int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k, double* cost_of = nullptr) {
   int best = c_lo;
   double best_cost = 1e300;
   for (int c = c_lo; c <= c_hi; ++c) {
@@ -624,6 +624,7 @@ int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitC
       best = c;
     }
   }
+  if (cost_of) *cost_of = best_cost;
   return best;
 }
 
@@ -673,35 +674,53 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   // Groups per unit: at most one per spectrum (or pair of them), and few
   // enough that every thread of a set has an output to reduce (gps <= |P| * R).
   const int turns = (L.M + si.SPI - 1) / si.SPI;  // iterations of a unit on one group
-  int gps = std::min(G, std::min(pow2_floor(np * si.R), pow2_floor(turns)));
-  L.sets = G / gps;
-  const int ublocks = (L.n_units + L.sets - 1) / L.sets;
-  const int max_chunks = (turns + gps - 1) / gps;
+  const int most_gps = std::min(G, std::min(pow2_floor(np * si.R), pow2_floor(turns)));
   int occ = 0, sms = 0;
   resident_ctas(L, &occ, &sms);
   L.sms = sms;
-  // The split of `units` units: spectra per chunk, and the chunks that makes.
-  auto split = [&](int units, int* spc, int* chunks) {
-    const int ub = (units + L.sets - 1) / L.sets;
+  // The split of `units` units, `gps` groups each: spectra per chunk, and the
+  // chunks that makes; returns its cost.
+  auto split = [&](int units, int gps, int* spc, int* chunks) {
+    const int sets = G / gps;
+    const int all = (L.n_units + sets - 1) / sets, ub = (units + sets - 1) / sets;
     const int aim = std::max(1, (target_ctas + ub - 1) / ub);  // chunks that fill the GPU
     // partial sums that fit the limit and the arrival counters
     const long long floats = (long long)L.n_units * np << L.logN;
-    int most = (int)std::min<long long>(max_chunks, std::max(8, 4 * aim));
+    int most = (int)std::min<long long>((turns + gps - 1) / gps, std::max(8, 4 * aim));
     if (max_partial) most = (int)std::min<long long>(most, std::max<long long>(1, (long long)max_partial / floats));
-    if (max_arrivals && ublocks > max_arrivals) most = 1;
+    if (max_arrivals && all > max_arrivals) most = 1;
     // a sample of both lanes takes about 2.3 ps of the GPU; partial sums are
     // written and read at about 4 TB/s
-    const SplitCost cost{si.TPB * si.R * sms * 2.3e-6, (double)ub * L.sets * np * (1 << L.logN) * 2e-6,
-                         (double)L.sets * np * (1 << L.logN) * 5e-5, sms, occ};
-    const int c = occ > 0 ? fit_chunks(turns, gps, ub, std::min(most, std::max(1, aim / 4)), std::max(1, most), cost)
+    const SplitCost k{si.TPB * si.R * sms * 2.3e-6, (double)ub * sets * np * (1 << L.logN) * 2e-6,
+                      (double)sets * np * (1 << L.logN) * 5e-5, sms, occ};
+    double cost = 0.0;
+    const int c = occ > 0 ? fit_chunks(turns, gps, ub, std::min(most, std::max(1, aim / 4)), std::max(1, most), k, &cost)
                           : std::max(1, std::min(aim, most));
     const int per = (turns + c - 1) / c;  // iterations' worth of spectra per chunk
     *spc = std::min(L.M, per * si.SPI);
     *chunks = (turns + per - 1) / per;
+    return cost;
   };
-  split(L.n_units, &L.spc, &L.chunks);
+  // Groups per unit: as many as that, or fewer where their last iteration
+  // would leave too many of them idle (9 spectra on eight groups: 16 turns).
+  // 64 Mi samples, always as many / by the cost: 64 points, 17 spectra a unit
+  // 264 / 129 us, 256 points in four planes, 9 spectra 413 / 240, 1024 points, 5
+  // spectra 275 / 203; powers of two the same either way.
+  int gps = most_gps;
+  double best = 0.0;
+  for (int g = most_gps; g >= 1; g /= 2) {
+    int spc = 0, chunks = 0;
+    const double cost = split(L.n_units, g, &spc, &chunks);
+    if (g == most_gps || cost < 0.95 * best) {
+      best = cost;
+      gps = g;
+    }
+  }
+  L.sets = G / gps;
+  const int ublocks = (L.n_units + L.sets - 1) / L.sets;
+  split(L.n_units, gps, &L.spc, &L.chunks);
   // the same for a launch over 1/pipe_groups of the units
-  split(std::max(1, L.n_units / std::max(1, pipe_groups)), &L.spc_pipe, &L.chunks_pipe);
+  split(std::max(1, L.n_units / std::max(1, pipe_groups)), gps, &L.spc_pipe, &L.chunks_pipe);
   const int cmax = std::max(L.chunks, L.chunks_pipe);
   *partial_floats = cmax > 1 ? (size_t)L.n_units * cmax * np * ((size_t)1 << L.logN) : 0;
   L.arrivals = cmax > 1 ? ublocks : 0;
