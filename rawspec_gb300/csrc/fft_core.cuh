@@ -126,12 +126,13 @@ __device__ __forceinline__ void bfly_const(cx<E>& a, cx<E>& b, int q, int len) {
     bfly_uv(a, b, eadd(y.re, y.im), esub(y.im, y.re), 0.70710678118654752f, mi);
     return;
   }
+  // (tangents of the rounded cosine, as in the tables)
   const float c = (float)cos_pi16(r), s = (float)sin_pi16(r);
   if (r < 4) {  // c (1 - i tan)
-    const float k = (float)(sin_pi16(r) / cos_pi16(r));
+    const float k = (float)(sin_pi16(r) / (double)c);
     bfly_uv(a, b, efma(y.im, k, y.re), efma(y.re, -k, y.im), c, mi);
   } else {      // s (cot - i)
-    const float k = (float)(cos_pi16(r) / sin_pi16(r));
+    const float k = (float)(cos_pi16(r) / (double)s);
     const E u = efma(y.re, k, y.im), nv = efma(y.im, -k, y.re);  // w y = s (u - i nv)
     if (!mi) {
       a = {efma(u, s, x.re), efma(nv, -s, x.im)};
