@@ -104,7 +104,10 @@ __device__ __forceinline__ void group_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
-// The cluster's size, its barrier, and a float of CTA `rank`'s shared memory.
+template <int V>
+using Int = std::integral_constant<int, V>;
+
+// The cluster's size and its barrier.
 __device__ __forceinline__ uint32_t cluster_ctas() {
   uint32_t n;
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
@@ -113,12 +116,15 @@ __device__ __forceinline__ uint32_t cluster_ctas() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ float cluster_load(uint32_t addr, uint32_t rank) {
+// The cluster address of `addr` of CTA `rank`'s shared memory, and its float.
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float cluster_load(uint32_t addr) {
   float f;
-  asm volatile("{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %1, %2;\n\tld.shared::cluster.f32 %0, [r];\n\t}"
-               : "=f"(f)
-               : "r"(addr), "r"(rank)
-               : "memory");
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(addr) : "memory");
   return f;
 }
 
@@ -338,44 +344,107 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     }
   }
 
-  // Reduce across the groups of each set: red[g][p][m][j].
-  cp_async_wait();  // nothing lands in the area any more (none is in flight after the last iteration)
-  __syncthreads();
-#pragma unroll
-  for (int m = 0; m < R; ++m) {
-    float acc[NP];
-    if constexpr (NP == 1) {
-      acc[0] = tp[m];
-    } else {
-      acc[0] = pw[m].x;
-      acc[1] = pw[m].y;
-      acc[2] = xr[m].x;
-      acc[3] = xr[m].y * im_sign;
-    }
-#pragma unroll
-    for (int p = 0; p < NP; ++p) red[g * C::RED + (p * R + m) * T + j] = acc[p];
-  }
-  __syncthreads();
-
+  // Bin j + m T of plane p as this thread summed it.
+  auto sum_of = [&](int p, int m) -> float {
+    if constexpr (NP == 1) return tp[m];
+    else return p == 0 ? pw[m].x : p == 1 ? pw[m].y : p == 2 ? xr[m].x : xr[m].y * im_sign;
+  };
   const bool clustered = cluster_ctas() > 1;
   const int set_threads = gps * T;
   const int t_in_set = tid - set * set_threads;
-  auto store = [&](int p, int k, float s) {
-    float* dst = a.out + (((size_t)d * NP + p) * a.Nc + c) * N + out_pos(k, N, a.inverse);
-    if (a.mode == ACC_ADD) *dst = __fmaf_rn(s, a.scale, *dst); else *dst = s * a.scale;
+  // Plane p of the unit's result, and the place of bin k in it (out_pos).
+  float* const out = a.out + ((size_t)d * NP * a.Nc + c) * N;
+  const size_t plane = (size_t)a.Nc * N;
+  const int dir = a.inverse ? -1 : 1;
+  auto place = [&](int k) { return ((k * dir) & (N - 1)) ^ (N >> 1); };
+  // Writes s[i], or adds it, to the addresses at(i), i < n (the old values are
+  // requested before the first is written).
+  auto store = [&](auto& s, int n, auto at) {
+    constexpr int U = sizeof(s) / sizeof(float);
+    if (a.mode == ACC_ADD) {
+      float old[U];
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (i < n) old[i] = *at(i);
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (i < n) *at(i) = __fmaf_rn(s[i], a.scale, old[i]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < U; ++i)
+        if (i < n) *at(i) = s[i] * a.scale;
+    }
   };
-  // (a cluster's CTA of one group has its sums where they belong)
-  for (int o = unit_ok && !(clustered && gps == 1) ? t_in_set : NP * N; o < NP * N; o += set_threads) {
-    const int p = o / N;
-    const int k = o - p * N;
-    const int m = k / T;
-    const int jj = k - m * T;
-    float s = 0.0f;
-    float* const slot = red + set * gps * C::RED + (p * R + m) * T + jj;
-    for (int q = 0; q < gps; ++q) s += slot[q * C::RED];
-    if (clustered) *slot = s;
-    else if (a.chunks > 1) __stcg(a.partial + (((size_t)unit * a.chunks + chunk) * NP + p) * N + k, s);
-    else store(p, k, s);
+  // Bins k + i step, i < n, of plane p: the result, or the chunk's partial sums.
+  float* const part = a.partial + ((size_t)unit * a.chunks + chunk) * NP * N;
+  auto store_or_part = [&](auto& s, int n, int p, int k, int step) {
+    if (a.chunks == 1) {
+      float* const o = out + p * plane;
+      store(s, n, [&](int i) { return o + place(k + i * step); });
+      return;
+    }
+    float* const o = part + p * N + k;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(s) / sizeof(float)); ++i)
+      if (i < n) __stcg(o + i * step, s[i]);
+  };
+
+  // What follows runs once a CTA, often with one warp to a scheduler, so that
+  // its time is its instructions': addresses move by additions.
+  cp_async_wait();  // none is in flight after the last iteration; nothing lands in the reduction area any more
+  float* const red_set = red + set * gps * C::RED;
+  constexpr bool kDirect = R < 32;
+  if (kDirect && gps == 1 && !clustered) {
+    // One group a unit: its threads hold the sums.  (Of 32 values each they go
+    // through shared memory all the same: with this branch the transforms'
+    // loop takes 1.5 % longer.)
+    if (unit_ok) {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        float s[R];
+#pragma unroll
+        for (int m = 0; m < R; ++m) s[m] = sum_of(p, m);
+        store_or_part(s, R, p, j, T);
+      }
+    }
+  } else {
+    // Reduce across the groups of each set: red[g][p][m][j] = red[g][p][k].
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < R; ++m)
+#pragma unroll
+      for (int p = 0; p < NP; ++p) red[g * C::RED + (p * R + m) * T + j] = sum_of(p, m);
+    __syncthreads();
+    const int kstep = min(set_threads, N), pstep = max(1, set_threads / N);
+    // U bins at a time, Q groups at a time (a divisor of their number)
+    auto sum_groups = [&](auto u_, auto q_) {
+      constexpr int U = decltype(u_)::value, Q = decltype(q_)::value;
+      for (int p = t_in_set / N; p < NP; p += pstep) {
+        for (int k = t_in_set % N; k < N; k += U * kstep) {
+          const int n = U == 1 ? 1 : (N - 1 - k) / kstep + 1;
+          float* const src = red_set + p * N + k;
+          float s[U] = {};
+          for (int q = 0; q < gps; q += Q)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (u < n) {
+                const float* f = src + q * C::RED + u * kstep;
+                s[u] += Q == 1 ? f[0] : Q == 2 ? f[0] + f[C::RED] : (f[0] + f[C::RED]) + (f[2 * C::RED] + f[3 * C::RED]);
+              }
+          if (clustered) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+              if (u < n) src[u * kstep] = s[u];
+          } else {
+            store_or_part(s, n, p, k, kstep);
+          }
+        }
+      }
+    };
+    // (a cluster's CTA of one group has its sums where they belong)
+    if (unit_ok && gps > 4) sum_groups(Int<1>{}, Int<4>{});
+    else if (unit_ok && gps > 1) sum_groups(Int<(NP * R >= 16 ? 4 : 1)>{}, Int<2>{});
+    else if (!kDirect && unit_ok && !clustered) sum_groups(Int<1>{}, Int<1>{});
   }
   if (a.chunks == 1) return;
 
@@ -386,21 +455,26 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   // 11.3; 64 Mi samples of 4096 points in four planes 390, so 353.
   if (clustered) {
     cluster_sync();
-    for (int o = unit_ok ? t_in_set + chunk * set_threads : NP * N; o < NP * N; o += set_threads * a.chunks) {
-      const int p = o / N;
-      const int k = o - p * N;
-      const int m = k / T;
-      const int jj = k - m * T;
-      const uint32_t slot =
-          static_cast<uint32_t>(__cvta_generic_to_shared(red + set * gps * C::RED + (p * R + m) * T + jj));
-      float f[kSmallCluster], s = 0.0f;
+    constexpr int U = NP * N >= 1024 ? 4 : 1;
+    uint32_t from[kSmallCluster];
 #pragma unroll
-      for (int q = 0; q < kSmallCluster; ++q)
-        if (q < a.chunks) f[q] = cluster_load(slot, q);
+    for (int q = 0; q < kSmallCluster; ++q)
+      if (q < a.chunks) from[q] = cluster_map(static_cast<uint32_t>(__cvta_generic_to_shared(red_set)), q);
+    const int step = set_threads * a.chunks;
+    for (int o = unit_ok ? t_in_set + chunk * set_threads : NP * N; o < NP * N; o += U * step) {
+      const int n = (NP * N - 1 - o) / step + 1;
+      float f[U][kSmallCluster], s[U] = {};
 #pragma unroll
-      for (int q = 0; q < kSmallCluster; ++q)
-        if (q < a.chunks) s += f[q];
-      store(p, k, s);
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < kSmallCluster; ++q)
+          if (u < n && q < a.chunks) f[u][q] = cluster_load(from[q] + (o + u * step) * sizeof(float));
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < kSmallCluster; ++q)
+          if (u < n && q < a.chunks) s[u] += f[u][q];
+      store(s, n, [&](int u) { return out + (o + u * step) / N * plane + place(o + u * step); });
     }
     cluster_sync();  // no CTA leaves before its sums are read
     return;
@@ -458,9 +532,9 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (o + u * step >= NP * N) break;
-#pragma unroll
-      for (int i = 0; i < V; ++i) store((o + u * step + i) / N, (o + u * step + i) % N, s[u][i]);
+      const int at = o + u * step;
+      if (at >= NP * N) break;
+      store(s[u], V, [&](int i) { return out + (at + i) / N * plane + place(at + i); });
     }
   }
 }

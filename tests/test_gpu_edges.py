@@ -82,3 +82,14 @@ def test_two_kernel_lengths(cuda_device, logn, Np, npol):
 def test_small_copies(cuda_device, Np, nbits, Ntpb, Nb, combined):
     total = Ntpb * Nb
     check(5, Np, Ntpb, Nb, nbits, [(8, 2 * total // 8, 1)], buffers=2, combined=combined, seed=Ntpb)
+
+
+# Units of one group of threads, which writes its sums itself: one spectrum a
+# unit, written and added over two buffers, and a chunk of one iteration.
+@pytest.mark.parametrize("npol", [1, 4])
+@pytest.mark.parametrize("nt", [1, 2, 8, 16, 32, 64, 512, 1024, 4096])
+def test_units_of_one_group(cuda_device, monkeypatch, nt, npol):
+    monkeypatch.setenv("RAWSPEC_GB300_TENSOR_DFT", "0")
+    check(5, 2, nt, 1, 8, [(nt, 2, npol)], buffers=4, fft_dir=-1, conj=1, seed=nt)
+    check(3, 2, 3 * nt, 1, 16, [(nt, 1, npol)], seed=nt + 1)
+    check(70, 2, 2 * nt, 1, 8, [(nt, 2, npol)], seed=nt + 2)
