@@ -21,20 +21,9 @@
 #include "detect.cuh"
 #include "fft_core.cuh"
 #include "internal.h"
+#include "small_split.h"
 
 namespace rsg {
-
-// Whether a launch of `ctas` CTAs whose units are spread over `chunks` of them
-// runs these as a cluster.  Up to 8 (what every GPU takes) while every CTA has
-// an SM of its own, else pairs: a larger cluster waits for that many places in
-// one cluster of SMs.  Four units of 8 x 2048 points in four planes: 28 us
-// without, 27 with pairs, 12 with 8; 64 Mi samples of 2048 points in four
-// planes, 1024 CTAs: 278 without, 256 with pairs, 259 with 4, 267 with 8; four
-// products in four planes, 4096 to 8 points: 108, 110, 110, 121.
-constexpr int kSmallCluster = 8;
-inline bool small_clustered(int chunks, int ctas, int sms) {
-  return chunks == 2 || (chunks > 1 && chunks <= kSmallCluster && ctas <= sms);
-}
 
 __host__ __device__ constexpr int small_r(int N, int NP) {
   const int most = NP == 1 && (N == 32 || N == 512 || N == 1024) ? 32 : 16;
@@ -667,41 +656,6 @@ cudaError_t small_dispatch(const SmallLaunch& L, cudaStream_t s, int op, int* oc
   }
 }
 
-// Chunks per unit: the split with the shortest schedule.  A launch lasts as
-// long as its most loaded SM: ceil(CTAs / SMs) CTAs of `iters` iterations each
-// (an SM with fewer CTAs resident than it holds loses little, so a split over
-// occupancy slots would be the wrong measure: 1024 CTAs of N = 64 run in
-// 127 us, 512 twice as long ones in 143, 2560 in 124), plus about 0.6
-// iterations for a CTA's start and reduction; a CTA alone on its SM is bound
-// by its own latency, about 1.5 times its share of a full one.  A unit split
-// within a cluster adds about 1.5 us; one split over more CTAs an arrival, the
-// traffic of the partial sums and their sum by one CTA (120 GB/s).  All times
-// in microseconds.
-struct SplitCost {
-  double unit;     // SM time of one iteration of a CTA
-  double partial;  // traffic of one chunk's partial sums of every unit
-  double serial;   // the last CTA's reading of one chunk's partial sums
-  int sms, occ;
-};
-int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k, double* cost_of = nullptr) {
-  int best = c_lo;
-  double best_cost = 1e300;
-  for (int c = c_lo; c <= c_hi; ++c) {
-    const int per = (turns + c - 1) / c;
-    if (c > c_lo && (turns + per - 1) / per != c) continue;
-    const double per_sm = std::ceil((double)ublocks * c / k.sms);
-    const double load = std::max(per_sm, 1.5 * std::ceil(per_sm / k.occ));
-    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : 2.0 + c * (k.partial + k.serial);
-    const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + sum;
-    if (cost < best_cost * 0.99) {
-      best_cost = cost;
-      best = c;
-    }
-  }
-  if (cost_of) *cost_of = best_cost;
-  return best;
-}
-
 // Resident CTAs per SM of the configuration and SMs of the current device, with
 // the kernel's dynamic shared-memory limit raised; asked of the runtime once
 // per configuration and device (it takes longer than a small launch).  0
@@ -744,57 +698,35 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   L.smem = si.smem;
   const int G = si.G;
   const int np = L.pol == POL_TP ? 1 : 4;
-  auto pow2_floor = [](int x) { int p = 1; while (p * 2 <= x) p *= 2; return p; };
-  // Groups per unit: at most one per spectrum (or pair of them), and few
-  // enough that every thread of a set has an output to reduce (gps <= |P| * R).
-  const int turns = (L.M + si.SPI - 1) / si.SPI;  // iterations of a unit on one group
-  const int most_gps = std::min(G, std::min(pow2_floor(np * si.R), pow2_floor(turns)));
   int occ = 0, sms = 0;
   resident_ctas(L, &occ, &sms);
   L.sms = sms;
-  // The split of `units` units, `gps` groups each: spectra per chunk, and the
-  // chunks that makes; returns its cost.
-  auto split = [&](int units, int gps, int* spc, int* chunks) {
-    const int sets = G / gps;
-    const int all = (L.n_units + sets - 1) / sets, ub = (units + sets - 1) / sets;
-    const int aim = std::max(1, (target_ctas + ub - 1) / ub);  // chunks that fill the GPU
-    // partial sums that fit the limit and the arrival counters
-    const long long floats = (long long)L.n_units * np << L.logN;
-    int most = (int)std::min<long long>((turns + gps - 1) / gps, std::max(8, 4 * aim));
-    if (max_partial) most = (int)std::min<long long>(most, std::max<long long>(1, (long long)max_partial / floats));
-    if (max_arrivals && all > max_arrivals) most = 1;
-    // a sample of both lanes takes about 2.3 ps of the GPU; partial sums are
-    // written and read at about 4 TB/s
-    const SplitCost k{si.TPB * si.R * sms * 2.3e-6, (double)ub * sets * np * (1 << L.logN) * 2e-6,
-                      (double)sets * np * (1 << L.logN) * 5e-5, sms, occ};
-    double cost = 0.0;
-    const int c = occ > 0 ? fit_chunks(turns, gps, ub, std::min(most, std::max(1, aim / 4)), std::max(1, most), k, &cost)
-                          : std::max(1, std::min(aim, most));
-    const int per = (turns + c - 1) / c;  // iterations' worth of spectra per chunk
+  SplitProblem p;
+  p.turns = (L.M + si.SPI - 1) / si.SPI;
+  p.units = p.all_units = L.n_units;
+  p.groups = G;
+  p.planes = np;
+  p.n = 1 << L.logN;
+  p.radix = si.R;
+  p.target_ctas = target_ctas;
+  p.sms = sms;
+  p.occ = occ;
+  // a sample of both lanes takes about 2.3 ps of the GPU
+  p.unit_us = si.TPB * si.R * sms * 2.3e-6;
+  p.max_partial = max_partial;
+  p.max_arrivals = max_arrivals;
+  const Split all = split_groups_and_chunks(p);
+  auto take = [&](const Split& s, int* spc, int* chunks) {
+    const int per = (p.turns + s.chunks - 1) / s.chunks;  // iterations' worth of spectra per chunk
     *spc = std::min(L.M, per * si.SPI);
-    *chunks = (turns + per - 1) / per;
-    return cost;
+    *chunks = (p.turns + per - 1) / per;
   };
-  // Groups per unit: as many as that, or fewer where their last iteration
-  // would leave too many of them idle (9 spectra on eight groups: 16 turns).
-  // 64 Mi samples, always as many / by the cost: 64 points, 17 spectra a unit
-  // 264 / 129 us, 256 points in four planes, 9 spectra 413 / 240, 1024 points, 5
-  // spectra 275 / 203; powers of two the same either way.
-  int gps = most_gps;
-  double best = 0.0;
-  for (int g = most_gps; g >= 1; g /= 2) {
-    int spc = 0, chunks = 0;
-    const double cost = split(L.n_units, g, &spc, &chunks);
-    if (g == most_gps || cost < 0.95 * best) {
-      best = cost;
-      gps = g;
-    }
-  }
-  L.sets = G / gps;
+  L.sets = G / all.gps;
   const int ublocks = (L.n_units + L.sets - 1) / L.sets;
-  split(L.n_units, gps, &L.spc, &L.chunks);
+  take(all, &L.spc, &L.chunks);
   // the same for a launch over 1/pipe_groups of the units
-  split(std::max(1, L.n_units / std::max(1, pipe_groups)), gps, &L.spc_pipe, &L.chunks_pipe);
+  p.units = std::max(1, L.n_units / std::max(1, pipe_groups));
+  take(p.units == p.all_units ? all : split_chunks(p, all.gps), &L.spc_pipe, &L.chunks_pipe);
   const int cmax = std::max(L.chunks, L.chunks_pipe);
   *partial_floats = cmax > 1 ? (size_t)L.n_units * cmax * np * ((size_t)1 << L.logN) : 0;
   L.arrivals = cmax > 1 ? ublocks : 0;

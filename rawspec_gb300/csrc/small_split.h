@@ -1,0 +1,154 @@
+// How k_small's units are split over groups and CTAs: plain host code.
+//
+// A unit's spectra are taken in turns (a spectrum, or two of one
+// polarisation) by `gps` groups of threads of each of `chunks` CTAs.  The
+// allocation-free entry point plans in every call, before a kernel of 8 to 30
+// us, so the search looks only at counts that can win.  One channel of 10^6
+// spectra of 8 points: every count of every number of groups 9124 and 80 us of
+// an x86 core, these 167 and 6.4; 20000 spectra of 64 points 47 -> 0.5 us.  The
+// split found is the same.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+#include <cstddef>
+
+namespace rsg {
+
+// Whether a launch of `ctas` CTAs whose units are spread over `chunks` of them
+// runs these as a cluster.  Up to 8 (what every GPU takes) while every CTA has
+// an SM of its own, else pairs: a larger cluster waits for that many places in
+// one cluster of SMs.  Four units of 8 x 2048 points in four planes: 28 us
+// without, 27 with pairs, 12 with 8; 64 Mi samples of 2048 points in four
+// planes, 1024 CTAs: 278 without, 256 with pairs, 259 with 4, 267 with 8; four
+// products in four planes, 4096 to 8 points: 108, 110, 110, 121.
+constexpr int kSmallCluster = 8;
+inline bool small_clustered(int chunks, int ctas, int sms) {
+  return chunks == 2 || (chunks > 1 && chunks <= kSmallCluster && ctas <= sms);
+}
+
+struct SplitProblem {
+  int turns = 1;        // of a unit
+  int units = 1;        // of the launch
+  int all_units = 1;    // of the product (what the scratch is sized for)
+  int groups = 1;       // of a CTA
+  int planes = 1, n = 1, radix = 1;  // output planes, FFT length, values per thread
+  int target_ctas = 1;  // CTAs that fill the GPU
+  int sms = 0, occ = 0; // of the device, and resident CTAs per SM (0: unknown)
+  double unit_us = 0;   // SM time of one iteration of a CTA
+  std::size_t max_partial = 0;  // floats of partial sums (0: no limit)
+  int max_arrivals = 0;         // arrival counters (0: no limit)
+};
+struct Split {
+  int gps = 1, chunks = 1;
+  double cost = 0;  // microseconds
+};
+
+// Times in microseconds of a launch with every count of chunks.
+struct SplitCost {
+  double unit;     // SM time of one iteration of a CTA
+  double partial;  // traffic of one chunk's partial sums of every unit
+  double serial;   // the last CTA's reading of one chunk's partial sums
+  int sms, occ;
+
+  // Iterations of a CTA with `per` turns.
+  static int iterations(int per, int gps) { return (per + gps - 1) / gps; }
+  // CTAs of the most loaded SM with `ctas` in all.
+  int on_one_sm(int ctas) const { return (ctas + sms - 1) / sms; }
+  double sum(int c, int ublocks) const {
+    return c == 1 ? 0.0 : small_clustered(c, ublocks * c, sms) ? 1.5 : 2.0 + c * (partial + serial);
+  }
+  double cost(int iters, int per_sm, double sum_us) const {
+    const double load = std::max((double)per_sm, 1.5 * ((per_sm + occ - 1) / occ));
+    return (iters + 0.6) * unit * load + sum_us;
+  }
+};
+
+// Chunks per unit: the split with the shortest schedule.  A launch lasts as
+// long as its most loaded SM: ceil(CTAs / SMs) CTAs of `iters` iterations each
+// (an SM with fewer CTAs resident than it holds loses little, so a split over
+// occupancy slots would be the wrong measure: 1024 CTAs of N = 64 run in
+// 127 us, 512 twice as long ones in 143, 2560 in 124), plus about 0.6
+// iterations for a CTA's start and reduction; a CTA alone on its SM is bound
+// by its own latency, about 1.5 times its share of a full one.  A unit split
+// within a cluster adds about 1.5 us; one split over more CTAs an arrival, the
+// traffic of the partial sums and their sum by one CTA (120 GB/s).
+//
+// Of the counts that load the SMs alike and leave a CTA as many iterations the
+// smallest is the best (the sum costs more with every chunk), so the search
+// goes from one such count to the next; and over all that load them alike if
+// the fewest iterations among them would not win.  *tried: counts looked at.
+inline int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k, double* cost_of,
+                      int* tried = nullptr) {
+  auto ceil_div = [](long long a, long long b) { return (int)std::min<long long>((a + b - 1) / b, 1 << 30); };
+  int best = c_lo, level = 0;
+  double best_cost = 1e300;
+  for (int c = c_lo; c <= c_hi;) {
+    const int per = ceil_div(turns, c), iters = SplitCost::iterations(per, gps);
+    const int per_sm = k.on_one_sm(ublocks * c);
+    const int beyond = (int)std::min<long long>((long long)per_sm * k.sms / ublocks + 1, (long long)c_hi + 1);
+    const double sum = k.sum(c, ublocks);
+    if (tried) ++*tried;
+    int next = beyond;
+    if (per_sm == level ||
+        k.cost(SplitCost::iterations(ceil_div(turns, beyond - 1), gps), per_sm, sum) < best_cost * 0.99) {
+      level = per_sm;
+      const double cost = k.cost(iters, per_sm, sum);
+      if (cost < best_cost * 0.99) {
+        best_cost = cost;
+        best = c;
+      }
+      if (iters > 1) next = std::min(next, ceil_div(turns, (long long)gps * (iters - 1)));
+    }
+    // the next count that no smaller one equals in turns per chunk
+    const int next_per = ceil_div(turns, next);
+    if (ceil_div(turns, next_per) != next) next = next_per > 1 ? ceil_div(turns, next_per - 1) : c_hi + 1;
+    c = next;
+  }
+  *cost_of = best_cost;
+  return best;
+}
+
+// Chunks of a launch with `gps` groups per unit.
+inline Split split_chunks(const SplitProblem& p, int gps, int* tried = nullptr) {
+  const int sets = p.groups / gps;
+  const int all = (p.all_units + sets - 1) / sets, ub = (p.units + sets - 1) / sets;
+  const int aim = std::max(1, (p.target_ctas + ub - 1) / ub);  // chunks that fill the GPU
+  // partial sums that fit the limit and the arrival counters
+  const long long floats = (long long)p.all_units * p.planes * p.n;
+  int most = (int)std::min<long long>((p.turns + gps - 1) / gps, std::max(8, 4 * aim));
+  if (p.max_partial) most = (int)std::min<long long>(most, std::max<long long>(1, (long long)p.max_partial / floats));
+  if (p.max_arrivals && all > p.max_arrivals) most = 1;
+  Split s;
+  s.gps = gps;
+  if (p.occ <= 0) {
+    s.chunks = std::max(1, std::min(aim, most));
+    return s;
+  }
+  // partial sums are written and read at about 4 TB/s
+  const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 5e-5, p.sms, p.occ};
+  s.chunks = fit_chunks(p.turns, gps, ub, std::min(most, std::max(1, aim / 4)), std::max(1, most), k, &s.cost, tried);
+  return s;
+}
+
+// Groups per unit: at most one per spectrum (or pair of them), few enough that
+// every thread of a set has an output to reduce (gps <= |P| * R), and fewer
+// where their last iteration would leave too many of them idle (9 spectra on
+// eight groups: 16 turns).  64 Mi samples, always as many / by the cost: 64
+// points, 17 spectra a unit 264 / 129 us, 256 points in four planes, 9 spectra
+// 413 / 240, 1024 points, 5 spectra 275 / 203; powers of two the same either way.
+inline Split split_groups_and_chunks(const SplitProblem& p, int* tried = nullptr) {
+  auto pow2_floor = [](int x) { int q = 1; while (q * 2 <= x) q *= 2; return q; };
+  const int most = std::min(p.groups, std::min(pow2_floor(p.planes * p.radix), pow2_floor(p.turns)));
+  Split best = split_chunks(p, most, tried);
+  for (int gps = most / 2; gps >= 1 && p.occ > 0; gps /= 2) {
+    // All turns of all units over all SMs: no split takes less.
+    const int sets = p.groups / gps, ub = (p.units + sets - 1) / sets;
+    if (0.999 * p.turns * ub * p.unit_us / ((double)gps * p.sms) >= 0.95 * best.cost) continue;
+    const Split s = split_chunks(p, gps, tried);
+    if (s.cost < 0.95 * best.cost) best = s;
+  }
+  return best;
+}
+
+}  // namespace rsg
