@@ -5,7 +5,7 @@
 // allocation-free entry point plans in every call, before a kernel of 8 to 30
 // us, so the search looks only at counts that can win.  One channel of 10^6
 // spectra of 8 points: every count of every number of groups 9124 and 80 us of
-// an x86 core, these 167 and 6.4; 20000 spectra of 64 points 47 -> 0.5 us.  The
+// an x86 core, these 320 and 4.8; 20000 spectra of 64 points 47 -> 3.0 us.  The
 // split found is the same.
 #pragma once
 
@@ -52,16 +52,17 @@ struct SplitCost {
   int sms, occ;
 
   // Iterations of a CTA with `per` turns.
-  static int iterations(int per, int gps) { return (per + gps - 1) / gps; }
+  static int iterations(unsigned per, unsigned gps) { return (int)((per + gps - 1) / gps); }
   // CTAs of the most loaded SM with `ctas` in all.
-  int on_one_sm(int ctas) const { return (ctas + sms - 1) / sms; }
+  int on_one_sm(int ctas) const { return (int)((unsigned)(ctas + sms - 1) / (unsigned)sms); }
   double sum(int c, int ublocks) const {
     return c == 1 ? 0.0 : small_clustered(c, ublocks * c, sms) ? 1.5 : 2.0 + c * (partial + serial);
   }
-  double cost(int iters, int per_sm, double sum_us) const {
-    const double load = std::max((double)per_sm, 1.5 * ((per_sm + occ - 1) / occ));
-    return (iters + 0.6) * unit * load + sum_us;
+  // SM time of an iteration of all of them, over that of one
+  double load(int per_sm) const {
+    return std::max((double)per_sm, 1.5 * (int)((unsigned)(per_sm + occ - 1) / (unsigned)occ));
   }
+  double cost(int iters, double load, double sum_us) const { return (iters + 0.6) * unit * load + sum_us; }
 };
 
 // Chunks per unit: the split with the shortest schedule.  A launch lasts as
@@ -76,34 +77,39 @@ struct SplitCost {
 //
 // Of the counts that load the SMs alike and leave a CTA as many iterations the
 // smallest is the best (the sum costs more with every chunk), so the search
-// goes from one such count to the next; and over all that load them alike if
-// the fewest iterations among them would not win.  *tried: counts looked at.
+// goes from one such count to the next with few enough iterations to win, and
+// over all that load them alike if the fewest among them would not.  *tried:
+// counts looked at.
 inline int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k, double* cost_of,
                       int* tried = nullptr) {
-  auto ceil_div = [](long long a, long long b) { return (int)std::min<long long>((a + b - 1) / b, 1 << 30); };
-  int best = c_lo, level = 0;
+  // (32-bit divisions: they are most of the search's time)
+  auto ceil_div = [](unsigned a, unsigned b) { return (int)((a + b - 1) / b); };
+  int best = c_lo;
   double best_cost = 1e300;
   for (int c = c_lo; c <= c_hi;) {
-    const int per = ceil_div(turns, c), iters = SplitCost::iterations(per, gps);
+    // the counts from here that load the most loaded SM alike
     const int per_sm = k.on_one_sm(ublocks * c);
-    const int beyond = (int)std::min<long long>((long long)per_sm * k.sms / ublocks + 1, (long long)c_hi + 1);
-    const double sum = k.sum(c, ublocks);
+    const int beyond = std::min((int)((unsigned)(per_sm * k.sms) / (unsigned)ublocks), c_hi) + 1;
+    const double load = k.load(per_sm);
     if (tried) ++*tried;
-    int next = beyond;
-    if (per_sm == level ||
-        k.cost(SplitCost::iterations(ceil_div(turns, beyond - 1), gps), per_sm, sum) < best_cost * 0.99) {
-      level = per_sm;
-      const double cost = k.cost(iters, per_sm, sum);
-      if (cost < best_cost * 0.99) {
-        best_cost = cost;
-        best = c;
+    if (k.cost(SplitCost::iterations(ceil_div(turns, beyond - 1), gps), load, k.sum(c, ublocks)) < best_cost * 0.99) {
+      while (c < beyond) {
+        if (tried) ++*tried;
+        const int iters = SplitCost::iterations(ceil_div(turns, c), gps);
+        const double sum = k.sum(c, ublocks), cost = k.cost(iters, load, sum);
+        if (cost < best_cost * 0.99) {
+          best_cost = cost;
+          best = c;
+        }
+        const double most = (best_cost * 0.99 - sum) / (k.unit * load) + 0.4;  // iterations with which one could win
+        const int fewer = most < iters - 1 ? (int)most : iters - 1;
+        c = fewer >= 1 ? ceil_div(turns, gps * fewer) : beyond;
       }
-      if (iters > 1) next = std::min(next, ceil_div(turns, (long long)gps * (iters - 1)));
     }
-    // the next count that no smaller one equals in turns per chunk
-    const int next_per = ceil_div(turns, next);
-    if (ceil_div(turns, next_per) != next) next = next_per > 1 ? ceil_div(turns, next_per - 1) : c_hi + 1;
-    c = next;
+    // the first count beyond that no smaller one equals in turns per chunk
+    c = beyond;
+    const int per = ceil_div(turns, c);
+    if (ceil_div(turns, per) != c) c = per > 1 ? ceil_div(turns, per - 1) : c_hi + 1;
   }
   *cost_of = best_cost;
   return best;
@@ -126,8 +132,8 @@ inline Split split_chunks(const SplitProblem& p, int gps, int* tried = nullptr) 
     return s;
   }
   // partial sums are written and read at about 4 TB/s
-  const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 5e-5, p.sms, p.occ};
-  s.chunks = fit_chunks(p.turns, gps, ub, std::min(most, std::max(1, aim / 4)), std::max(1, most), k, &s.cost, tried);
+  const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ};
+  s.chunks = fit_chunks(p.turns, gps, ub, 1, std::max(1, most), k, &s.cost, tried);
   return s;
 }
 

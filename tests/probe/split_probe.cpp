@@ -1,6 +1,7 @@
 // The split search of k_small against the plain loops over every count, on the
 // host.  Prints one line per problem of a sweep that differs, then for the
-// allocation-free call's longest integrations the counts tried by both.
+// allocation-free call's longest integrations the counts tried by both, then
+// the chunks of single units in four planes.
 #include <cstdio>
 #include <cstdlib>
 
@@ -40,10 +41,10 @@ static Split every(const SplitProblem& p, int* tried) {
     int c_hi = (int)std::min<long long>((p.turns + gps - 1) / gps, std::max(8, 4 * aim));
     if (p.max_partial) c_hi = (int)std::min<long long>(c_hi, std::max<long long>(1, (long long)p.max_partial / floats));
     if (p.max_arrivals && all > p.max_arrivals) c_hi = 1;
-    const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 5e-5, p.sms, p.occ};
+    const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ};
     Split s;
     s.gps = gps;
-    s.chunks = fit_every(p.turns, gps, ub, std::min(c_hi, std::max(1, aim / 4)), std::max(1, c_hi), k, &s.cost, tried);
+    s.chunks = fit_every(p.turns, gps, ub, 1, std::max(1, c_hi), k, &s.cost, tried);
     if (gps == most || s.cost < 0.95 * best.cost) best = s;
   }
   return best;
@@ -97,5 +98,8 @@ int main() {
     every(p, &b);
     printf("tried %d of %d\n", a, b);
   }
+  // One unit's partial sums are summed by one CTA: more chunks than a cluster
+  // takes cost more than they save.
+  for (int n : {1024, 2048, 4096}) printf("chunks %d\n", split_groups_and_chunks(problem(n, 4, 1, 64, false)).chunks);
   return differ != 0;
 }
