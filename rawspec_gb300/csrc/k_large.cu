@@ -35,8 +35,11 @@ namespace {
 // a sample of both polarisations (4 in, 16 out), pass B 16 and the result.
 //   * Pass A: CTAs of 128 threads, C neighbouring columns each, whose
 //     words come through shared memory (cp.async, 16 bytes of a row a copy) one
-//     tile ahead of the transforms.  16 values per thread up to 256 points, 32
-//     for 512 and 1024 (one exchange).
+//     tile ahead of the transforms, where a CTA has whole sectors (32 bytes) of
+//     a row: of half ones the copies fetch every sector twice (2^22 points of 16
+//     bits, columns of 2048: 2055 us copied, 1186 read directly, 1815 with 256
+//     threads and a polarisation at a time).  16 values per thread up to 256
+//     points, 32 for 512 and 1024 (one exchange).
 //   * Pass B: 16 values per thread and two neighbouring rows across the lanes,
 //     so that a warp's load takes 256 contiguous bytes of each row; with
 //     eight rows (64 bytes) a load it took 333 us per 64 Mi samples, with two
@@ -55,7 +58,7 @@ struct ColumnCfg {
   static constexpr int TW = stockham_tw_size(NSUB, R);
   static constexpr bool SPLIT = R == 32;          // one exchange buffer: three CTAs fit an SM
   static constexpr int WB = FMT == FMT_I16 ? 8 : 4;
-  static constexpr bool STAGED = C * WB >= 16;
+  static constexpr bool STAGED = C * WB >= 32;
   static constexpr int STAGE = STAGED ? NSUB * C * WB : 0;
 };
 // OUT: results staged until a CTA has several neighbouring rows (units of one
