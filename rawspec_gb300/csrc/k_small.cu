@@ -339,10 +339,20 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     else return p == 0 ? pw[m].x : p == 1 ? pw[m].y : p == 2 ? xr[m].x : xr[m].y * im_sign;
   };
   const bool clustered = cluster_ctas() > 1;
-  const int set_threads = gps * T;
-  const int t_in_set = tid - set * set_threads;
-  // Plane p of the unit's result, and the place of bin k in it (out_pos).
-  float* const out = a.out + ((size_t)d * NP * a.Nc + c) * N;
+  // The sums of the CTA's units are shared out over its threads: to those of
+  // the unit's own groups, or where it has fewer units than sets, to 2, 4, ...
+  // times as many (one unit of four spectra of 32 points in four planes, 8 and
+  // all of 128 threads: 7.9 and 5.8 us).
+  const int here = min(a.sets, a.unit0 + a.unit_count - (unit - set));
+  int set_threads = gps * T;
+  while (2 * here * set_threads <= TPB) set_threads *= 2;
+  const int sum_set = tid / set_threads, t_in_set = tid % set_threads;
+  const int sum_unit = unit - set + sum_set;
+  const bool sum_ok = sum_set < here;
+  // A unit's result (its plane 0), and the place of bin k in a plane (out_pos).
+  auto result = [&](int u) {
+    return a.out + ((size_t)(u % a.units_per_chan) * NP * a.Nc + u / a.units_per_chan) * N;
+  };
   const size_t plane = (size_t)a.Nc * N;
   const int dir = a.inverse ? -1 : 1;
   auto place = [&](int k) { return ((k * dir) & (N - 1)) ^ (N >> 1); };
@@ -364,15 +374,18 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
         if (i < n) *at(i) = s[i] * a.scale;
     }
   };
-  // Bins k + i step, i < n, of plane p: the result, or the chunk's partial sums.
-  float* const part = a.partial + ((size_t)unit * a.chunks + chunk) * NP * N;
-  auto store_or_part = [&](auto& s, int n, int p, int k, int step) {
+  // Where unit u's sums go, the result or the chunk's partial sums, and bins k +
+  // i step, i < n, of its plane p.
+  auto target = [&](int u) {
+    return a.chunks == 1 ? result(u) : a.partial + ((size_t)u * a.chunks + chunk) * NP * N;
+  };
+  auto store_or_part = [&](float* to, auto& s, int n, int p, int k, int step) {
     if (a.chunks == 1) {
-      float* const o = out + p * plane;
+      float* const o = to + p * plane;
       store(s, n, [&](int i) { return o + place(k + i * step); });
       return;
     }
-    float* const o = part + p * N + k;
+    float* const o = to + p * N + k;
 #pragma unroll
     for (int i = 0; i < (int)(sizeof(s) / sizeof(float)); ++i)
       if (i < n) __stcg(o + i * step, s[i]);
@@ -381,19 +394,20 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   // What follows runs once a CTA, often with one warp to a scheduler, so that
   // its time is its instructions': addresses move by additions.
   cp_async_wait();  // none is in flight after the last iteration; nothing lands in the reduction area any more
-  float* const red_set = red + set * gps * C::RED;
+  float* const red_set = red + sum_set * gps * C::RED;
   constexpr bool kDirect = R < 32;
   if (kDirect && gps == 1 && !clustered) {
     // One group a unit: its threads hold the sums.  (Of 32 values each they go
     // through shared memory all the same: with this branch the transforms'
     // loop takes 1.5 % longer.)
     if (unit_ok) {
+      float* const to = target(unit);
 #pragma unroll
       for (int p = 0; p < NP; ++p) {
         float s[R];
 #pragma unroll
         for (int m = 0; m < R; ++m) s[m] = sum_of(p, m);
-        store_or_part(s, R, p, j, T);
+        store_or_part(to, s, R, p, j, T);
       }
     }
   } else {
@@ -404,6 +418,7 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
 #pragma unroll
       for (int p = 0; p < NP; ++p) red[g * C::RED + (p * R + m) * T + j] = sum_of(p, m);
     __syncthreads();
+    float* const to = target(sum_unit);
     const int kstep = min(set_threads, N), pstep = max(1, set_threads / N);
     // U bins at a time, Q groups at a time (a divisor of their number)
     auto sum_groups = [&](auto u_, auto q_) {
@@ -425,15 +440,15 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
             for (int u = 0; u < U; ++u)
               if (u < n) src[u * kstep] = s[u];
           } else {
-            store_or_part(s, n, p, k, kstep);
+            store_or_part(to, s, n, p, k, kstep);
           }
         }
       }
     };
     // (a cluster's CTA of one group has its sums where they belong)
-    if (unit_ok && gps > 4) sum_groups(Int<1>{}, Int<4>{});
-    else if (unit_ok && gps > 1) sum_groups(Int<(NP * R >= 16 ? 4 : 1)>{}, Int<2>{});
-    else if (!kDirect && unit_ok && !clustered) sum_groups(Int<1>{}, Int<1>{});
+    if (sum_ok && gps > 4) sum_groups(Int<1>{}, Int<4>{});
+    else if (sum_ok && gps > 1) sum_groups(Int<(NP * R >= 16 ? 4 : 1)>{}, Int<2>{});
+    else if (!kDirect && sum_ok && !clustered) sum_groups(Int<1>{}, Int<1>{});
   }
   if (a.chunks == 1) return;
 
@@ -450,7 +465,8 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     for (int q = 0; q < kSmallCluster; ++q)
       if (q < a.chunks) from[q] = cluster_map(static_cast<uint32_t>(__cvta_generic_to_shared(red_set)), q);
     const int step = set_threads * a.chunks;
-    for (int o = unit_ok ? t_in_set + chunk * set_threads : NP * N; o < NP * N; o += U * step) {
+    float* const out = result(sum_unit);
+    for (int o = sum_ok ? t_in_set + chunk * set_threads : NP * N; o < NP * N; o += U * step) {
       const int n = (NP * N - 1 - o) / step + 1;
       float f[U][kSmallCluster], s[U] = {};
 #pragma unroll
@@ -484,13 +500,14 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  if (!unit_ok) return;
+  if (!sum_ok) return;
   // U accesses of V outputs a thread and Q chunks at a time: the sum is a
   // chain of trips to L2 otherwise (four planes of 4096 points in 4 chunks: 64
   // trips, 12 us).
   constexpr int V = NP * N % 4 == 0 ? 4 : 1, U = NP * N >= 2048 ? 4 : 1, Q = U == 4 ? 2 : 8;
   const int step = set_threads * V;
-  const float* const base = a.partial + (size_t)unit * a.chunks * NP * N;
+  const float* const base = a.partial + (size_t)sum_unit * a.chunks * NP * N;
+  float* const out = result(sum_unit);
   for (int o = t_in_set * V; o < NP * N; o += step * U) {
     float s[U][V] = {};
     for (int q0 = 0; q0 < a.chunks; q0 += Q) {

@@ -93,3 +93,14 @@ def test_units_of_one_group(cuda_device, monkeypatch, nt, npol):
     check(5, 2, nt, 1, 8, [(nt, 2, npol)], buffers=4, fft_dir=-1, conj=1, seed=nt)
     check(3, 2, 3 * nt, 1, 16, [(nt, 1, npol)], seed=nt + 1)
     check(70, 2, 2 * nt, 1, 8, [(nt, 2, npol)], seed=nt + 2)
+
+
+# Fewer units than a CTA has sets of groups: their sums are shared out over all
+# of its threads, written and added, on one CTA and on more.
+@pytest.mark.parametrize("npol", [1, -4])
+@pytest.mark.parametrize("Nc,nt,na", [(1, 32, 4), (3, 32, 2), (5, 8, 4), (1, 64, 8), (2, 256, 3), (9, 16, 6), (1, 512, 2),
+                                      (1, 128, 300), (3, 16, 700)])
+def test_few_units(cuda_device, monkeypatch, Nc, nt, na, npol):
+    monkeypatch.setenv("RAWSPEC_GB300_TENSOR_DFT", "0")
+    check(Nc, 2, nt * na, 1, 8, [(nt, 2 * na, npol)], buffers=4, fft_dir=-1 if na % 2 else 1, conj=1, seed=nt)
+    check(Nc, 2, nt * na, 1, 16, [(nt, na, npol)], seed=nt + 1)
