@@ -35,7 +35,8 @@ struct SmallLaunch {
   int pol = POL_TP;  // PolMode
   // geometry (filled by small_configure)
   int sets = 1, chunks = 1, spc = 0;
-  int sms = 0;       // of the device (0: units are not summed within clusters)
+  int finalize = 0;  // the chunks' partial sums are left to finalize_launch
+  int sms = 0;       // of the device (0: clusters are pairs only)
   size_t smem = 0;
   // problem
   int Nc = 0, M = 0, units_per_chan = 0, n_units = 0;
@@ -54,7 +55,7 @@ struct SmallLaunch {
   int unit0 = 0, unit_count = 0;  // units of this launch (a channel range; all by default)
   // split of a unit for launches over a channel group (the pipelined path),
   // which see 1/pipe_groups of the units and need more CTAs per unit
-  int chunks_pipe = 1, spc_pipe = 0;
+  int chunks_pipe = 1, spc_pipe = 0, finalize_pipe = 0;
 };
 
 // Chooses block size, units per block and chunks per unit.  target_ctas is

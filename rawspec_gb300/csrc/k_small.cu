@@ -450,7 +450,7 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     else if (sum_ok && gps > 1) sum_groups(Int<(NP * R >= 16 ? 4 : 1)>{}, Int<2>{});
     else if (!kDirect && sum_ok && !clustered) sum_groups(Int<1>{}, Int<1>{});
   }
-  if (a.chunks == 1) return;
+  if (a.chunks == 1 || a.finalize) return;
 
   // Units spread over the CTAs of a cluster: every CTA keeps its sums where
   // the first group's were, and sums a share of the outputs over the chunks,
@@ -488,8 +488,9 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   // Units spread over more CTAs than a cluster holds, and the launches that
   // share a grid: the last CTA of the block of units to arrive sums
   // the chunks' partials in chunk order (the same order whichever CTA it is)
-  // and leaves the arrival counter zeroed for the next launch.  A kernel of
-  // its own for this sum cost a launch and a drained GPU, 6-10 us a product.
+  // and leaves the arrival counter zeroed for the next launch.  A kernel of its
+  // own for this sum costs a launch and a drained GPU, and is left for sums that
+  // take one CTA longer (SplitCost).
   __shared__ int s_last;
   __threadfence();
   __syncthreads();
@@ -620,7 +621,7 @@ cudaError_t launch_t(const SmallLaunch& L, cudaStream_t s, int op, int* occ, con
   }
   const int grid = small_grid(L);
   if (grid < 1) return cudaSuccess;
-  if (small_clustered(L.chunks, grid, L.sms)) {
+  if (!L.finalize && small_clustered(L.chunks, grid, L.sms)) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(C::TPB);
@@ -733,17 +734,19 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   p.max_partial = max_partial;
   p.max_arrivals = max_arrivals;
   const Split all = split_groups_and_chunks(p);
-  auto take = [&](const Split& s, int* spc, int* chunks) {
+  auto take = [&](const Split& s, int* spc, int* chunks, int* finalize) {
     const int per = (p.turns + s.chunks - 1) / s.chunks;  // iterations' worth of spectra per chunk
     *spc = std::min(L.M, per * si.SPI);
     *chunks = (p.turns + per - 1) / per;
+    *finalize = s.finalize;
   };
   L.sets = G / all.gps;
   const int ublocks = (L.n_units + L.sets - 1) / L.sets;
-  take(all, &L.spc, &L.chunks);
+  take(all, &L.spc, &L.chunks, &L.finalize);
   // the same for a launch over 1/pipe_groups of the units
   p.units = std::max(1, L.n_units / std::max(1, pipe_groups));
-  take(p.units == p.all_units ? all : split_chunks(p, all.gps), &L.spc_pipe, &L.chunks_pipe);
+  take(p.units == p.all_units ? all : split_chunks(p, all.gps), &L.spc_pipe, &L.chunks_pipe,
+       &L.finalize_pipe);
   const int cmax = std::max(L.chunks, L.chunks_pipe);
   *partial_floats = cmax > 1 ? (size_t)L.n_units * cmax * np * ((size_t)1 << L.logN) : 0;
   L.arrivals = cmax > 1 ? ublocks : 0;

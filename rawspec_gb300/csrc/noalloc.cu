@@ -192,6 +192,21 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
     e = stockham_twiddle_fill(tw, (int)Nt, small_radix(L.logN, L.pol), s);
   }
   if (e == cudaSuccess) e = small_launch(L, s);
+  if (e == cudaSuccess && L.finalize) {
+    FinalizeLaunch F;
+    F.partial = scratch;
+    F.out = d_out;
+    F.n_units = L.n_units;
+    F.chunks = L.chunks;
+    F.np = npol == 1 ? 1 : 4;
+    F.N = (int)Nt;
+    F.Nc = (int)Nc;
+    F.units_per_chan = L.units_per_chan;
+    F.mode = ACC_WRITE;
+    F.inverse = L.inverse;
+    F.scale = L.scale;
+    e = finalize_launch(F, s);
+  }
   if (e != cudaSuccess) {
     fprintf(stderr, "rawspec_gb300_product_noalloc: %s\n", cudaGetErrorName(e));
     return 1;

@@ -576,7 +576,7 @@ struct DeferredSmall {
 // Queues product i's kernels for the channels [c0, c1) of the buffer.  With
 // compensated integration the buffers after an integration's first write
 // their sums to the staging plane.  With `defer`, a k_small launch over all
-// channels is recorded there instead.
+// channels is recorded there instead (with its finalisation).
 int launch_product(rawspec_context* ctx, GpuCtx* g, int i, int mode, int inverse, int c0, int c1,
                    std::vector<DeferredSmall>* defer = nullptr) {
   Product& P = g->prod[i];
@@ -614,6 +614,7 @@ int launch_product(rawspec_context* ctx, GpuCtx* g, int i, int mode, int inverse
     if (c1 - c0 < (int)ctx->Nc) {  // a channel group: the finer split
       L.chunks = L.chunks_pipe;
       L.spc = L.spc_pipe;
+      L.finalize = L.finalize_pipe;
     } else if (defer && !g->profiling) {
       defer->push_back(DeferredSmall{ctx, g, i, L, out});
       return 0;
@@ -623,6 +624,9 @@ int launch_product(rawspec_context* ctx, GpuCtx* g, int i, int mode, int inverse
       RSG_CUDA(small_launch(L, P.stream));
       g->launches++;
     }
+    if (L.finalize &&
+        launch_finalize(ctx, g, P, out, L.unit0, L.unit_count, L.chunks, L.units_per_chan, mode, inverse, L.scale))
+      return 1;
   } else {
     LargeLaunch L = P.ll;
     L.out = out;
@@ -748,7 +752,8 @@ int process_buffer(rawspec_context* ctx, GpuCtx* g, int fft_dir, int ngroups, co
 // Queues the deferred k_small launches of several contexts: launches of the
 // same kernel configuration share one grid (up to kSmallGroupMax), issued on
 // the first one's product stream after every member's stream has reached
-// it; each member's stream then continues after the shared launch.
+// it; each member's stream then continues after the shared launch with its
+// own finalisation, where its split needs one.
 int launch_deferred(std::vector<DeferredSmall>& d) {
   std::vector<char> done(d.size(), 0);
   for (size_t a = 0; a < d.size(); a++) {
@@ -788,6 +793,10 @@ int launch_deferred(std::vector<DeferredSmall>& d) {
       DeferredSmall& e = d[m];
       e.g->launches++;  // every member's context counts the launch it took part in
       if (mem.size() > 1) e.g->shared_launches++;
+      Product& P = e.g->prod[e.product];
+      if (e.L.finalize && launch_finalize(e.ctx, e.g, P, e.out, e.L.unit0, e.L.unit_count, e.L.chunks,
+                                          e.L.units_per_chan, e.L.mode, e.L.inverse, e.L.scale))
+        return 1;
     }
   }
   return 0;

@@ -41,6 +41,7 @@ struct SplitProblem {
 };
 struct Split {
   int gps = 1, chunks = 1;
+  bool finalize = false;  // the chunks are summed by a kernel of its own
   double cost = 0;  // microseconds
 };
 
@@ -55,8 +56,13 @@ struct SplitCost {
   static int iterations(unsigned per, unsigned gps) { return (int)((per + gps - 1) / gps); }
   // CTAs of the most loaded SM with `ctas` in all.
   int on_one_sm(int ctas) const { return (int)((unsigned)(ctas + sms - 1) / (unsigned)sms); }
+  double by_last_cta(int c) const { return 2.0 + c * (partial + serial); }
+  double by_kernel(int c) const { return 4.0 + c * (partial + 0.04); }
+  bool finalize(int c, int ublocks) const {
+    return c > 1 && !small_clustered(c, ublocks * c, sms) && by_kernel(c) < by_last_cta(c);
+  }
   double sum(int c, int ublocks) const {
-    return c == 1 ? 0.0 : small_clustered(c, ublocks * c, sms) ? 1.5 : 2.0 + c * (partial + serial);
+    return c == 1 ? 0.0 : small_clustered(c, ublocks * c, sms) ? 1.5 : std::min(by_last_cta(c), by_kernel(c));
   }
   // SM time of an iteration of all of them, over that of one
   double load(int per_sm) const {
@@ -72,8 +78,10 @@ struct SplitCost {
 // 127 us, 512 twice as long ones in 143, 2560 in 124), plus about 0.6
 // iterations for a CTA's start and reduction; a CTA alone on its SM is bound
 // by its own latency, about 1.5 times its share of a full one.  A unit split
-// within a cluster adds about 1.5 us; one split over more CTAs an arrival, the
-// traffic of the partial sums and their sum by one CTA (120 GB/s).
+// within a cluster adds about 1.5 us; one split over more CTAs the traffic of the
+// partial sums, and an arrival and their sum by one CTA (36 GB/s) or a kernel
+// over all outputs.  One channel, 64 spectra of 4096 points in four planes: 8
+// chunks in a cluster 33 us, 32 and a kernel 19.
 //
 // Of the counts that load the SMs alike and leave a CTA as many iterations the
 // smallest is the best (the sum costs more with every chunk), so the search
@@ -134,6 +142,7 @@ inline Split split_chunks(const SplitProblem& p, int gps, int* tried = nullptr) 
   // partial sums are written and read at about 4 TB/s
   const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ};
   s.chunks = fit_chunks(p.turns, gps, ub, 1, std::max(1, most), k, &s.cost, tried);
+  s.finalize = k.finalize(s.chunks, ub);
   return s;
 }
 

@@ -18,7 +18,7 @@ static int fit_every(int turns, int gps, int ublocks, int c_lo, int c_hi, const 
     if (c > c_lo && (turns + per - 1) / per != c) continue;
     const double per_sm = std::ceil((double)ublocks * c / k.sms);
     const double load = std::max(per_sm, 1.5 * std::ceil(per_sm / k.occ));
-    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : 2.0 + c * (k.partial + k.serial);
+    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : std::min(2.0 + c * (k.partial + k.serial), 4.0 + c * (k.partial + 0.04));
     const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + sum;
     if (cost < best_cost * 0.99) {
       best_cost = cost;
@@ -98,8 +98,11 @@ int main() {
     every(p, &b);
     printf("tried %d of %d\n", a, b);
   }
-  // One unit's partial sums are summed by one CTA: more chunks than a cluster
-  // takes cost more than they save.
-  for (int n : {1024, 2048, 4096}) printf("chunks %d\n", split_groups_and_chunks(problem(n, 4, 1, 64, false)).chunks);
+  // One unit's partial sums, summed by one CTA, cost more than chunks beyond a
+  // cluster's save.
+  for (int n : {1024, 2048, 4096}) {
+    const Split s = split_groups_and_chunks(problem(n, 4, 1, 64, false));
+    printf("chunks %d %d\n", s.chunks, s.finalize ? 1 : 0);
+  }
   return differ != 0;
 }

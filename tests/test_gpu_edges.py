@@ -104,3 +104,31 @@ def test_few_units(cuda_device, monkeypatch, Nc, nt, na, npol):
     monkeypatch.setenv("RAWSPEC_GB300_TENSOR_DFT", "0")
     check(Nc, 2, nt * na, 1, 8, [(nt, 2 * na, npol)], buffers=4, fft_dir=-1 if na % 2 else 1, conj=1, seed=nt)
     check(Nc, 2, nt * na, 1, 16, [(nt, na, npol)], seed=nt + 1)
+
+
+# Units whose partial sums a kernel of its own adds, alone and in shared launches
+# (one channel, four planes), written and added.
+@pytest.mark.parametrize("nt,na,npol", [(4096, 64, 4), (2048, 70, -4), (4096, 129, 1)])
+def test_units_summed_by_a_kernel(cuda_device, monkeypatch, nt, na, npol):
+    monkeypatch.setenv("RAWSPEC_GB300_TENSOR_DFT", "0")
+    check(1, 2, nt * na, 1, 8, [(nt, 2 * na, npol)], buffers=4, fft_dir=-1, conj=1, seed=na)
+    rng = np.random.default_rng(na)
+    blocks = [codes(rng, (1, 1, nt * na, 2, 2), 8).view(np.uint8).reshape(1, -1) for _ in range(2)]
+    specs = [api.Spectrometer(1, 2, nt * na, 8, [(nt, na, npol)], Nb=1) for _ in blocks]
+    try:
+        alone = []
+        for spec, b in zip(specs, blocks):
+            spec.process(b)
+            alone.append(np.array(spec.dumps[0]))
+            spec.load_blocks(b)
+            spec.copy_to_gpu()
+        before = specs[0].kernel_launches()
+        api.start_group(specs, [1, 1])
+        for spec in specs:
+            assert spec.wait() == 0
+        assert specs[0].kernel_launches() - before == 2  # the shared launch and the sum
+        for spec, a in zip(specs, alone):
+            assert np.array_equal(np.array(spec.dumps[0])[-1:], a[-1:])
+    finally:
+        for spec in specs:
+            spec.close()

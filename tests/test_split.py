@@ -26,5 +26,5 @@ def test_split_is_that_of_every_count_at_a_few(probe):
 
 
 def test_one_unit_is_not_split_beyond_what_its_sum_costs(probe):
-    chunks = [int(line.split()[1]) for line in probe.stdout.splitlines() if line.startswith("chunks")]
-    assert len(chunks) == 3 and all(2 <= c <= 8 for c in chunks), probe.stdout
+    chunks = [line.split()[1:] for line in probe.stdout.splitlines() if line.startswith("chunks")]
+    assert len(chunks) == 3 and all(int(c) <= 8 or finalize == "1" for c, finalize in chunks), probe.stdout
