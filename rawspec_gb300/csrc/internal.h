@@ -228,6 +228,7 @@ struct GatherLaunch {
   void* dst = nullptr;                  // [Nc][Nb][row_bytes], twice that if expanded
   long long row_bytes = 0;              // bytes of a channel in a host block
   int Nc = 0, Nb = 0, dst_block = 0, num_blocks = 0, expand = 0;
+  int on_grid = 0;                      // every row starts and ends on 16 bytes
 };
 cudaError_t gather_launch(const GatherLaunch& L, cudaStream_t s);
 

@@ -208,8 +208,7 @@ __global__ void k_gather(const __grid_constant__ GatherLaunch a) {
   const char* src = static_cast<const char*>(a.src[b]) + (long long)c * a.row_bytes;
   const long long at = ((long long)c * a.Nb + (a.dst_block + b) % a.Nb) * a.row_bytes;
   const long long step = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool vec = ((reinterpret_cast<uintptr_t>(src) | (uintptr_t)a.row_bytes) & 15) == 0;
-  const long long n16 = vec ? a.row_bytes / 16 : 0;
+  const long long n16 = a.on_grid ? a.row_bytes / 16 : 0;
   if (a.expand) {
     int8_t* dst = static_cast<int8_t*>(a.dst) + 2 * at;
     for (long long i = first; i < n16; i += step) {
@@ -232,8 +231,8 @@ __global__ void k_gather(const __grid_constant__ GatherLaunch a) {
 }
 
 cudaError_t gather_launch(const GatherLaunch& L, cudaStream_t s) {
-  const long long units = std::max<long long>(1, L.row_bytes / 16);
-  const int gx = (int)std::max<long long>(1, std::min<long long>((units + 127) / 128, 64));
+  const long long units = L.on_grid ? L.row_bytes / 16 : L.row_bytes;
+  const int gx = (int)std::max<long long>(1, std::min<long long>((units + 127) / 128, L.on_grid ? 64 : 1024));
   k_gather<<<dim3(gx, (unsigned)L.Nc, (unsigned)L.num_blocks), 128, 0, s>>>(L);
   return cudaGetLastError();
 }

@@ -802,15 +802,31 @@ int launch_deferred(std::vector<DeferredSmall>& d) {
   return 0;
 }
 
-// Copies of at most this many host bytes are done by a kernel, larger ones by
-// the copy engines.  The corner turn, one product and its dump, us: 0.5 MiB in
-// 8 blocks 53 by the engines, 23 by the kernel; 2 MiB in 8 blocks 52 and 35; 4
-// MiB in one block 58 and 48 with the call alone, 35 both ways back to back; 8
-// MiB 77 and 74, 55 both ways; 16 MiB 130 both ways.
+// Whether a copy of at most kGatherBytes host bytes, num_blocks blocks of Nc rows
+// of `row` bytes, is faster by a kernel than by the copy engines.  Measured in
+// us from call to return over 692 shapes.  The engines take 8.5 and 1.75 a
+// block, at 205 GB/s or 0.32 ns a row, and for rows off the 16-byte grid 45 ns a
+// row (less for rows below 120 bytes); an expansion 3.5, at 1200 GB/s (off the
+// grid 200), and 0.5 ns a row up to 16.  The kernel takes 11.5, at 205 GB/s or
+// 0.51 ns a CTA (one or more a row), and off the grid, a byte a thread, at 80
+// GB/s (140 of one channel).  Engines and kernel: 64 KiB in 1, 4 and 16 blocks
+// 10.6 and 12.1, 17 and 12, 36 and 12; 8 MiB in 16 blocks 88 and 53; 1 MiB off
+// the grid in 64 rows 16 and 28, in 8192 rows 177 and 25; 32768 channels, 16
+// blocks, 16 bytes a row 205 and 277.
 constexpr size_t kGatherBytes = size_t(8) << 20;
+bool gather_wanted(size_t Nc, size_t num_blocks, size_t row, bool on_grid, bool expand) {
+  const double rows = (double)Nc * num_blocks, bytes = rows * row;
+  const double link = bytes / 205e3;  // us at 205 GB/s
+  const double expansion = expand ? 3.5 + bytes / (on_grid ? 1200e3 : 200e3) + std::min(16.0, rows * 0.5e-3) : 0.0;
+  const double off_grid = on_grid ? 0.0 : rows * 45e-3 * std::max(0.0, std::min(1.0, (row - 8.0) / 110.0));
+  const double engines = 8.5 + 1.75 * num_blocks + std::max(link, rows * 0.32e-3) + off_grid + expansion;
+  const double kernel =
+      11.5 + std::max({link, rows * 0.51e-3, on_grid ? row / 131e3 : bytes / (Nc == 1 ? 140e3 : 80e3)});
+  return kernel < engines;
+}
 
-// Queues the corner turn of a small copy as one kernel if it can be one: few
-// blocks, distinct destinations, and every block one that this context
+// Queues the corner turn of a small copy as one kernel if it can be one and is
+// faster so: few blocks, distinct destinations, and every block one that this context
 // page-locked (a caller may have put other memory in its place).  *done tells.
 int queue_gather(rawspec_context* ctx, GpuCtx* g, off_t src_idx, off_t dst_idx, size_t num_blocks, size_t row, bool expand,
                  bool* done) {
@@ -820,11 +836,14 @@ int queue_gather(rawspec_context* ctx, GpuCtx* g, off_t src_idx, off_t dst_idx, 
       row * (expand ? 2 : 1) * ctx->Nc * ctx->Nb > g->in_bytes)
     return 0;
   GatherLaunch L;
+  L.on_grid = row % 16 == 0;
   for (size_t b = 0; b < num_blocks; b++) {
     const size_t i = (size_t)((src_idx + (off_t)b) % ctx->Nb_host);
     if (i >= g->host_blocks.size() || !ctx->h_blkbufs[i] || g->host_blocks[i].first != ctx->h_blkbufs[i]) return 0;
     L.src[b] = g->host_blocks[i].second;
+    if (reinterpret_cast<uintptr_t>(L.src[b]) % 16) L.on_grid = 0;
   }
+  if (!gather_wanted(ctx->Nc, num_blocks, row, L.on_grid, expand)) return 0;
   L.dst = g->d_in;
   L.row_bytes = (long long)row;
   L.Nc = (int)ctx->Nc;

@@ -132,3 +132,22 @@ def test_units_summed_by_a_kernel(cuda_device, monkeypatch, nt, na, npol):
     finally:
         for spec in specs:
             spec.close()
+
+
+# A copy goes by the kernel or by the copy engines, whichever is the faster; the
+# bytes are the same.
+@pytest.mark.parametrize("Nc,Np,nbits,Ntpb,Nb,kernels", [(2, 1, 8, 262143, 1, 0), (3, 2, 8, 4096, 1, 0), (3, 2, 8, 4096, 4, 1),
+                                                         (3, 1, 8, 4095, 16, 1), (5, 2, 4, 4096, 1, 1), (5, 1, 4, 262143, 1, 0),
+                                                         (30000, 1, 8, 8, 4, 0), (600, 1, 8, 63, 4, 1)])
+def test_small_copies_by_kernel_or_engine(cuda_device, Nc, Np, nbits, Ntpb, Nb, kernels):
+    spec = api.Spectrometer(Nc, Np, Ntpb, nbits, [(1, Ntpb * Nb, 1)], Nb=Nb)
+    try:
+        spec.copy_to_gpu()
+        before = spec.kernel_launches()
+        spec.copy_to_gpu()
+        launched = spec.kernel_launches() - before
+    finally:
+        spec.close()
+    # the engines' copies of 4-bit samples are followed by their expansion
+    assert launched == (1 if nbits == 4 else kernels)
+    check(Nc, Np, Ntpb, Nb, nbits, [(1, Ntpb * Nb, 1)], buffers=1, seed=Ntpb)
