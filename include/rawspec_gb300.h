@@ -172,9 +172,9 @@ int rawspec_gb300_device_bytes_estimate(const rawspec_context *ctx, size_t *byte
  *   stream   cudaStream_t to queue the work on (0 = legacy default stream)
  *
  * Scratch: file-scope device arrays of 4 MiB of partial sums, a 4096-entry
- * twiddle table, arrival counters and the twiddle tables of every FFT length
- * (4.16 MiB in all), held by every GPU that loads the library until the
- * process exits.  The partial-sum split is limited to what fits; FFT lengths
+ * twiddle table and the twiddle tables of every FFT length (4.13 MiB in all),
+ * held by every GPU that loads the library until the process exits.  The
+ * partial-sum split is limited to what fits; FFT lengths
  * above 4096 are rejected with an error.  The first call on a device looks up
  * the arrays' device addresses, fills the twiddle tables on its stream and
  * waits for that (make that first call before any stream capture on that
@@ -186,7 +186,8 @@ int rawspec_gb300_device_bytes_estimate(const rawspec_context *ctx, size_t *byte
  * runtime's); after cudaDeviceReset the library must be reloaded before this
  * entry point is used again.
  * Calls that overlap on the GPU (different streams, or another host thread)
- * race on the array and must be serialised by the caller.
+ * race on the sums and must be serialised by the caller; they spoil their own
+ * results, not those of later calls.
  * Returns 0 when the work is queued, 1 on invalid arguments or a CUDA error
  * (message on stderr). */
 int rawspec_gb300_product_noalloc(const void *d_in, unsigned int Nc, unsigned int Np,

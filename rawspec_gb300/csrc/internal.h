@@ -61,9 +61,10 @@ struct SmallLaunch {
 // Chooses block size, units per block and chunks per unit.  target_ctas is
 // the number of CTAs that fills the GPU.  Returns 0, or -1 if N is out of
 // range.  partial_floats receives the scratch the launch needs (0 if none),
-// which max_partial (floats) and max_arrivals limit where they are not 0.
+// which max_partial (floats) limits where it is not 0.  Without `counters` no
+// launch uses arrival counters.
 int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int pipe_groups = 1,
-                    size_t max_partial = 0, int max_arrivals = 0);
+                    size_t max_partial = 0, bool counters = true);
 cudaError_t small_launch(const SmallLaunch& L, cudaStream_t s);
 // Up to kSmallGroupMax launches of the same kernel configuration (FFT length,
 // sample format, polarisations, mode) in one grid, e.g. the buffers of

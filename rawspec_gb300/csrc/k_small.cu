@@ -709,7 +709,7 @@ void resident_ctas(const SmallLaunch& L, int* occ, int* sms) {
 int small_radix(int logN, int pol) { return small_r(1 << logN, pol == POL_TP ? 1 : 4); }
 
 int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int pipe_groups, size_t max_partial,
-                    int max_arrivals) {
+                    bool counters) {
   if (L.logN < 0 || L.logN > 12 || L.M < 1 || L.n_units < 1) return -1;
   SmallInfo si{};
   if (small_dispatch(L, nullptr, 4, nullptr, nullptr, &si) != cudaSuccess) return -1;
@@ -732,13 +732,13 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   // a sample of both lanes takes about 2.3 ps of the GPU
   p.unit_us = si.TPB * si.R * sms * 2.3e-6;
   p.max_partial = max_partial;
-  p.max_arrivals = max_arrivals;
+  p.counters = counters;
   const Split all = split_groups_and_chunks(p);
   auto take = [&](const Split& s, int* spc, int* chunks, int* finalize) {
     const int per = (p.turns + s.chunks - 1) / s.chunks;  // iterations' worth of spectra per chunk
     *spc = std::min(L.M, per * si.SPI);
     *chunks = (p.turns + per - 1) / per;
-    *finalize = s.finalize;
+    *finalize = s.finalize && *chunks > 1;
   };
   L.sets = G / all.gps;
   const int ublocks = (L.n_units + L.sets - 1) / L.sets;
@@ -749,7 +749,7 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
        &L.finalize_pipe);
   const int cmax = std::max(L.chunks, L.chunks_pipe);
   *partial_floats = cmax > 1 ? (size_t)L.n_units * cmax * np * ((size_t)1 << L.logN) : 0;
-  L.arrivals = cmax > 1 ? ublocks : 0;
+  L.arrivals = counters && cmax > 1 ? ublocks : 0;
   L.unit0 = 0;
   L.unit_count = L.n_units;
   const long long wbytes = (L.fmt == FMT_I16 ? 4 : 2) * L.nv;

@@ -6,9 +6,15 @@
 // other stream of the process), or a host framework that owns all device
 // memory through its own pool and budget.  This entry point takes the input
 // and output as caller-provided device pointers and keeps its only scratch --
-// the per-chunk partial sums of the fused small-FFT kernel, its twiddle tables
-// and its arrival counters -- in the file-scope arrays below, which every GPU
-// that loads the library holds until the process exits.
+// the per-chunk partial sums of the fused small-FFT kernel and its twiddle
+// tables -- in the file-scope arrays below, which every GPU that loads the
+// library holds until the process exits.
+//
+// Nothing but the tables is kept from one call for the next: units split over
+// more CTAs than a cluster are summed by a kernel of their own, not by the last
+// CTA to arrive, whose counter two calls that overlap by mistake would leave
+// wrong for all calls after them (1 channel, 131072 spectra of 8 points in four
+// planes: 24.2 us, by the last CTA 23.2).
 #include <cstdint>
 #include <cstdio>
 #include <mutex>
@@ -21,15 +27,14 @@ namespace {
 constexpr size_t kPartialFloats = size_t(1) << 20;  // 4 MiB of partial sums
 constexpr int kMaxLogNt = 12;
 constexpr int kMaxNt = 1 << kMaxLogNt;              // twiddle table capacity of one call
-constexpr int kArrivals = 8192;                     // arrival counters of split units, zero between calls
 constexpr int kTableEntries = 3 * kMaxNt;           // the tables of every FFT length and mode
-constexpr size_t kScratchFloats = kPartialFloats + 2 * (size_t)kMaxNt + kArrivals;
+constexpr size_t kScratchFloats = kPartialFloats + 2 * (size_t)kMaxNt;
 constexpr int kMaxDevices = 64;
 
 }  // namespace
 
-// The shared scratch (zero when the library is loaded): partial sums [0,
-// kPartialFloats), one call's twiddles after them, then the arrival counters.
+// The shared scratch: partial sums [0, kPartialFloats), one call's twiddles
+// after them.
 static __device__ __align__(256) float g_noalloc_scratch[kScratchFloats];
 // Twiddle tables of every FFT length, for total power and for the four
 // planes, filled by the first call on a device outside a stream capture.
@@ -164,7 +169,6 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
   L.in = d_in;
   L.out = d_out;
   L.partial = scratch;
-  L.arrived = reinterpret_cast<unsigned*>(scratch + kPartialFloats + 2 * (size_t)kMaxNt);
   L.mode = ACC_WRITE;
   L.inverse = fft_dir <= 0 ? 1 : 0;
   L.conj = input_conjugated ? 1 : 0;
@@ -173,10 +177,9 @@ extern "C" int rawspec_gb300_product_noalloc(const void* d_in, unsigned int Nc, 
 
   int sms = 152;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // Units are split over CTAs only as far as the partial sums and the arrival
-  // counters fit the scratch.
+  // Units are split over CTAs only as far as the partial sums fit the scratch.
   size_t need = 0;
-  if (small_configure(L, sms * 4, &need, 1, kPartialFloats, kArrivals) != 0) {
+  if (small_configure(L, sms * 4, &need, 1, kPartialFloats, false) != 0) {
     fprintf(stderr, "rawspec_gb300_product_noalloc: unsupported configuration\n");
     return 1;
   }

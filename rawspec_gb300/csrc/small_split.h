@@ -37,7 +37,7 @@ struct SplitProblem {
   int sms = 0, occ = 0; // of the device, and resident CTAs per SM (0: unknown)
   double unit_us = 0;   // SM time of one iteration of a CTA
   std::size_t max_partial = 0;  // floats of partial sums (0: no limit)
-  int max_arrivals = 0;         // arrival counters (0: no limit)
+  bool counters = true;         // arrival counters: a unit's last CTA may sum it
 };
 struct Split {
   int gps = 1, chunks = 1;
@@ -51,6 +51,7 @@ struct SplitCost {
   double partial;  // traffic of one chunk's partial sums of every unit
   double serial;   // the last CTA's reading of one chunk's partial sums
   int sms, occ;
+  bool counters;
 
   // Iterations of a CTA with `per` turns.
   static int iterations(unsigned per, unsigned gps) { return (int)((per + gps - 1) / gps); }
@@ -59,10 +60,12 @@ struct SplitCost {
   double by_last_cta(int c) const { return 2.0 + c * (partial + serial); }
   double by_kernel(int c) const { return 4.0 + c * (partial + 0.04); }
   bool finalize(int c, int ublocks) const {
-    return c > 1 && !small_clustered(c, ublocks * c, sms) && by_kernel(c) < by_last_cta(c);
+    return c > 1 && !small_clustered(c, ublocks * c, sms) && (!counters || by_kernel(c) < by_last_cta(c));
   }
   double sum(int c, int ublocks) const {
-    return c == 1 ? 0.0 : small_clustered(c, ublocks * c, sms) ? 1.5 : std::min(by_last_cta(c), by_kernel(c));
+    if (c == 1) return 0.0;
+    if (small_clustered(c, ublocks * c, sms)) return 1.5;
+    return counters ? std::min(by_last_cta(c), by_kernel(c)) : by_kernel(c);
   }
   // SM time of an iteration of all of them, over that of one
   double load(int per_sm) const {
@@ -126,21 +129,22 @@ inline int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const
 // Chunks of a launch with `gps` groups per unit.
 inline Split split_chunks(const SplitProblem& p, int gps, int* tried = nullptr) {
   const int sets = p.groups / gps;
-  const int all = (p.all_units + sets - 1) / sets, ub = (p.units + sets - 1) / sets;
+  const int ub = (p.units + sets - 1) / sets;
   const int aim = std::max(1, (p.target_ctas + ub - 1) / ub);  // chunks that fill the GPU
-  // partial sums that fit the limit and the arrival counters
+  // partial sums that fit the limit
   const long long floats = (long long)p.all_units * p.planes * p.n;
   int most = (int)std::min<long long>((p.turns + gps - 1) / gps, std::max(8, 4 * aim));
   if (p.max_partial) most = (int)std::min<long long>(most, std::max<long long>(1, (long long)p.max_partial / floats));
-  if (p.max_arrivals && all > p.max_arrivals) most = 1;
   Split s;
   s.gps = gps;
   if (p.occ <= 0) {
     s.chunks = std::max(1, std::min(aim, most));
+    s.finalize = s.chunks > 1 && !p.counters;
     return s;
   }
   // partial sums are written and read at about 4 TB/s
-  const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ};
+  const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ,
+                    p.counters};
   s.chunks = fit_chunks(p.turns, gps, ub, 1, std::max(1, most), k, &s.cost, tried);
   s.finalize = k.finalize(s.chunks, ub);
   return s;

@@ -18,7 +18,7 @@ static int fit_every(int turns, int gps, int ublocks, int c_lo, int c_hi, const 
     if (c > c_lo && (turns + per - 1) / per != c) continue;
     const double per_sm = std::ceil((double)ublocks * c / k.sms);
     const double load = std::max(per_sm, 1.5 * std::ceil(per_sm / k.occ));
-    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : std::min(2.0 + c * (k.partial + k.serial), 4.0 + c * (k.partial + 0.04));
+    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : std::min(k.counters ? 2.0 + c * (k.partial + k.serial) : 1e300, 4.0 + c * (k.partial + 0.04));
     const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + sum;
     if (cost < best_cost * 0.99) {
       best_cost = cost;
@@ -35,13 +35,12 @@ static Split every(const SplitProblem& p, int* tried) {
   Split best;
   for (int gps = most; gps >= 1; gps /= 2) {
     const int sets = p.groups / gps;
-    const int ub = (p.units + sets - 1) / sets, all = (p.all_units + sets - 1) / sets;
+    const int ub = (p.units + sets - 1) / sets;
     const int aim = std::max(1, (p.target_ctas + ub - 1) / ub);
     const long long floats = (long long)p.all_units * p.planes * p.n;
     int c_hi = (int)std::min<long long>((p.turns + gps - 1) / gps, std::max(8, 4 * aim));
     if (p.max_partial) c_hi = (int)std::min<long long>(c_hi, std::max<long long>(1, (long long)p.max_partial / floats));
-    if (p.max_arrivals && all > p.max_arrivals) c_hi = 1;
-    const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ};
+    const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ, p.counters};
     Split s;
     s.gps = gps;
     s.chunks = fit_every(p.turns, gps, ub, 1, std::max(1, c_hi), k, &s.cost, tried);
@@ -65,7 +64,7 @@ static SplitProblem problem(int n, int planes, int units, int turns, bool limits
   p.unit_us = tpb * p.radix * 152 * 2.3e-6;
   if (limits) {
     p.max_partial = 1 << 20;
-    p.max_arrivals = 8192;
+    p.counters = false;
   }
   return p;
 }
@@ -82,6 +81,12 @@ int main() {
     int a = 0, b = 0;
     const Split s = split_groups_and_chunks(p, &a), e = every(p, &b);
     ++compared;
+    // without counters nothing but a cluster or a kernel sums the chunks
+    const int sets = p.groups / s.gps, ub = (p.units + sets - 1) / sets;
+    if (!p.counters && s.chunks > 1 && !s.finalize && !small_clustered(s.chunks, ub * s.chunks, p.sms)) {
+      ++differ;
+      printf("counters used: n %d planes %d units %d turns %d\n", n, planes, units, turns);
+    }
     if (s.gps != e.gps || s.chunks != e.chunks || s.cost != e.cost) {
       if (++differ <= 10)
         printf("differ n %d planes %d units %d turns %d: %d x %d, every count %d x %d\n", n, planes, units, turns, s.gps,
