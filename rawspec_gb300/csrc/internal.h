@@ -148,7 +148,7 @@ struct LargeLaunch {
   float* partial = nullptr;
   const float2* twN2 = nullptr;   // pass-ordered Stockham table of the N2-point FFT
   const float2* twN1 = nullptr;   // pass-ordered Stockham table of the N1-point FFT
-  const float2* twLo = nullptr;   // W_N^i, i < 2^h
+  const float2* twLo = nullptr;   // f W_N^i, i < 2^h: f = 1, or f^2 scale the codes' unit and `scale` a power of two
   const float2* twHi = nullptr;   // W_N^(i*2^h), i < N / 2^h
   const float2* twM = nullptr;    // [m][n1] = W_N^(n1*m*T2), m < R_A, the pass-A output twiddles
   int h = 0;
@@ -202,7 +202,7 @@ cudaError_t large_fused_launch(const LargeLaunch& L, cudaStream_t s);
 // ---------------------------------------------------------------------------
 // W_n^m = exp(-2 pi i m stride / n) for m < count, computed in FP64 with
 // sincospi and rounded to float.
-cudaError_t twiddle_fill(float2* dst, long long count, long long n, long long stride, cudaStream_t s);
+cudaError_t twiddle_fill(float2* dst, long long count, long long n, long long stride, double factor, cudaStream_t s);
 // Pass-ordered Stockham table of an N-point GroupFFT of radix R.
 cudaError_t stockham_twiddle_fill(float2* dst, int N, int R, cudaStream_t s);
 // dst[m*N1 + n1] = W_N^((n1*m*T) mod N) for m < R, n1 < N1.

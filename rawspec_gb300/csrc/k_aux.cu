@@ -8,21 +8,21 @@
 
 namespace rsg {
 
-// W_n^(m*stride) = exp(-2 pi i m stride / n), FP64 sincospi rounded to float.
-// Used only when a context is initialised.
-__global__ void k_twiddle(float2* dst, long long count, long long n, long long stride) {
+// factor * W_n^(m*stride), W_n = exp(-2 pi i / n), FP64 sincospi rounded to
+// float.  Used only when a context is initialised.
+__global__ void k_twiddle(float2* dst, long long count, long long n, long long stride, double factor) {
   for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < count;
        m += (long long)gridDim.x * blockDim.x) {
     const long long e = (m * stride) % n;
     double s, c;
     sincospi(2.0 * (double)e / (double)n, &s, &c);
-    dst[m] = make_float2((float)c, (float)(-s));
+    dst[m] = make_float2((float)(factor * c), (float)(-factor * s));
   }
 }
 
-cudaError_t twiddle_fill(float2* dst, long long count, long long n, long long stride, cudaStream_t s) {
+cudaError_t twiddle_fill(float2* dst, long long count, long long n, long long stride, double factor, cudaStream_t s) {
   const int blocks = (int)std::min<long long>((count + 255) / 256, 4096);
-  k_twiddle<<<std::max(blocks, 1), 256, 0, s>>>(dst, count, n, stride);
+  k_twiddle<<<std::max(blocks, 1), 256, 0, s>>>(dst, count, n, stride, factor);
   return cudaGetLastError();
 }
 

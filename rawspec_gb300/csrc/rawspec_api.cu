@@ -1298,11 +1298,17 @@ int rawspec_initialize(rawspec_context* ctx) {
       L.twHi = P.d_tw + o_hi;
       L.twM = P.d_tw + o_m;
       L.twJ = P.fused ? P.d_tw + o_j : nullptr;
-      L.scale = scale;
+      // Over several buffers the two kernels leave a power of two to the results
+      // (2^-14, 2^-30), by which a sum is multiplied without rounding, so that it
+      // enters the running sum with one; the rest of 1/127^2 or 1/32767^2 is in
+      // their twiddles.
+      const bool split_scale = !P.fused && P.Nis > 1;
+      const double unit = ctx->Nbps == 16 ? 32768.0 : 128.0;
+      L.scale = split_scale ? (float)(1.0 / (unit * unit)) : scale;
       CK(stockham_twiddle_fill(P.d_tw, n2, RA, g->stream));
       CK(stockham_twiddle_fill(P.d_tw + o_tb, n1, RB, g->stream));
-      CK(twiddle_fill(P.d_tw + o_lo, (long long)nlo, (long long)P.N, 1, g->stream));
-      CK(twiddle_fill(P.d_tw + o_hi, (long long)nhi, (long long)P.N, (long long)nlo, g->stream));
+      CK(twiddle_fill(P.d_tw + o_lo, (long long)nlo, (long long)P.N, 1, split_scale ? unit / (unit - 1.0) : 1.0, g->stream));
+      CK(twiddle_fill(P.d_tw + o_hi, (long long)nhi, (long long)P.N, (long long)nlo, 1.0, g->stream));
       CK(passa_twiddle_fill(P.d_tw + o_m, n1, RA, (long long)(n2 / RA), (long long)P.N, g->stream));
       if (P.fused) CK(passa_twiddle_fill(P.d_tw + o_j, n1, n2 / RA, 1, (long long)P.N, g->stream));
       if (P.fused) {

@@ -2,6 +2,8 @@
 
 The tolerance of the parity tests is a hundred times the rounding of an FP32
 transform; these tests hold the rounding itself."""
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
@@ -45,3 +47,40 @@ def test_twiddles_add_no_error(cuda_device, nt, na, npol, before):
     err = rms_error(64, 2, nt, na, npol)
     print(f"{nt} points, {na} spectra, Npolout {npol}: {err:.2e}")
     assert err < 1.1 * before
+
+
+def f32(x):
+    """The float32 nearest to an exact value (a Fraction)."""
+    y = np.float32(float(x))
+    near = [np.nextafter(y, np.float32(-np.inf)), y, np.nextafter(y, np.float32(np.inf))]
+    return min(near, key=lambda v: (abs(Fraction(float(v)) - x), int(v.view(np.int32)) & 1))
+
+
+# A buffer's sum enters the running sum of the two-kernel path with one rounding.
+# Constant voltages show every one of them: bin 0 of a transform is N times the
+# code, times 128/127 in the twiddles; its square, the sum of the spectra and the
+# running sum round, the scale 2^-14 does not.  (With the scale 1/127^2 as a
+# float the product with it rounded as well.)
+@pytest.mark.parametrize("Nc,logn,na,fft_dir", [(1, 16, 1, 1), (1, 16, 1, -1), (1, 16, 3, 1), (2, 13, 3, -1), (1, 20, 2, 1)])
+def test_sums_are_added_with_one_rounding(cuda_device, Nc, logn, na, fft_dir):
+    nt = 1 << logn
+    f = f32(Fraction(128, 127))
+    for c1, c2 in ((1, 3), (7, 43), (10, 92), (37, 120), (64, 43), (118, 106)):
+        x = np.zeros((2, Nc, nt * na, 1, 2), np.int8)
+        x[0, ..., 0], x[1, ..., 1] = c1, c2
+        spec = api.Spectrometer(Nc, 1, nt * na, 8, [(nt, 2 * na, 1)], Nb=1)
+        try:
+            assert spec.product_kernel(0) == "large_a"
+            spec.process(x.view(np.uint8).reshape(2, -1), fft_dir=fft_dir)
+            got = np.array(spec.dumps[0]).reshape(Nc, nt)
+        finally:
+            spec.close()
+        sums = []
+        for c in (c1, c2):
+            v = f32(Fraction(float(f)) * c)
+            p, s = f32(Fraction(float(v)) ** 2), np.float32(0)
+            for _ in range(na):
+                s = f32(Fraction(float(s)) + Fraction(float(p)))
+            sums.append(Fraction(float(s)))
+        want = float(f32(sum(sums))) * nt ** 2 / 2 ** 14
+        assert np.all(got[:, nt // 2] == want), (c1, c2, got[:, nt // 2], want)
