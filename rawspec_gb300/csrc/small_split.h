@@ -51,21 +51,17 @@ struct SplitCost {
   double partial;  // traffic of one chunk's partial sums of every unit
   double serial;   // the last CTA's reading of one chunk's partial sums
   int sms, occ;
-  bool counters;
+  bool kernel;     // chunks beyond a cluster are summed by a kernel, not by the last CTA
 
   // Iterations of a CTA with `per` turns.
   static int iterations(unsigned per, unsigned gps) { return (int)((per + gps - 1) / gps); }
   // CTAs of the most loaded SM with `ctas` in all.
   int on_one_sm(int ctas) const { return (int)((unsigned)(ctas + sms - 1) / (unsigned)sms); }
-  double by_last_cta(int c) const { return 2.0 + c * (partial + serial); }
-  double by_kernel(int c) const { return 4.0 + c * (partial + 0.04); }
-  bool finalize(int c, int ublocks) const {
-    return c > 1 && !small_clustered(c, ublocks * c, sms) && (!counters || by_kernel(c) < by_last_cta(c));
-  }
+  bool finalize(int c, int ublocks) const { return kernel && c > 1 && !small_clustered(c, ublocks * c, sms); }
   double sum(int c, int ublocks) const {
     if (c == 1) return 0.0;
     if (small_clustered(c, ublocks * c, sms)) return 1.5;
-    return counters ? std::min(by_last_cta(c), by_kernel(c)) : by_kernel(c);
+    return kernel ? 4.0 + c * (partial + 0.04) : 2.0 + c * (partial + serial);
   }
   // SM time of an iteration of all of them, over that of one
   double load(int per_sm) const {
@@ -83,8 +79,7 @@ struct SplitCost {
 // by its own latency, about 1.5 times its share of a full one.  A unit split
 // within a cluster adds about 1.5 us; one split over more CTAs the traffic of the
 // partial sums, and an arrival and their sum by one CTA (36 GB/s) or a kernel
-// over all outputs.  One channel, 64 spectra of 4096 points in four planes: 8
-// chunks in a cluster 33 us, 32 and a kernel 19.
+// over all outputs.
 //
 // Of the counts that load the SMs alike and leave a CTA as many iterations the
 // smallest is the best (the sum costs more with every chunk), so the search
@@ -126,7 +121,20 @@ inline int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const
   return best;
 }
 
-// Chunks of a launch with `gps` groups per unit.
+// All turns of all units over all SMs: no split takes less.
+inline double least_us(const SplitProblem& p, int gps) {
+  const int sets = p.groups / gps, ub = (p.units + sets - 1) / sets;
+  return p.turns * (double)ub * p.unit_us / ((double)gps * p.sms);
+}
+
+// Chunks of a launch with `gps` groups per unit.  A kernel of its own for the sum
+// of the chunks is a launch behind a drained GPU, against a CTA that others' work
+// can hide, so it is taken only where the GPU idles: where the best split without
+// one takes kIdle times the least.  One channel, 64 spectra of 4096 points in four
+// planes (a thirtieth of it busy): 8 chunks in a cluster 33 us, 32 and a kernel
+// 19; 8 channels x 256 spectra (a third): a pass among others 36 us without the
+// kernel, 41 with it.
+constexpr double kIdle = 8.0;
 inline Split split_chunks(const SplitProblem& p, int gps, int* tried = nullptr) {
   const int sets = p.groups / gps;
   const int ub = (p.units + sets - 1) / sets;
@@ -135,18 +143,29 @@ inline Split split_chunks(const SplitProblem& p, int gps, int* tried = nullptr) 
   const long long floats = (long long)p.all_units * p.planes * p.n;
   int most = (int)std::min<long long>((p.turns + gps - 1) / gps, std::max(8, 4 * aim));
   if (p.max_partial) most = (int)std::min<long long>(most, std::max<long long>(1, (long long)p.max_partial / floats));
+  most = std::max(1, most);
   Split s;
   s.gps = gps;
   if (p.occ <= 0) {
-    s.chunks = std::max(1, std::min(aim, most));
+    s.chunks = std::min(aim, most);
     s.finalize = s.chunks > 1 && !p.counters;
     return s;
   }
   // partial sums are written and read at about 4 TB/s
-  const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ,
-                    p.counters};
-  s.chunks = fit_chunks(p.turns, gps, ub, 1, std::max(1, most), k, &s.cost, tried);
+  SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ,
+              !p.counters};
+  s.chunks = fit_chunks(p.turns, gps, ub, 1, most, k, &s.cost, tried);
   s.finalize = k.finalize(s.chunks, ub);
+  if (p.counters && s.cost > kIdle * least_us(p, gps)) {
+    k.kernel = true;
+    double cost = 0.0;
+    const int c = fit_chunks(p.turns, gps, ub, 1, most, k, &cost, tried);
+    if (cost < s.cost) {
+      s.chunks = c;
+      s.cost = cost;
+      s.finalize = k.finalize(c, ub);
+    }
+  }
   return s;
 }
 
@@ -161,9 +180,7 @@ inline Split split_groups_and_chunks(const SplitProblem& p, int* tried = nullptr
   const int most = std::min(p.groups, std::min(pow2_floor(p.planes * p.radix), pow2_floor(p.turns)));
   Split best = split_chunks(p, most, tried);
   for (int gps = most / 2; gps >= 1 && p.occ > 0; gps /= 2) {
-    // All turns of all units over all SMs: no split takes less.
-    const int sets = p.groups / gps, ub = (p.units + sets - 1) / sets;
-    if (0.999 * p.turns * ub * p.unit_us / ((double)gps * p.sms) >= 0.95 * best.cost) continue;
+    if (0.999 * least_us(p, gps) >= 0.95 * best.cost) continue;
     const Split s = split_chunks(p, gps, tried);
     if (s.cost < 0.95 * best.cost) best = s;
   }

@@ -18,7 +18,7 @@ static int fit_every(int turns, int gps, int ublocks, int c_lo, int c_hi, const 
     if (c > c_lo && (turns + per - 1) / per != c) continue;
     const double per_sm = std::ceil((double)ublocks * c / k.sms);
     const double load = std::max(per_sm, 1.5 * std::ceil(per_sm / k.occ));
-    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : std::min(k.counters ? 2.0 + c * (k.partial + k.serial) : 1e300, 4.0 + c * (k.partial + 0.04));
+    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : k.kernel ? 4.0 + c * (k.partial + 0.04) : 2.0 + c * (k.partial + k.serial);
     const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + sum;
     if (cost < best_cost * 0.99) {
       best_cost = cost;
@@ -40,10 +40,16 @@ static Split every(const SplitProblem& p, int* tried) {
     const long long floats = (long long)p.all_units * p.planes * p.n;
     int c_hi = (int)std::min<long long>((p.turns + gps - 1) / gps, std::max(8, 4 * aim));
     if (p.max_partial) c_hi = (int)std::min<long long>(c_hi, std::max<long long>(1, (long long)p.max_partial / floats));
-    const SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ, p.counters};
+    SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ, !p.counters};
     Split s;
     s.gps = gps;
     s.chunks = fit_every(p.turns, gps, ub, 1, std::max(1, c_hi), k, &s.cost, tried);
+    double cost = 0.0;
+    if (p.counters && s.cost > kIdle * least_us(p, gps)) {
+      k.kernel = true;
+      const int c = fit_every(p.turns, gps, ub, 1, std::max(1, c_hi), k, &cost, tried);
+      if (cost < s.cost) s.chunks = c, s.cost = cost;
+    }
     if (gps == most || s.cost < 0.95 * best.cost) best = s;
   }
   return best;
