@@ -68,6 +68,18 @@ float* scratch_for_device(int dev) {
   return g_scratch_ptr[dev];
 }
 
+// Where the table of every FFT length starts, for total power and four planes.
+struct TableOffsets {
+  int offset[2][kMaxLogNt + 1], total = 0;
+  TableOffsets() {
+    for (int m = 0; m < 2; ++m)
+      for (int l = 0; l <= kMaxLogNt; ++l) {
+        offset[m][l] = total;
+        total += (rsg::stockham_table_size(1 << l, rsg::small_radix(l, m == 0 ? rsg::POL_TP : rsg::POL_FULL)) + 1) & ~1;
+      }
+  }
+};
+
 // The twiddle table of an FFT length and mode on the current device, or null
 // where it has to be filled for the call (a first call inside a stream
 // capture, or an error).  The first call outside one fills all of them and
@@ -76,13 +88,9 @@ float* scratch_for_device(int dev) {
 const float2* twiddles_for(int dev, int logN, int pol, cudaStream_t s) {
   using namespace rsg;
   std::lock_guard<std::mutex> lock(g_mu);
-  int offset[2][kMaxLogNt + 1], total = 0;
-  for (int m = 0; m < 2; ++m)
-    for (int l = 0; l <= kMaxLogNt; ++l) {
-      offset[m][l] = total;
-      total += (stockham_table_size(1 << l, small_radix(l, m == 0 ? POL_TP : POL_FULL)) + 1) & ~1;
-    }
-  if (total > kTableEntries) return nullptr;
+  static const TableOffsets T;
+  const auto& offset = T.offset;
+  if (T.total > kTableEntries) return nullptr;
   if (!g_tables_filled[dev]) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
