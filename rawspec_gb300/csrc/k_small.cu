@@ -726,6 +726,7 @@ int small_configure(SmallLaunch& L, int target_ctas, size_t* partial_floats, int
   p.planes = np;
   p.n = 1 << L.logN;
   p.radix = si.R;
+  p.threads = si.TPB;
   p.target_ctas = target_ctas;
   p.sms = sms;
   p.occ = occ;

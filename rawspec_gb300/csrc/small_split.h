@@ -33,6 +33,7 @@ struct SplitProblem {
   int all_units = 1;    // of the product (what the scratch is sized for)
   int groups = 1;       // of a CTA
   int planes = 1, n = 1, radix = 1;  // output planes, FFT length, values per thread
+  int threads = 1;      // of a CTA
   int target_ctas = 1;  // CTAs that fill the GPU
   int sms = 0, occ = 0; // of the device, and resident CTAs per SM (0: unknown)
   double unit_us = 0;   // SM time of one iteration of a CTA
@@ -50,6 +51,7 @@ struct SplitCost {
   double unit;     // SM time of one iteration of a CTA
   double partial;  // traffic of one chunk's partial sums of every unit
   double serial;   // the last CTA's reading of one chunk's partial sums
+  double outputs;  // of a CTA's units, for each of its threads
   int sms, occ;
   bool kernel;     // chunks beyond a cluster are summed by a kernel, not by the last CTA
 
@@ -60,7 +62,7 @@ struct SplitCost {
   bool finalize(int c, int ublocks) const { return kernel && c > 1 && !small_clustered(c, ublocks * c, sms); }
   double sum(int c, int ublocks) const {
     if (c == 1) return 0.0;
-    if (small_clustered(c, ublocks * c, sms)) return 1.5;
+    if (small_clustered(c, ublocks * c, sms)) return 0.5 + 0.15 * outputs / c;
     return kernel ? 4.0 + c * (partial + 0.04) : 2.0 + c * (partial + serial);
   }
   // SM time of an iteration of all of them, over that of one
@@ -77,22 +79,39 @@ struct SplitCost {
 // 127 us, 512 twice as long ones in 143, 2560 in 124), plus about 0.6
 // iterations for a CTA's start and reduction; a CTA alone on its SM is bound
 // by its own latency, about 1.5 times its share of a full one.  A unit split
-// within a cluster adds about 1.5 us; one split over more CTAs the traffic of the
-// partial sums, and an arrival and their sum by one CTA (36 GB/s) or a kernel
+// within a cluster adds about 0.5 us and 0.15 for each output that a thread sums
+// (two spectra of 4096 points in four planes: one CTA 10.3 us a call, a pair, 32
+// outputs a thread, 14.4); one split over more CTAs the traffic of the partial sums, and an arrival and their sum by one CTA (36 GB/s) or a kernel
 // over all outputs.
 //
-// Of the counts that load the SMs alike and leave a CTA as many iterations the
-// smallest is the best (the sum costs more with every chunk), so the search
-// goes from one such count to the next with few enough iterations to win, and
-// over all that load them alike if the fewest among them would not.  *tried:
-// counts looked at.
+// Counts of a cluster are all looked at.  Of larger ones that load the SMs alike
+// and leave a CTA as many iterations the smallest is the best (the sum costs more
+// with every chunk), so the search goes from one such count to the next with few
+// enough iterations to win, and over all that load them alike if the fewest among
+// them would not.  *tried: counts looked at.
 inline int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const SplitCost& k, double* cost_of,
                       int* tried = nullptr) {
   // (32-bit divisions: they are most of the search's time)
   auto ceil_div = [](unsigned a, unsigned b) { return (int)((a + b - 1) / b); };
   int best = c_lo;
   double best_cost = 1e300;
-  for (int c = c_lo; c <= c_hi;) {
+  int c = c_lo;
+  for (; c <= std::min(c_hi, kSmallCluster); ++c) {
+    const int per = ceil_div(turns, c);
+    if (c > c_lo && ceil_div(turns, per) != c) continue;
+    if (tried) ++*tried;
+    const double cost = k.cost(SplitCost::iterations(per, gps), k.load(k.on_one_sm(ublocks * c)), k.sum(c, ublocks));
+    if (cost < best_cost * 0.99) {
+      best_cost = cost;
+      best = c;
+    }
+  }
+  // the first count from c that no smaller one equals in turns per chunk
+  auto distinct = [&](int c) {
+    const int per = ceil_div(turns, c);
+    return ceil_div(turns, per) == c ? c : per > 1 ? ceil_div(turns, per - 1) : c_hi + 1;
+  };
+  for (c = distinct(c); c <= c_hi;) {
     // the counts from here that load the most loaded SM alike
     const int per_sm = k.on_one_sm(ublocks * c);
     const int beyond = std::min((int)((unsigned)(per_sm * k.sms) / (unsigned)ublocks), c_hi) + 1;
@@ -112,10 +131,7 @@ inline int fit_chunks(int turns, int gps, int ublocks, int c_lo, int c_hi, const
         c = fewer >= 1 ? ceil_div(turns, gps * fewer) : beyond;
       }
     }
-    // the first count beyond that no smaller one equals in turns per chunk
-    c = beyond;
-    const int per = ceil_div(turns, c);
-    if (ceil_div(turns, per) != c) c = per > 1 ? ceil_div(turns, per - 1) : c_hi + 1;
+    c = distinct(beyond);
   }
   *cost_of = best_cost;
   return best;
@@ -152,8 +168,8 @@ inline Split split_chunks(const SplitProblem& p, int gps, int* tried = nullptr) 
     return s;
   }
   // partial sums are written and read at about 4 TB/s
-  SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ,
-              !p.counters};
+  const double sums = (double)sets * p.planes * p.n;
+  SplitCost k{p.unit_us, ub * sums * 2e-6, sums * 1.1e-4, sums / p.threads, p.sms, p.occ, !p.counters};
   s.chunks = fit_chunks(p.turns, gps, ub, 1, most, k, &s.cost, tried);
   s.finalize = k.finalize(s.chunks, ub);
   if (p.counters && s.cost > kIdle * least_us(p, gps)) {

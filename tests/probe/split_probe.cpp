@@ -18,7 +18,7 @@ static int fit_every(int turns, int gps, int ublocks, int c_lo, int c_hi, const 
     if (c > c_lo && (turns + per - 1) / per != c) continue;
     const double per_sm = std::ceil((double)ublocks * c / k.sms);
     const double load = std::max(per_sm, 1.5 * std::ceil(per_sm / k.occ));
-    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 1.5 : k.kernel ? 4.0 + c * (k.partial + 0.04) : 2.0 + c * (k.partial + k.serial);
+    const double sum = c == 1 ? 0.0 : small_clustered(c, ublocks * c, k.sms) ? 0.5 + 0.15 * k.outputs / c : k.kernel ? 4.0 + c * (k.partial + 0.04) : 2.0 + c * (k.partial + k.serial);
     const double cost = ((per + gps - 1) / gps + 0.6) * k.unit * load + sum;
     if (cost < best_cost * 0.99) {
       best_cost = cost;
@@ -40,7 +40,8 @@ static Split every(const SplitProblem& p, int* tried) {
     const long long floats = (long long)p.all_units * p.planes * p.n;
     int c_hi = (int)std::min<long long>((p.turns + gps - 1) / gps, std::max(8, 4 * aim));
     if (p.max_partial) c_hi = (int)std::min<long long>(c_hi, std::max<long long>(1, (long long)p.max_partial / floats));
-    SplitCost k{p.unit_us, (double)ub * sets * p.planes * p.n * 2e-6, (double)sets * p.planes * p.n * 1.1e-4, p.sms, p.occ, !p.counters};
+    SplitCost k{p.unit_us, ub * ((double)sets * p.planes * p.n) * 2e-6, (double)sets * p.planes * p.n * 1.1e-4,
+                (double)sets * p.planes * p.n / p.threads, p.sms, p.occ, !p.counters};
     Split s;
     s.gps = gps;
     s.chunks = fit_every(p.turns, gps, ub, 1, std::max(1, c_hi), k, &s.cost, tried);
@@ -62,6 +63,7 @@ static SplitProblem problem(int n, int planes, int units, int turns, bool limits
   p.radix = planes == 1 && (n == 32 || n == 512 || n == 1024) ? 32 : n < 16 ? n : 16;
   const int t = n / p.radix, tpb = t > 128 ? t : 128;
   p.groups = tpb / t;
+  p.threads = tpb;
   p.units = p.all_units = units;
   p.turns = turns;
   p.sms = 152;
@@ -115,5 +117,7 @@ int main() {
     const Split s = split_groups_and_chunks(problem(n, 4, 1, 64, false));
     printf("chunks %d %d\n", s.chunks, s.finalize ? 1 : 0);
   }
+  // Two spectra whose sums within a pair of CTAs take longer than the second one.
+  for (int n : {2048, 4096}) printf("pair %d\n", split_groups_and_chunks(problem(n, 4, 1, 2, false)).chunks);
   return differ != 0;
 }

@@ -28,3 +28,8 @@ def test_split_is_that_of_every_count_at_a_few(probe):
 def test_one_unit_is_not_split_beyond_what_its_sum_costs(probe):
     chunks = [line.split()[1:] for line in probe.stdout.splitlines() if line.startswith("chunks")]
     assert len(chunks) == 3 and all(int(c) <= 8 or finalize == "1" for c, finalize in chunks), probe.stdout
+
+
+def test_large_spectra_are_not_split_over_a_pair(probe):
+    pairs = [line.split()[1] for line in probe.stdout.splitlines() if line.startswith("pair")]
+    assert pairs == ["1", "1"], probe.stdout
