@@ -398,8 +398,8 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
   constexpr bool kDirect = R < 32;
   if (kDirect && gps == 1 && !clustered) {
     // One group a unit: its threads hold the sums.  (Of 32 values each they go
-    // through shared memory all the same: with this branch the transforms'
-    // loop takes 1.5 % longer.)
+    // through shared memory all the same, eight at a time: with this branch the
+    // transforms' loop takes 5 % longer.)
     if (unit_ok) {
       float* const to = target(unit);
 #pragma unroll
@@ -448,7 +448,7 @@ __device__ __forceinline__ void small_body(const SmallLaunch& a, const int bid) 
     // (a cluster's CTA of one group has its sums where they belong)
     if (sum_ok && gps > 4) sum_groups(Int<1>{}, Int<4>{});
     else if (sum_ok && gps > 1) sum_groups(Int<(NP * R >= 16 ? 4 : 1)>{}, Int<2>{});
-    else if (!kDirect && sum_ok && !clustered) sum_groups(Int<1>{}, Int<1>{});
+    else if (!kDirect && sum_ok && !clustered) sum_groups(Int<8>{}, Int<1>{});
   }
   if (a.chunks == 1 || a.finalize) return;
 
