@@ -105,11 +105,18 @@ __device__ __forceinline__ float code_float(uint32_t offset) {
   return __uint_as_float(__byte_perm(offset, 0x47000000u, 0x7404 | (K << 4)));
 }
 
+// Asynchronous copies of 16 bytes from global to shared memory (past L1), and the
+// wait for all of a thread's.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------
 // Complex helpers.
 // ----------------------------------------------------------------------------
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 // a * w
 __device__ __forceinline__ float2 cmul(float2 a, float2 w) {
   return make_float2(__fmaf_rn(a.x, w.x, -a.y * w.y), __fmaf_rn(a.x, w.y, a.y * w.x));

@@ -82,12 +82,6 @@ struct RowCfg {
   static constexpr int ROWS_OUT = C * ROWS * GROUPS;
 };
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // *p += v for four floats, without a round trip.
 __device__ __forceinline__ void red_add4(float* p, float4 v) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
@@ -284,79 +278,79 @@ k_large_b(const __grid_constant__ LargeLaunch a) {
   float2* const my_xch = xch + (size_t)row * sub_stride<N1, CR, 2>();
 #pragma unroll 1
   for (int g = 0; g < Cf::GROUPS; ++g) {
-  const int r0 = (g * C + row) * ROWS;    // the transform's first row of the CTA's
-  const int k2 = tile * ROWS_OUT + r0;
-  // total power: per lane (a row each) of one polarisation, else their sum
-  float2 acc[NP == 4 || NV == 1 ? R : 1], xr[NP == 4 ? R : 1];
-  float tp[NP == 1 && NV == 2 ? R : 1];
-#pragma unroll
-  for (int m = 0; m < R; ++m) {
-    if constexpr (NP == 4 || NV == 1) acc[m] = make_float2(0.f, 0.f);
-    if constexpr (NP == 4) xr[m] = make_float2(0.f, 0.f);
-    if constexpr (NP == 1 && NV == 2) tp[m] = 0.0f;
-  }
-
-  for (int sl = s_begin; sl < s_end; ++sl) {
-    const int slab = c * a.Nss + d * a.M + sl;
-    cpair v[R];
-    if constexpr (NV == 2) {
-      const float4* src = reinterpret_cast<const float4*>(a.scratch) + ((size_t)slab * N2 + k2) * N1 + j;
-#pragma unroll
-      for (int m = 0; m < R; ++m) {
-        const float4 f = __ldcs(src + m * T);
-        v[m] = cpair{make_float2(f.x, f.y), make_float2(f.z, f.w)};
-      }
-    } else {
-      const float2* src = a.scratch + ((size_t)slab * N2 + k2) * N1 + j;
-#pragma unroll
-      for (int m = 0; m < R; ++m) v[m] = pack2(__ldcs(src + m * T), __ldcs(src + N1 + m * T));
-    }
-    GroupFFT<N1, R>::template run_packed<false>(v, j, my_xch, smem_padded_len(N1), tw_s, BlockSyncL{});
+    const int r0 = (g * C + row) * ROWS;    // the transform's first row of the CTA's
+    const int k2 = tile * ROWS_OUT + r0;
+    // total power: per lane (a row each) of one polarisation, else their sum
+    float2 acc[NP == 4 || NV == 1 ? R : 1], xr[NP == 4 ? R : 1];
+    float tp[NP == 1 && NV == 2 ? R : 1];
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      if constexpr (NP == 4) {
-        add_planes<POL>(v[m], acc[m], xr[m]);
-      } else if constexpr (NV == 1) {
-        acc[m] = f2add(acc[m], powers(v[m]));
+      if constexpr (NP == 4 || NV == 1) acc[m] = make_float2(0.f, 0.f);
+      if constexpr (NP == 4) xr[m] = make_float2(0.f, 0.f);
+      if constexpr (NP == 1 && NV == 2) tp[m] = 0.0f;
+    }
+
+    for (int sl = s_begin; sl < s_end; ++sl) {
+      const int slab = c * a.Nss + d * a.M + sl;
+      cpair v[R];
+      if constexpr (NV == 2) {
+        const float4* src = reinterpret_cast<const float4*>(a.scratch) + ((size_t)slab * N2 + k2) * N1 + j;
+#pragma unroll
+        for (int m = 0; m < R; ++m) {
+          const float4 f = __ldcs(src + m * T);
+          v[m] = cpair{make_float2(f.x, f.y), make_float2(f.z, f.w)};
+        }
       } else {
-        tp[m] += both_powers(v[m]);
+        const float2* src = a.scratch + ((size_t)slab * N2 + k2) * N1 + j;
+#pragma unroll
+        for (int m = 0; m < R; ++m) v[m] = pack2(__ldcs(src + m * T), __ldcs(src + N1 + m * T));
+      }
+      GroupFFT<N1, R>::template run_packed<false>(v, j, my_xch, smem_padded_len(N1), tw_s, BlockSyncL{});
+#pragma unroll
+      for (int m = 0; m < R; ++m) {
+        if constexpr (NP == 4) {
+          add_planes<POL>(v[m], acc[m], xr[m]);
+        } else if constexpr (NV == 1) {
+          acc[m] = f2add(acc[m], powers(v[m]));
+        } else {
+          tp[m] += both_powers(v[m]);
+        }
       }
     }
-  }
-  // value (plane p, or the lanes' rows) of element m
-  auto result = [&](int m, int p, int lane) -> float {
-    if constexpr (NP == 4) {
-      if (p == 2) return xr[m].x;
-      if (p == 3) return xr[m].y * im_sign;
-      return p == 0 ? acc[m].x : acc[m].y;
-    } else if constexpr (NV == 1) {
-      return lane == 0 ? acc[m].x : acc[m].y;
-    } else {
-      return tp[m];
-    }
-  };
+    // value (plane p, or the lanes' rows) of element m
+    auto result = [&](int m, int p, int lane) -> float {
+      if constexpr (NP == 4) {
+        if (p == 2) return xr[m].x;
+        if (p == 3) return xr[m].y * im_sign;
+        return p == 0 ? acc[m].x : acc[m].y;
+      } else if constexpr (NV == 1) {
+        return lane == 0 ? acc[m].x : acc[m].y;
+      } else {
+        return tp[m];
+      }
+    };
 
-  if constexpr (OUT) {  // k1 = j + m*T of the rows into the staging area
+    if constexpr (OUT) {  // k1 = j + m*T of the rows into the staging area
 #pragma unroll
-    for (int m = 0; m < R; ++m)
+      for (int m = 0; m < R; ++m)
 #pragma unroll
-      for (int p = 0; p < NP; ++p)
+        for (int p = 0; p < NP; ++p)
 #pragma unroll
-        for (int l = 0; l < ROWS; ++l) outs[((size_t)p * N1 + j + m * T) * ROWS_OUT + r0 + l] = result(m, p, l);
-  } else {
+          for (int l = 0; l < ROWS; ++l) outs[((size_t)p * N1 + j + m * T) * ROWS_OUT + r0 + l] = result(m, p, l);
+    } else {
 #pragma unroll
-    for (int m = 0; m < R; ++m)
+      for (int m = 0; m < R; ++m)
 #pragma unroll
-      for (int p = 0; p < NP; ++p)
+        for (int p = 0; p < NP; ++p)
 #pragma unroll
-        for (int l = 0; l < ROWS; ++l) {
-          const int k = k2 + l + N2 * (j + m * T);
-          float* o = obase + p * plane + (part ? k : out_pos(k, N, a.inverse));
-          const float x = result(m, p, l) * scale;
-          if (add) atomicAdd(o, x);  // each element once per launch: a plain add, without a round trip
-          else *o = x;
-        }
-  }
+          for (int l = 0; l < ROWS; ++l) {
+            const int k = k2 + l + N2 * (j + m * T);
+            float* o = obase + p * plane + (part ? k : out_pos(k, N, a.inverse));
+            const float x = result(m, p, l) * scale;
+            if (add) atomicAdd(o, x);  // each element once per launch: a plain add, without a round trip (with: 2^19 points 258 -> 314 us)
+            else *o = x;
+          }
+    }
   }
   if constexpr (!OUT) return;
   __syncthreads();
@@ -407,7 +401,7 @@ cudaError_t launch_a_t(const LargeLaunch& L, cudaStream_t s, bool prep) {
   return cudaGetLastError();
 }
 
-// Units of at most this many spectra per chunk stage their results: one
+// Units of at most this many spectra in a buffer stage their results: one
 // spectrum, 2^16 points 319 -> 270 us, 2^18 496 -> 375; with 16 the staging
 // costs more than it gives (2^18 237 -> 311).
 constexpr int kStageOutSpectra = 2;

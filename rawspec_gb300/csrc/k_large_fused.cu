@@ -800,8 +800,8 @@ bool large_fused_supported(const LargeLaunch& L) {
 // 2^16 804 / 833, 2^20 1150 / 1600.  A single transform or two leave it nothing
 // to overlap (2^16, one: 67 against 28 us from call to result; 2^20 88 / 62).
 // Short total-power transforms of small buffers would gain too (twelve of 2^16
-// 83 against 43 us) but stay: the choice of this kernel at such a size is
-// part of what the tuning table's users (and its tests) rely on.
+// 83 against 43 us) but stay: tuning tables set this kernel's lag and ring at such
+// sizes against the library's own choice of it.
 constexpr long long kSmallBuffer = 1ll << 20;  // time samples over all channels
 bool large_fused_wanted(const LargeLaunch& L) {
   const long long slabs = (long long)L.Nc * L.Nss;

@@ -117,11 +117,6 @@ __device__ __forceinline__ float cluster_load(uint32_t addr) {
   return f;
 }
 
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
 // The same through L1 (neighbouring copies share a 32-byte sector).
 __device__ __forceinline__ void cp_async16_l1(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
@@ -134,7 +129,6 @@ __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
                "l"(src)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The kernel body for CTA `bid` of launch `a` (k_small: one launch;
 // k_small_group: several launches of the same configuration, e.g. the

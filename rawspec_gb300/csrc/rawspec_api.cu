@@ -216,10 +216,11 @@ bool graphs_wanted(const GpuCtx* g) {
 
 // Which products of 8-bit input run their DFT on the tensor cores (k_tc)
 // rather than in k_small: by default the 1024-point total-power products of
-// buffers of at most 2^18 time samples over all channels, where the launch is
-// the time and k_tc, which splits a unit further, is not the slower one
-// (4 channels x 16384 samples 7.8 against 8.0 us a buffer, 1 x 65536 8.0
-// against 10.8; 8 x 65536 9.9 against 8.8, 64 x 262144 59 against 42).
+// buffers of at most 2^18 time samples over all channels, where the launches
+// and the dump are the time with either kernel (from call to result by k_tc and
+// by k_small: 4 channels x 16384 samples 24.4 and 24.1 us, 1 x 65536 23.7 and
+// 23.5, 64 x 4096 25.2 and 25.4; a buffer among others 8 x 65536 9.9 and 8.8, 64
+// x 262144 59 and 42).
 // RAWSPEC_GB300_TENSOR_DFT=1 at initialisation selects k_tc for every case it
 // supports (N = 256, 1024, 4096, all modes up to 1024), =0 for none.  Without
 // the variable, a tuning-table entry's dft= decides before the default.

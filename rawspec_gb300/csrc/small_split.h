@@ -21,7 +21,8 @@ namespace rsg {
 // one cluster of SMs.  Four units of 8 x 2048 points in four planes: 28 us
 // without, 27 with pairs, 12 with 8; 64 Mi samples of 2048 points in four
 // planes, 1024 CTAs: 278 without, 256 with pairs, 259 with 4, 267 with 8; four
-// products in four planes, 4096 to 8 points: 108, 110, 110, 121.
+// products in four planes, 4096 to 8 points: 108, 110, 110, 121.  (Launches that
+// share a grid have no clusters: their units' last CTAs sum.)
 constexpr int kSmallCluster = 8;
 inline bool small_clustered(int chunks, int ctas, int sms) {
   return chunks == 2 || (chunks > 1 && chunks <= kSmallCluster && ctas <= sms);
@@ -81,8 +82,9 @@ struct SplitCost {
 // by its own latency, about 1.5 times its share of a full one.  A unit split
 // within a cluster adds about 0.5 us and 0.15 for each output that a thread sums
 // (two spectra of 4096 points in four planes: one CTA 10.3 us a call, a pair, 32
-// outputs a thread, 14.4); one split over more CTAs the traffic of the partial sums, and an arrival and their sum by one CTA (36 GB/s) or a kernel
-// over all outputs.
+// outputs a thread, 14.4); one split over more CTAs the traffic of the partial
+// sums, and an arrival and their sum by one CTA (36 GB/s) or a kernel over all
+// outputs.
 //
 // Counts of a cluster are all looked at.  Of larger ones that load the SMs alike
 // and leave a CTA as many iterations the smallest is the best (the sum costs more
